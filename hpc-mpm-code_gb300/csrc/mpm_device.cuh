@@ -469,6 +469,29 @@ __device__ __forceinline__ void tait_stress(R *s, const R inc[3][3], R jm1, R rh
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// A launch of kernel k on st; with pdl, with programmatic stream
+// serialization, so that its CTAs are scheduled while its predecessor drains
+// (the kernel's pdl_wait orders its memory accesses after the predecessor).
+template <typename... P, typename... A>
+inline void launch(bool pdl, void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                   A... args) {
+    if (!pdl) {
+        k<<<grid, block, smem, st>>>(args...);
+        return;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, args...);
+}
+
 // det(I + H) - 1 in FP64 for a row-major H[9] (host and device)
 __host__ __device__ inline double det_ipm1_d(const double *H) {
     const double tr = H[0] + H[4] + H[8];

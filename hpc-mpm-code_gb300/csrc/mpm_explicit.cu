@@ -3329,29 +3329,6 @@ static int num_sms() {
     return n;
 }
 
-// A launch of kernel k on st; with pdl, with programmatic stream
-// serialization, so that its CTAs are scheduled while its predecessor drains
-// (the kernel's pdl_wait orders its memory accesses after the predecessor).
-template <typename... P, typename... A>
-static void launch(bool pdl, void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
-                   A... args) {
-    if (!pdl) {
-        k<<<grid, block, smem, st>>>(args...);
-        return;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k, args...);
-}
-
 // persistent grid over the active-brick list: never more CTAs than bricks
 static int list_grid(const mpm_ctx *c, int per_sm) {
     return std::min(c->g.nbricks, per_sm * num_sms());

@@ -17,6 +17,7 @@
 
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <new>
 #include <vector>
@@ -324,7 +325,7 @@ struct NsVec {
 };
 
 // Sums of V per-thread values over the grid: block partials in part[v * gridDim.x + b];
-// the last block to finish adds them in block order (run-to-run identical) and returns true.
+// the last block to finish adds them in a fixed order (run-to-run identical) and returns true.
 template <int V>
 __device__ bool ns_reduce(double (&v)[V], double *part, unsigned *cnt, double (&tot)[V]) {
     __shared__ double sh[V][8];
@@ -348,10 +349,14 @@ __device__ bool ns_reduce(double (&v)[V], double *part, unsigned *cnt, double (&
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    if ((int)threadIdx.x < V) {
+    // one warp per value: lane l adds the partials l, l + 32, ..., then the lanes
+    // are added by a fixed tree (one thread per value, block after block, took
+    // longer than the rest of the kernel)
+    for (int j = wid; j < V; j += (int)(blockDim.x >> 5)) {
         double t = 0.0;
-        for (unsigned b = 0; b < gridDim.x; b++) t += __ldcg(part + threadIdx.x * gridDim.x + b);
-        sh[threadIdx.x][0] = t;
+        for (unsigned b = lane; b < gridDim.x; b += 32) t += __ldcg(part + (size_t)j * gridDim.x + b);
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) sh[j][0] = t;
     }
     __syncthreads();
 #pragma unroll
@@ -386,30 +391,54 @@ __global__ void k_nsv_scale_mat(KGeom<double> g, double *A, const double *adiag)
     }
 }
 
-// y = A x with the BC rows zeroed (MatVecMult + BCResidualSet)
-__global__ void __launch_bounds__(256) k_nsv_matvec(KGeom<double> g, const double *__restrict__ A,
-                                                    const unsigned char *__restrict__ bcf, const double *x, double *y,
-                                                    const double *done) {
-    if (done && *done != 0.0) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= g.nodec) return;
+// y = A x with the BC rows zeroed (MatVecMult + BCResidualSet).  The block's
+// NSV_NODES nodes are its x dimension (coalesced in A), and G threads share a
+// node's 27 slots; the node's row sums are added over the groups in order.
+// With one thread per node (432 FMAs and as many loads in a row) a fluid box
+// has far too few warps for the loads' latency and the FP64 pipe, which bounds the
+// product (at 8,925 nodes the pipe needs 6.6 us; ns_matvec chooses G).
+constexpr int NSV_NODES = 32;
+constexpr int NSV_T = 128;   // nodes per CTA of the vector passes
+template <int G>
+__global__ void __launch_bounds__(NSV_NODES * G) k_nsv_matvec(KGeom<double> g, const double *__restrict__ A,
+                                                              const unsigned char *__restrict__ bcf, const double *x,
+                                                              double *y, const double *done) {
+    static_assert(27 % G == 0 && G >= 3, "slots per thread");
+    constexpr int SL = 27 / G;
+    __shared__ double sh[G][4][NSV_NODES];
+    pdl_wait();
+    if (done && *done != 0.0) return;   // uniform over the grid
+    const int lane = threadIdx.x % NSV_NODES, grp = threadIdx.x / NSV_NODES;
+    const int n = blockIdx.x * NSV_NODES + lane;
     const size_t N = (size_t)g.nodec;
-    const int i = n % g.nnc[0], j = (n / g.nnc[0]) % g.nnc[1], k = n / (g.nnc[0] * g.nnc[1]);
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    if (n < g.nodec) {
+        const int i = n % g.nnc[0], j = (n / g.nnc[0]) % g.nnc[1], k = n / (g.nnc[0] * g.nnc[1]);
 #pragma unroll
-    for (int s = 0; s < 27; s++) {
-        const int ii = i + s % 3 - 1, jj = j + (s / 3) % 3 - 1, kk = k + s / 9 - 1;
-        if (ii < 0 || jj < 0 || kk < 0 || ii >= g.nnc[0] || jj >= g.nnc[1] || kk >= g.nnc[2]) continue;
-        const size_t col = ii + (size_t)g.nnc[0] * (jj + (size_t)g.nnc[1] * kk);
-        const double xc[4] = {x[col], x[N + col], x[2 * N + col], x[3 * N + col]};
+        for (int q = 0; q < SL; q++) {
+            const int s = grp * SL + q;
+            const int ii = i + s % 3 - 1, jj = j + (s / 3) % 3 - 1, kk = k + s / 9 - 1;
+            if (ii < 0 || jj < 0 || kk < 0 || ii >= g.nnc[0] || jj >= g.nnc[1] || kk >= g.nnc[2]) continue;
+            const size_t col = ii + (size_t)g.nnc[0] * (jj + (size_t)g.nnc[1] * kk);
+            const double xc[4] = {x[col], x[N + col], x[2 * N + col], x[3 * N + col]};
+            const double *As = A + (size_t)s * 16 * N + n;
 #pragma unroll
-        for (int r = 0; r < 4; r++)
+            for (int r = 0; r < 4; r++)
 #pragma unroll
-            for (int c = 0; c < 4; c++) acc[r] = fma(__ldg(A + (size_t)(s * 16 + 4 * r + c) * N + n), xc[c], acc[r]);
+                for (int c = 0; c < 4; c++) acc[r] = fma(__ldg(As + (size_t)(4 * r + c) * N), xc[c], acc[r]);
+        }
     }
-    const unsigned char f = bcf[n];
 #pragma unroll
-    for (int r = 0; r < 4; r++) y[r * N + n] = (f >> r) & 1 ? 0.0 : acc[r];
+    for (int r = 0; r < 4; r++) sh[grp][r][lane] = acc[r];
+    __syncthreads();
+    if (n >= g.nodec) return;
+    const unsigned char f = bcf[n];
+    for (int r = grp; r < 4; r += G) {
+        double t = sh[0][r][lane];
+#pragma unroll
+        for (int q = 1; q < G; q++) t += sh[q][r][lane];
+        y[r * N + n] = (f >> r) & 1 ? 0.0 : t;
+    }
 }
 
 // ScaleSolution + BCResidualSet: xs = x / D, rr = b D (zero where D < mtol and on BC rows)
@@ -452,35 +481,49 @@ __global__ void __launch_bounds__(256) k_nsv_init(int nodec, NsVec v, double *pa
     }
 }
 
+// The vector passes of an iteration: one thread per node, and the loads of its
+// four values are issued before the first store (walking the values one after
+// another took four times the memory latency, which is all that such a pass
+// costs on a fluid box).  One thread per value is as fast there and slower on
+// large grids, where the FP64 adds of the warp reductions count: 502 against
+// 464 us per iteration at 198,000 nodes.
 // pp = rr + beta (pp - uu), Ap = Ar + beta (Ap - Au); the six dots; then alpha, zeta, eta
-__global__ void __launch_bounds__(256) k_gpb_1(int nodec, NsVec v, double *part, unsigned *cnt, double *scal) {
+__global__ void __launch_bounds__(NSV_T) k_gpb_1(int nodec, NsVec v, double *part, unsigned *cnt, double *scal) {
+    pdl_wait();
     if (scal[NS_DONE] != 0.0) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const double beta = scal[NS_BETA];
     double d[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     if (n < nodec) {
         const size_t N = (size_t)nodec;
+        double r[4], pp[4], uu[4], ar[4], ap[4], au[4], az[4], rs[4];
+#pragma unroll
         for (int m = 0; m < 4; m++) {
             const size_t i = m * N + n;
-            const double p = v.rr[i] + beta * (v.pp[i] - v.uu[i]);
-            const double ap = v.Ar[i] + beta * (v.Ap[i] - v.Au[i]);
-            v.pp[i] = p;
-            v.Ap[i] = ap;
-            const double az = v.Az[i], ar = v.Ar[i], r = v.rr[i];
-            d[0] += v.rs[i] * ap;
-            d[1] += az * az;
-            d[2] += ar * r;
-            d[3] += az * r;
-            d[4] += ar * az;
-            d[5] += ar * ar;
+            r[m] = v.rr[i], pp[m] = v.pp[i], uu[m] = v.uu[i], ar[m] = v.Ar[i];
+            ap[m] = v.Ap[i], au[m] = v.Au[i], az[m] = v.Az[i], rs[m] = v.rs[i];
+        }
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const size_t i = m * N + n;
+            const double w = ar[m] + beta * (ap[m] - au[m]);
+            v.pp[i] = r[m] + beta * (pp[m] - uu[m]);
+            v.Ap[i] = w;
+            d[0] += rs[m] * w;
+            d[1] += az[m] * az[m];
+            d[2] += ar[m] * r[m];
+            d[3] += az[m] * r[m];
+            d[4] += ar[m] * az[m];
+            d[5] += ar[m] * ar[m];
         }
     }
     double t[6];
     if (!ns_reduce<6>(d, part, cnt, t)) return;
     if (threadIdx.x == 0) {
         const double rAp = t[0], AzAz = t[1], Arrr = t[2], Azrr = t[3], ArAz = t[4], ArAr = t[5];
-        scal[NS_RSR0] = scal[NS_RSR];
-        scal[NS_ALPH] = scal[NS_RSR] / rAp;
+        const double rsr = scal[NS_RSR];
+        scal[NS_RSR0] = rsr;
+        scal[NS_ALPH] = rsr / rAp;
         if (scal[NS_ITER] == 0.0) {
             scal[NS_ZETA] = Arrr / ArAr;
             scal[NS_ETA] = 0.0;
@@ -492,41 +535,46 @@ __global__ void __launch_bounds__(256) k_gpb_1(int nodec, NsVec v, double *part,
     }
 }
 
-// uu = zeta Ap + eta (Az + beta uu)
-__global__ void k_gpb_2(int nodec, NsVec v, const double *scal) {
+// uu = zeta Ap + eta (Az + beta uu), one thread per value
+__global__ void __launch_bounds__(256) k_gpb_2(int n4, NsVec v, const double *scal) {
+    pdl_wait();
     if (scal[NS_DONE] != 0.0) return;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= nodec) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n4) return;
     const double zeta = scal[NS_ZETA], eta = scal[NS_ETA], beta = scal[NS_BETA];
-    const size_t N = (size_t)nodec;
-    for (int m = 0; m < 4; m++) {
-        const size_t i = m * N + n;
-        v.uu[i] = zeta * v.Ap[i] + eta * (v.Az[i] + beta * v.uu[i]);
-    }
+    v.uu[i] = zeta * v.Ap[i] + eta * (v.Az[i] + beta * v.uu[i]);
 }
 
 // tt = rr - alpha Ap; zz = zeta rr + eta zz - alpha uu; Az = zeta Ar + eta Az - alpha Au;
 // x += alpha pp + zz; rr = tt - Az; then rsr, rtr, the stopping test rtr < eps btb and beta
-__global__ void __launch_bounds__(256) k_gpb_3(int nodec, NsVec v, double eps, double *part, unsigned *cnt,
-                                               double *scal) {
+__global__ void __launch_bounds__(NSV_T) k_gpb_3(int nodec, NsVec v, double eps, double *part, unsigned *cnt,
+                                                 double *scal) {
+    pdl_wait();
     if (scal[NS_DONE] != 0.0) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const double alph = scal[NS_ALPH], zeta = scal[NS_ZETA], eta = scal[NS_ETA];
     double d[2] = {0.0, 0.0};
     if (n < nodec) {
         const size_t N = (size_t)nodec;
+        double r[4], ap[4], zz[4], uu[4], ar[4], az[4], au[4], xs[4], pp[4], rs[4];
+#pragma unroll
         for (int m = 0; m < 4; m++) {
             const size_t i = m * N + n;
-            const double r = v.rr[i];
-            const double tt = r - alph * v.Ap[i];
-            const double zz = zeta * r + eta * v.zz[i] - alph * v.uu[i];
-            const double az = zeta * v.Ar[i] + eta * v.Az[i] - alph * v.Au[i];
-            v.zz[i] = zz;
-            v.Az[i] = az;
-            v.xs[i] += alph * v.pp[i] + zz;
-            const double rn = tt - az;
+            r[m] = v.rr[i], ap[m] = v.Ap[i], zz[m] = v.zz[i], uu[m] = v.uu[i], ar[m] = v.Ar[i];
+            az[m] = v.Az[i], au[m] = v.Au[i], xs[m] = v.xs[i], pp[m] = v.pp[i], rs[m] = v.rs[i];
+        }
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const size_t i = m * N + n;
+            const double tt = r[m] - alph * ap[m];
+            const double z = zeta * r[m] + eta * zz[m] - alph * uu[m];
+            const double a = zeta * ar[m] + eta * az[m] - alph * au[m];
+            const double rn = tt - a;
+            v.zz[i] = z;
+            v.Az[i] = a;
+            v.xs[i] = xs[m] + (alph * pp[m] + z);
             v.rr[i] = rn;
-            d[0] += v.rs[i] * rn;
+            d[0] += rs[m] * rn;
             d[1] += rn * rn;
         }
     }
@@ -840,6 +888,9 @@ struct mpm_ns {
     unsigned *cnt = nullptr;
     int *status = nullptr;
     NsVec v{};
+    cudaGraphExec_t graph = nullptr;   // NS_BLOCK GPBiCGSafe iterations (ns_graph)
+    double graph_eps = 0.0;
+    bool no_graph = false;
     std::vector<int> bc_nodes[4];
     std::vector<double> bc_vals[4];
     // time step (mpm_ns_step): nodal state, P2G sums and bounds, particle scratch
@@ -868,6 +919,7 @@ struct mpm_ns {
 
 extern "C" void mpm_ns_destroy(mpm_ns *s) {
     if (!s) return;
+    if (s->graph) cudaGraphExecDestroy(s->graph);
     void *bufs[] = {s->A,     s->b,      s->adiag,  s->x,      s->bcv,    s->part, s->scal,  s->bcf,
                     s->cnt,   s->status, s->v.rr,   s->v.rs,   s->v.pp,   s->v.Ap, s->v.Ar,  s->v.Az,
                     s->v.Au,  s->v.uu,   s->v.zz,   s->v.xs,   s->v.Ax,   s->nmass, s->nvof, s->nvel,
@@ -891,7 +943,7 @@ extern "C" mpm_status mpm_ns_create(const mpm_grid_desc *grid, const mpm_ns_para
     s->a = a;
     s->nodec = a.g.nodec;
     const size_t N = (size_t)a.g.nodec;
-    const int nb = (int)((N + 255) / 256);
+    const size_t npart = (N + NSV_T - 1) / NSV_T;
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void **p, size_t bytes) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
@@ -901,7 +953,7 @@ extern "C" mpm_status mpm_ns_create(const mpm_grid_desc *grid, const mpm_ns_para
     alloc((void **)&s->adiag, sizeof(double) * 4 * N);
     alloc((void **)&s->x, sizeof(double) * 4 * N);
     alloc((void **)&s->bcv, sizeof(double) * 4 * N);
-    alloc((void **)&s->part, sizeof(double) * 8 * (size_t)nb);
+    alloc((void **)&s->part, sizeof(double) * 8 * npart);
     alloc((void **)&s->scal, sizeof(double) * NS_NSCAL);
     alloc((void **)&s->bcf, N);
     alloc((void **)&s->cnt, sizeof(unsigned) * 4);
@@ -950,12 +1002,27 @@ extern "C" mpm_status mpm_ns_set_bc(mpm_ns *s, int comp, int n, const int *nodes
     return MPM_OK;
 }
 
+// y = A x on the context's stream.  A small box has too few nodes to fill the
+// chip with one warp per 32 of them: nine threads share a node up to 32,768
+// nodes (8,925 nodes: 50 us per GPBiCGSafe iteration against 62 with three and
+// 115 with one); on larger grids three do, which add six FP64 numbers per row
+// less (198,000 nodes: 441 against 481 and 572 us).
+static void ns_matvec(const mpm_ns *s, const double *x, double *y, const double *done, cudaStream_t st) {
+    const unsigned nb = (unsigned)((s->nodec + NSV_NODES - 1) / NSV_NODES);
+    if (s->nodec <= 32768)
+        launch(true, k_nsv_matvec<9>, nb, 9 * NSV_NODES, 0, st, s->a.g, (const double *)s->A,
+               (const unsigned char *)s->bcf, x, y, done);
+    else
+        launch(true, k_nsv_matvec<3>, nb, 3 * NSV_NODES, 0, st, s->a.g, (const double *)s->A,
+               (const unsigned char *)s->bcf, x, y, done);
+}
+
 // ||b - A x|| and sqrt(rtr / idof) of the scaled system in s (ComputeRefResidual /
 // ComputeAbsResidual); x is physical.  Synchronises the stream.
 static mpm_status ns_residual(mpm_ns *s, const double *x, double *ref, double *absr) {
     const int nodec = s->nodec, nb = (nodec + 255) / 256, nb4 = (4 * nodec + 255) / 256;
     k_nsv_prep<<<nb4, 256, 0, s->stream>>>(nodec, s->a.mtol, x, s->adiag, s->v.Ax);
-    k_nsv_matvec<<<nb, 256, 0, s->stream>>>(s->a.g, s->A, s->bcf, s->v.Ax, s->v.Ar, nullptr);
+    ns_matvec(s, s->v.Ax, s->v.Ar, nullptr, s->stream);
     k_nsv_resid<<<nb, 256, 0, s->stream>>>(nodec, s->a.mtol, s->bcf, s->b, s->v.Ar, s->adiag, s->part, s->cnt,
                                            s->scal);
     CKN(cudaMemcpyAsync(s->h_scal, s->scal, sizeof(double) * NS_NSCAL, cudaMemcpyDeviceToHost, s->stream));
@@ -968,25 +1035,69 @@ static mpm_status ns_residual(mpm_ns *s, const double *x, double *ref, double *a
 
 // One GPBiCGSafe call (solver.cpp:19-141) on the scaled system from the current
 // physical s->x, stopped at rtr < eps btb as the reference does, or at kmax
-// iterations.  Iterations are launched in blocks of 8; once the device-side
-// test has stopped the solve the remaining launches of a block return at once.
+// iterations.  Iterations are launched in blocks of NS_BLOCK (one graph launch);
+// once the device-side test has stopped the solve the remaining launches of a
+// block return at once.
+static constexpr int NS_BLOCK = 8;
+
+// One GPBiCGSafe iteration: two products and three vector passes, each launched
+// while its predecessor drains.  Latency bounds it on a fluid box (five dependent
+// passes, three grid-wide reductions); at 8,925 nodes it takes 50 us, 115 before
+// the products were split and the passes issued their loads together in a graph.
+static void ns_iteration(const mpm_ns *s, double eps, cudaStream_t st) {
+    const int n = s->nodec, nb = (n + NSV_T - 1) / NSV_T;
+    const double *done = s->scal + NS_DONE;
+    ns_matvec(s, s->v.rr, s->v.Ar, done, st);
+    launch(true, k_gpb_1, nb, NSV_T, 0, st, n, s->v, s->part, s->cnt + 1, s->scal);
+    launch(true, k_gpb_2, (4 * n + 255) / 256, 256, 0, st, 4 * n, s->v, (const double *)s->scal);
+    ns_matvec(s, s->v.uu, s->v.Au, done, st);
+    launch(true, k_gpb_3, nb, NSV_T, 0, st, n, s->v, eps, s->part, s->cnt + 2, s->scal);
+}
+
+// The graph of NS_BLOCK iterations with stopping test eps, captured on a stream
+// of its own (the context's may be the legacy default stream, which cannot be
+// captured).  Every pointer in it is the context's and lives as long as the
+// graph.  False when there is none: the iterations are then launched one by one.
+static bool ns_graph(mpm_ns *s, double eps) {
+    if (s->graph && s->graph_eps == eps) return true;
+    if (s->no_graph) return false;
+    if (s->graph) cudaGraphExecDestroy(s->graph);
+    s->graph = nullptr;
+    cudaStream_t cap = nullptr;
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+        for (int k = 0; k < NS_BLOCK; k++) ns_iteration(s, eps, cap);
+        e = cudaStreamEndCapture(cap, &g);
+    }
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&s->graph, g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (cap) cudaStreamDestroy(cap);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        s->graph = nullptr;
+        s->no_graph = true;
+        return false;
+    }
+    s->graph_eps = eps;
+    return true;
+}
+
 static mpm_status ns_gpbicgsafe(mpm_ns *s, double eps, int kmax, int *iters) {
     const int nodec = s->nodec, nb = (nodec + 255) / 256, nb4 = (4 * nodec + 255) / 256;
     cudaStream_t st = s->stream;
-    const double *done = s->scal + NS_DONE;
     k_nsv_scale_in<<<nb, 256, 0, st>>>(nodec, s->a.mtol, s->bcf, s->x, s->b, s->adiag, s->v.xs, s->v.rr);
-    k_nsv_matvec<<<nb, 256, 0, st>>>(s->a.g, s->A, s->bcf, s->v.xs, s->v.Ax, nullptr);
+    ns_matvec(s, s->v.xs, s->v.Ax, nullptr, st);
     k_nsv_init<<<nb, 256, 0, st>>>(nodec, s->v, s->part, s->cnt, s->scal);
     int it = 0;
     bool finished = false;
     while (!finished && it < kmax) {
-        const int blk = kmax - it < 8 ? kmax - it : 8;
-        for (int k = 0; k < blk; k++) {
-            k_nsv_matvec<<<nb, 256, 0, st>>>(s->a.g, s->A, s->bcf, s->v.rr, s->v.Ar, done);
-            k_gpb_1<<<nb, 256, 0, st>>>(nodec, s->v, s->part, s->cnt + 1, s->scal);
-            k_gpb_2<<<nb, 256, 0, st>>>(nodec, s->v, s->scal);
-            k_nsv_matvec<<<nb, 256, 0, st>>>(s->a.g, s->A, s->bcf, s->v.uu, s->v.Au, done);
-            k_gpb_3<<<nb, 256, 0, st>>>(nodec, s->v, eps, s->part, s->cnt + 2, s->scal);
+        const int blk = kmax - it < NS_BLOCK ? kmax - it : NS_BLOCK;
+        if (blk == NS_BLOCK && ns_graph(s, eps)) {
+            CKN(cudaGraphLaunch(s->graph, st));
+        } else {
+            for (int k = 0; k < blk; k++) ns_iteration(s, eps, st);
         }
         CKN(cudaGetLastError());
         CKN(cudaMemcpyAsync(s->h_scal, s->scal, sizeof(double) * NS_NSCAL, cudaMemcpyDeviceToHost, st));
