@@ -1,0 +1,207 @@
+// Arguments and building blocks shared by the explicit step's kernels
+// (mpm_explicit.cu, mpm_cells.cu).
+#pragma once
+
+#include "mpm_device.cuh"
+
+namespace mpm {
+
+template <typename R>
+struct StepArgs {
+    KGeom<R> g;
+    Particles<R> P;
+    int64_t num;
+    const WorkItem *work;
+    const int *nwork;
+    const int *cstart;          // nbricks * (BRC + 1)
+    int *miss;                  // particles that left their sorted cell, processed by a deferred pass
+    const int *blist;           // bricks holding particles (brick order) and their count
+    const int *nblist;
+    const int *tlist;           // active node tiles of this step (tile order) and their count
+    const int *ntlist;
+    int nbrick[3];
+    unsigned long long *acc;    // NACC * nodec
+    unsigned long long *acc2;   // 3 * nodec
+    unsigned long long *facc;   // nodec (F-bar contexts)
+    R *G;                       // gather field for the velocity gather (3 * nodec)
+    R *nei;                     // nodec
+    R *nvel2;                   // 3 * nodec
+    R *nvel_dl, *naccel_dl;     // 3 * nodec each, written only in download mode
+    const double *nvol;
+    const unsigned char *bcflag;
+    const R *bcval;
+    unsigned char *tileflag;
+    double *eu_part;
+    DevCtl *ctl;
+    const int *iprop;
+    const double *matprop;
+    const float *matpropf;      // the same table in FP32 (the FP32 particle kernels)
+    R dt, facl, mtol, grav[3];
+    int parity;
+    int scheme;
+    int shifting;
+    int all_tiles;              // process every tile in the grid passes (download mode)
+    int gnorm;                  // FP32 gathers divide by their weight sum
+    int implicit;               // implicit solid: the force fields carry sum N m a (AccelP2G)
+    int fbar;                   // F-bar projection: k_grid2 leaves the nodal volume sums to k_fbar_grid
+    int sigma_in;               // some material's stress update reads the previous stress (model 0)
+    int single_mat;             // one material: every particle's matid is 0
+    int fluidj;                 // Tait fluid only: F field 0 holds J - 1, fields 1-8 unused (FP32)
+    // traversal directions of the particle kernels: each starts where the
+    // previous particle pass ended, so its first bricks are still in L2
+    int rev_p2g, rev_g2p, rev_upd;
+    double nump;                // particle count as a bound factor
+    double mmax;                // max particle mass
+    double gshape;              // bound on |dN/dx|
+    double gsum;                // bound on sum_i |dN_i/dx|
+};
+
+// ----------------------------------------------------------------- helpers
+template <typename R>
+__device__ __forceinline__ R ld(const R *p) { return __ldg(p); }
+
+__device__ __forceinline__ void tile_coords(int t, const int *nt, int &tx, int &ty, int &tz) {
+    tx = t % nt[0];
+    ty = (t / nt[0]) % nt[1];
+    tz = t / (nt[0] * nt[1]);
+}
+
+template <typename R>
+__device__ __forceinline__ int tile_of_node(const KGeom<R> &g, int gx, int gy, int gz) {
+    return gx / TILE + g.ntile[0] * (gy / TILE + g.ntile[1] * (gz / TILE));
+}
+
+template <typename R>
+__device__ __forceinline__ size_t node_id(const KGeom<R> &g, int gx, int gy, int gz) {
+    return (size_t)gx + (size_t)g.nnc[0] * ((size_t)gy + (size_t)g.nnc[1] * (size_t)gz);
+}
+
+// Fixed-point scales.  Computed by one thread of a CTA (FP64 scalar work)
+// and shared; producer and consumer kernels derive them from the same
+// device-resident bounds, so they agree exactly.
+
+template <typename R>
+__device__ void compute_scales(const StepArgs<R> &a, Scales &s) {
+    const unsigned *nb = a.ctl->nxt[a.parity];
+    double gabs = fmax(fabs((double)a.grav[0]), fmax(fabs((double)a.grav[1]), fabs((double)a.grav[2])));
+    s.m = make_fix(a.nump * a.mmax);
+    s.v = make_fix(a.nump * (double)bits_f(nb[B_VOLMAX]));
+    s.p = make_fix(a.nump * a.mmax * (double)bits_f(nb[B_VMAX]));
+    s.f = a.implicit ? make_fix(a.nump * a.mmax * (double)bits_f(nb[B_AMAX]) * 1.0000001)
+                     : make_fix(a.nump * ((double)bits_f(nb[B_VOLSMAX]) * 3.0 * a.gshape +
+                                          a.mmax * gabs * fabs((double)a.facl)));
+    double vb = (double)bits_f(a.ctl->cur[C_GMAX]);
+    if (a.scheme == MPM_FLIP) vb = (double)bits_f(nb[B_VMAX]) + fabs((double)a.dt) * vb;
+    s.q = make_fix(a.nump * a.mmax * vb * 1.0000001);
+    double gb = 2.0 * (double)bits_f(nb[B_VOLMAX]) * a.gsum * (double)bits_f(a.ctl->cur[C_NEIMAX]);
+    s.gd = make_fix(a.nump * 3.0 * gb * gb * 1.0000001);
+}
+
+// The scales of a step are computed once: the P2G ones by k_step_reset, the
+// gather/MUSL ones by the last CTA of k_grid1 (they depend on the grid
+// maxima it records).  Kernels copy them into shared memory.
+template <typename R>
+__device__ __forceinline__ void load_scales_from(const Scales *src, Scales &sh) {
+    constexpr int W = (int)(sizeof(Scales) / 4);
+    if ((int)threadIdx.x < W) reinterpret_cast<unsigned *>(&sh)[threadIdx.x] = reinterpret_cast<const unsigned *>(src)[threadIdx.x];
+    __syncthreads();
+}
+template <typename R>
+__device__ __forceinline__ void load_scales(const StepArgs<R> &a, Scales &sh) {
+    load_scales_from<R>(&a.ctl->sc_p2g, sh);
+}
+template <typename R>
+__device__ __forceinline__ void load_scales_musl(const StepArgs<R> &a, Scales &sh) {
+    load_scales_from<R>(&a.ctl->sc_musl, sh);
+}
+
+// Block-wide reduction (fixed order: deterministic); result valid in thread 0.
+template <typename T, typename Op>
+__device__ __forceinline__ T block_reduce(T v, Op op, T *sh) {
+    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_down_sync(0xffffffffu, v, o));
+    __syncthreads();
+    if (lane == 0) sh[wid] = v;
+    __syncthreads();
+    T r = sh[0];
+    if (threadIdx.x == 0)
+        for (int w = 1; w < (int)(blockDim.x >> 5); w++) r = op(r, sh[w]);
+    return r;
+}
+
+struct OpAddD { __device__ double operator()(double a, double b) const { return a + b; } };
+struct OpAddL { __device__ long long operator()(long long a, long long b) const { return a + b; } };
+struct OpAddI { __device__ int operator()(int a, int b) const { return a + b; } };
+struct OpMaxF { __device__ float operator()(float a, float b) const { return fmaxf(a, b); } };
+
+// The eight P2G contributions of one particle to one node
+// (StandardVarP2G x3, ComputeInternalForce + ComputeExternalForce,
+// material_point.h:223-247, solid_material_point.h:48-73).
+template <typename R>
+__device__ __forceinline__ void p2g_terms(R N, R d0, R d1, R d2, R m, R vol, const R *v, const R *s, R mfx, R mfy,
+                                          R mfz, R *q) {
+    const R Nm = N * m;
+    q[0] = Nm;
+    q[1] = N * vol;
+    q[2] = Nm * v[0];
+    q[3] = Nm * v[1];
+    q[4] = Nm * v[2];
+    q[5] = -vol * (s[0] * d0 + s[5] * d1 + s[4] * d2) + N * mfx;
+    q[6] = -vol * (s[5] * d0 + s[1] * d1 + s[3] * d2) + N * mfy;
+    q[7] = -vol * (s[4] * d0 + s[3] * d1 + s[2] * d2) + N * mfz;
+}
+
+template <typename R>
+__device__ __forceinline__ void fx_terms(const R *q, const Scales &S, long long *o) {
+    o[0] = fx(q[0], S.m);
+    o[1] = fx(q[1], S.v);
+    o[2] = fx(q[2], S.p);
+    o[3] = fx(q[3], S.p);
+    o[4] = fx(q[4], S.p);
+    o[5] = fx(q[5], S.f);
+    o[6] = fx(q[6], S.f);
+    o[7] = fx(q[7], S.f);
+}
+
+__device__ __forceinline__ void brick_origin(int b, const int *nb, int &ox, int &oy, int &oz) {
+    ox = (b % nb[0]) * BRX;
+    oy = ((b / nb[0]) % nb[1]) * BRY;
+    oz = (b / (nb[0] * nb[1])) * BRZ;
+}
+
+// Control-point coordinate xyc[idx][d] along one axis (DefineCpPos,
+// module/mesh.h:32-47, on one rank: the open-knot end points of a quadratic
+// axis sit on the walls).
+template <typename R, int O>
+__device__ __forceinline__ R cp_coord(const KGeom<R> &g, int d, int idx) {
+    if (O == 1) return g.xmin[d] + g.dx[d] * (R)idx;
+    if (idx == 0) return g.xmin[d];
+    if (idx == g.nnc[d] - 1) return g.xmin[d] + g.dx[d] * (R)g.nel[d];
+    return g.xmin[d] + g.dx[d] * ((R)idx - (R)0.5);
+}
+
+// v + A (x_i - x_p): the velocity a TPIC / APIC particle carries to node i
+// (TPIC::VarP2G / APIC::VarP2G, module/map_and_interpolate.h:62-77,104-130,
+// with the coordinate read as xyc[nid][j]).
+template <typename R>
+__device__ __forceinline__ void affine_velocity(const R *v, const R *A, R d0, R d1, R d2, R *out) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) out[c] = v[c] + (A[3 * c] * d0 + A[3 * c + 1] * d1 + A[3 * c + 2] * d2);
+}
+
+// ------------------------------------------------------------- mpm_cells.cu
+// What a cell scatter sums: the eight P2G fields (plain, with the affine
+// momentum of TPIC / APIC, with the implicit solid's N m a in the force
+// fields) or the MUSL momentum (plain, affine).
+enum CellKind { CELL_P2G = 0, CELL_P2G_AFF, CELL_P2G_ACC, CELL_MUSL, CELL_MUSL_AFF };
+// The scatter of kind `kind` as per-cell register sums, then the deferred pass
+// over the particles that left their sorted cell; two launches on st.
+template <typename R>
+void launch_cell_scatter(const StepArgs<R> &a, const int *order, int kind, int nbricks, int nsm, bool pdl,
+                         cudaStream_t st);
+// The velocity gather of PIC / FLIP and sum |geup|^2, one thread per particle.
+template <typename R>
+void launch_gather(const StepArgs<R> &a, const int *order, int nsm, bool pdl, cudaStream_t st);
+
+}  // namespace mpm
