@@ -12,9 +12,9 @@
 // before one int64 fixed-point RED per node and field.  Deterministic: every
 // sum is in a fixed order.  The staging box it replaces spent its time in 64-bit
 // shared-memory atomics, one per particle, node and field.  P2G class per step,
-// staging box -> here: FP64 linear, 201,872 particles, 296 -> 136 us; FP32
+// staging box -> here: FP64 linear, 201,872 particles, 296 -> 128 us; FP32
 // B-splines, 216,000 particles, 444 -> 66 us; FP64 B-splines, 46,656 particles,
-// 643 -> 156 us; implicit FP32 linear, 1,728,000 particles, 802 -> 62 us.
+// 643 -> 146 us; implicit FP32 linear, 1,728,000 particles, 802 -> 62 us.
 //
 // FP32 B-splines form each contribution as the staging box (mpm_explicit.cu)
 // does and sum it in an unevaluated pair of FP32 numbers (two-sum: 48 bits),
@@ -27,11 +27,13 @@
 // FP64 sums, and the FP32 ones of the implicit solid on linear grids, are kept
 // in the working precision.
 //
-// On those, within a cell the weights are polynomials of the offset t in [0, 1) from its
-// lower face, with coefficients that depend on the cell alone (cell_axis): no
-// division, no search for the spline's piece.  On FP64 grids the work is bound
-// by the FP64 pipe (2 FMAs per SM and clock), so the row's products are formed
-// once and a node costs 11 FMAs.
+// On those, within a cell the weights are polynomials of the offset t in [0, 1)
+// from its lower face, with coefficients that depend on the cell alone
+// (CellAxis): no division, no search for the spline's piece.  FP64 grids are
+// bound by the FP64 pipe (2 FMAs per SM and clock; ncu: 71 % busy in the linear
+// P2G, 292 FP64 instructions per particle), so a row's products are formed once,
+// a node costs 11 FMAs, and the in-cell test reads the high words of the offsets
+// in place of 6 FP64 comparisons (135 -> 128 us).
 #include <cstdio>
 #include <cstring>
 #include <type_traits>
@@ -39,58 +41,6 @@
 #include "mpm_step.cuh"
 
 namespace mpm {
-
-// ------------------------------------------------------------ cell-local axes
-// The quadratic B-spline of MakSf (module/shape_function.cpp:52-105) inside
-// cell c of an axis with nel cells, as functions of t: node k = 0, 1, 2 has
-//   w0 = s0 (1 - t)^2, w1 = a1 t^2 + b1 t + c1, w2 = s2 t^2
-// with the open-knot pieces at the two walls.  (The pieces meet with equal
-// values and slopes, so choosing them by the cell is exact at its faces too.)
-template <typename R>
-struct QuadCoef {
-    R s0, a1, b1, c1, s2;
-};
-template <typename R>
-__device__ __forceinline__ QuadCoef<R> quad_coef(int c, int nel) {
-    const bool lo = c == 0, hi = c == nel - 1;
-    QuadCoef<R> q;
-    q.s0 = lo ? (R)1 : (R)0.5;
-    q.a1 = (lo || hi) ? (R)-1.5 : (R)-1;
-    q.b1 = lo ? (R)2 : (R)1;
-    q.c1 = lo ? (R)0 : (R)0.5;
-    q.s2 = hi ? (R)1 : (R)0.5;
-    return q;
-}
-
-// weights and derivatives of an axis' nodes at offset t of cell c
-template <typename R, int O>
-struct CellAxis;
-template <typename R>
-struct CellAxis<R, 1> {
-    R inv;
-    __device__ __forceinline__ CellAxis(int, int, R inv_dx) : inv(inv_dx) {}
-    __device__ __forceinline__ void eval(R t, R *w, R *d) const {
-        w[0] = (R)1 - t;
-        w[1] = t;
-        d[0] = -inv;
-        d[1] = inv;
-    }
-};
-template <typename R>
-struct CellAxis<R, 2> {
-    QuadCoef<R> q;
-    R inv;
-    __device__ __forceinline__ CellAxis(int c, int nel, R inv_dx) : q(quad_coef<R>(c, nel)), inv(inv_dx) {}
-    __device__ __forceinline__ void eval(R t, R *w, R *d) const {
-        const R u = (R)1 - t, su = q.s0 * u, st = q.s2 * t, at = q.a1 * t;
-        w[0] = su * u;
-        w[1] = fma(at + q.b1, t, q.c1);
-        w[2] = st * t;
-        d[0] = (R)-2 * su * inv;
-        d[1] = fma((R)2, at, q.b1) * inv;
-        d[2] = (R)2 * st * inv;
-    }
-};
 
 // one node of an axis: weight (a t + b) t + c, derivative (2 a t + b) / dx
 template <typename R, int O>
@@ -160,35 +110,15 @@ struct PieceNode<R, 1> {
     }
 };
 
-// Offset of x from the lower face of cell c, in cells.
-template <typename R>
-__device__ __forceinline__ R cell_t(R x, const KGeom<R> &g, int d, int c) {
-    return (x - (g.xmin[d] + g.dx[d] * (R)c)) * g.inv_dx[d];
-}
 // Whether x lies in cell c as cell_of decides it (the reference's
 // floor((x - xmin) / dx) in FP64).  Away from the faces the offset alone tells;
-// within 1e-9 of one (FP64; the offset's rounding is below that for a million
-// cells) cell_of does, with its division.  A point outside the grid is in none.
+// near one cell_of does, with its division.  A point outside the grid is in none.
 template <typename R>
 __device__ __forceinline__ bool in_cell_axis(R x, R t, const KGeom<R> &g, int d, int c) {
-    const R e = sizeof(R) == 8 ? (R)1e-9 : (R)1e-3;
-    if (t > e && t < (R)1 - e) return true;
-    if (!(t > -e && t < (R)1 + e)) return false;
+    if (off_faces(t)) return true;
+    if (!(t > (R)-1e-3 && t < (R)1.001)) return false;
     bool oob = false;
     return cell_of(x, g, d, oob) == c && !oob;
-}
-// cell_of without its FP64 division away from the cell faces; t the offset in that cell
-template <typename R>
-__device__ __forceinline__ int fast_cell(R x, const KGeom<R> &g, int d, R &t) {
-    int c = (int)floor((x - g.xmin[d]) * g.inv_dx[d]);
-    t = cell_t(x, g, d, c);
-    const R e = sizeof(R) == 8 ? (R)1e-9 : (R)1e-3;
-    if ((unsigned)c >= (unsigned)g.nel[d] || !(t > e && t < (R)1 - e)) {
-        bool oob = false;
-        c = cell_of(x, g, d, oob);
-        t = cell_t(x, g, d, c);
-    }
-    return c;
 }
 
 // ------------------------------------------------------------------- scatter
@@ -251,11 +181,13 @@ struct CellShape {
     static constexpr int JP = (OX == 1 && OY == 1) ? NY : 1;
     static constexpr int P = NZ * (NY / JP);              // threads per cell
     // cells of a CTA (z-slabs of a brick): as many as leave the accumulators,
-    // 8 JP NX values per thread, in registers
-    static constexpr int CELLS = P == 2 ? BRC : P == 9 && (EXACT || sizeof(R) == 8) ? BRC / 4 : BRC / 2;
+    // 8 JP NX values per thread, in registers.  FP64 B-splines: 32 cells; with 64
+    // the P2G of 46,656 particles takes 139 us in place of 146, but that of 17,472
+    // 89 in place of 51, and with 16 they take 187 and 54
+    static constexpr int CELLS = P == 2 ? BRC : P == 9 || sizeof(R) == 8 ? BRC / 4 : BRC / 2;
     static constexpr int SLABS = BRC / CELLS, BZ = BRZ / SLABS;
     static constexpr int THREADS = CELLS * P;
-    static constexpr int MINB = EXACT ? 2 : 1;
+    static constexpr int MINB = (EXACT || P == 2) ? 2 : 1;   // CTAs per SM to compile for
     static constexpr int BX = BRX + OX, BY = BRY + OY, BZN = BZ + OZ, BOX = BX * BY * BZN;
     static constexpr int FR = 4 / W;                      // sums per round of the node pass
     static constexpr size_t SMEM = sizeof(Sum) * FR * NE * CELLS;
@@ -602,10 +534,10 @@ __global__ void __launch_bounds__(256) k_cell_misses(StepArgs<R> a) {
 
 // -------------------------------------------------------------------- gather
 // PIC: v = sum N G, FLIP: v += dt sum N G; geup = 2 vol sum dN nei and the sum
-// of its squares (only when the shifting is on).  FP64 sums axis by axis (rows,
-// layers, cell): 4 FMAs per node instead of 4 weights and 6 products.
-// With the MUSL scatter it replaces one staging-box kernel: 221 -> 109 us (FP64
-// linear, 201,872 particles), 180 -> 50 us (FP32 B-splines, 216,000), 393 -> 108
+// of its squares (only when the shifting is on).  FP64 sums axis by axis
+// (cell_field).
+// With the MUSL scatter it replaces one staging-box kernel: 221 -> 99 us (FP64
+// linear, 201,872 particles), 180 -> 50 us (FP32 B-splines, 216,000), 393 -> 99
 // us (FP64 B-splines, 46,656).
 template <typename R, int OX, int OY, int OZ>
 __global__ void __launch_bounds__(256) k_gather(StepArgs<R> a) {
@@ -663,47 +595,13 @@ __global__ void __launch_bounds__(256) k_gather(StepArgs<R> a) {
                         }
                     }
         } else {
-            R t0, t1, t2;
-            const int cx = fast_cell(ld(P.x[0] + p), a.g, 0, t0), cy = fast_cell(ld(P.x[1] + p), a.g, 1, t1),
-                      cz = fast_cell(ld(P.x[2] + p), a.g, 2, t2);
-            R wx[NX], dx[NX], wy[NY], dy[NY], wz[NZ], dz[NZ];
-            CellAxis<R, OX>(cx, a.g.nel[0], a.g.inv_dx[0]).eval(t0, wx, dx);
-            CellAxis<R, OY>(cy, a.g.nel[1], a.g.inv_dx[1]).eval(t1, wy, dy);
-            CellAxis<R, OZ>(cz, a.g.nel[2], a.g.inv_dx[2]).eval(t2, wz, dz);
-            const size_t b0 = node_id(a.g, cx, cy, cz);
+            const R x[3] = {ld(P.x[0] + p), ld(P.x[1] + p), ld(P.x[2] + p)};
+            CellWeights<R, OX, OY, OZ> w;
+            const size_t b0 = cell_weights(a.g, x, w);
 #pragma unroll
-            for (int k = 0; k < NZ; k++) {
-                R bv[3] = {(R)0, (R)0, (R)0}, e0 = (R)0, ex = (R)0, ey = (R)0;
-#pragma unroll
-                for (int j = 0; j < NY; j++) {
-                    const size_t b = b0 + j * sy + k * sz;
-                    R r[3] = {(R)0, (R)0, (R)0}, ew = (R)0, ed = (R)0;
-#pragma unroll
-                    for (int i = 0; i < NX; i++) {
-#pragma unroll
-                        for (int c = 0; c < 3; c++) r[c] = fma(wx[i], ld(a.G + c * N + b + i), r[c]);
-                        if (shift) {
-                            const R e = ld(a.nei + b + i);
-                            ew = fma(wx[i], e, ew);
-                            ed = fma(dx[i], e, ed);
-                        }
-                    }
-#pragma unroll
-                    for (int c = 0; c < 3; c++) bv[c] = fma(wy[j], r[c], bv[c]);
-                    if (shift) {
-                        e0 = fma(wy[j], ew, e0);
-                        ex = fma(wy[j], ed, ex);
-                        ey = fma(dy[j], ew, ey);
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < 3; c++) v[c] = fma(wz[k], bv[c], v[c]);
-                if (shift) {
-                    gu[0] = fma(wz[k], ex, gu[0]);
-                    gu[1] = fma(wz[k], ey, gu[1]);
-                    gu[2] = fma(dz[k], e0, gu[2]);
-                }
-            }
+            for (int c = 0; c < 3; c++) cell_field<true, false>(a.G + c * N, b0, sy, sz, w, v[c], gu);
+            R none;
+            if (shift) cell_field<false, true>(a.nei, b0, sy, sz, w, none, gu);
 #pragma unroll
             for (int c = 0; c < 3; c++)
                 if (flip) v[c] = fma(a.dt, v[c], ld(P.v[c] + p));

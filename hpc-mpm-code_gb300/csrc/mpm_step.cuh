@@ -190,6 +190,133 @@ __device__ __forceinline__ void affine_velocity(const R *v, const R *A, R d0, R 
     for (int c = 0; c < 3; c++) out[c] = v[c] + (A[3 * c] * d0 + A[3 * c + 1] * d1 + A[3 * c + 2] * d2);
 }
 
+// ------------------------------------------------------------ cell-local axes
+// The quadratic B-spline of MakSf (module/shape_function.cpp:52-105) inside
+// cell c of an axis with nel cells, as functions of t: node k = 0, 1, 2 has
+//   w0 = s0 (1 - t)^2, w1 = a1 t^2 + b1 t + c1, w2 = s2 t^2
+// with the open-knot pieces at the two walls.  (The pieces meet with equal
+// values and slopes, so choosing them by the cell is exact at its faces too.)
+template <typename R>
+struct QuadCoef {
+    R s0, a1, b1, c1, s2;
+};
+template <typename R>
+__device__ __forceinline__ QuadCoef<R> quad_coef(int c, int nel) {
+    const bool lo = c == 0, hi = c == nel - 1;
+    QuadCoef<R> q;
+    q.s0 = lo ? (R)1 : (R)0.5;
+    q.a1 = (lo || hi) ? (R)-1.5 : (R)-1;
+    q.b1 = lo ? (R)2 : (R)1;
+    q.c1 = lo ? (R)0 : (R)0.5;
+    q.s2 = hi ? (R)1 : (R)0.5;
+    return q;
+}
+
+// weights and derivatives of an axis' nodes at offset t of cell c
+template <typename R, int O>
+struct CellAxis;
+template <typename R>
+struct CellAxis<R, 1> {
+    R inv;
+    __device__ __forceinline__ CellAxis(int, int, R inv_dx) : inv(inv_dx) {}
+    __device__ __forceinline__ void eval(R t, R *w, R *d) const {
+        w[0] = (R)1 - t;
+        w[1] = t;
+        d[0] = -inv;
+        d[1] = inv;
+    }
+};
+template <typename R>
+struct CellAxis<R, 2> {
+    QuadCoef<R> q;
+    R inv;
+    __device__ __forceinline__ CellAxis(int c, int nel, R inv_dx) : q(quad_coef<R>(c, nel)), inv(inv_dx) {}
+    __device__ __forceinline__ void eval(R t, R *w, R *d) const {
+        const R u = (R)1 - t, su = q.s0 * u, st = q.s2 * t, at = q.a1 * t;
+        w[0] = su * u;
+        w[1] = fma(at + q.b1, t, q.c1);
+        w[2] = st * t;
+        d[0] = (R)-2 * su * inv;
+        d[1] = fma((R)2, at, q.b1) * inv;
+        d[2] = (R)2 * st * inv;
+    }
+};
+
+// Offset of x from the lower face of cell c, in cells.
+template <typename R>
+__device__ __forceinline__ R cell_t(R x, const KGeom<R> &g, int d, int c) {
+    return (x - (g.xmin[d] + g.dx[d] * (R)c)) * g.inv_dx[d];
+}
+// Whether an offset lies inside (0, 1) and farther from its ends than rounding
+// can move it (FP64: 1e-9 and 1e-6, above the rounding of the offset up to a
+// million cells; the test reads the high words of the numbers, since an FP64
+// comparison takes a slot of the FP64 pipe).
+__device__ __forceinline__ bool off_faces(float t) { return t > 1e-3f && t < 0.999f; }
+__device__ __forceinline__ bool off_faces(double t) {
+    const unsigned hi = (unsigned)__double2hiint(t);   // a negative t, an infinity and a NaN are above 1
+    return hi > 0x3E112E0Bu && hi < 0x3FEFFFFFu;       // 1e-9 and 1 - 2^-20
+}
+// cell_of without its FP64 division away from the cell faces (a guess from FP32
+// arithmetic, which the offset confirms); t the offset in that cell
+template <typename R>
+__device__ __forceinline__ int fast_cell(R x, const KGeom<R> &g, int d, R &t) {
+    int c = __float2int_rd((float)(x - g.xmin[d]) * (float)g.inv_dx[d]);
+    t = cell_t(x, g, d, c);
+    if ((unsigned)c >= (unsigned)g.nel[d] || !off_faces(t)) {
+        bool oob = false;
+        c = cell_of(x, g, d, oob);
+        t = cell_t(x, g, d, c);
+    }
+    return c;
+}
+
+// sum_n N_n f_n (VAL) and sum_n dN_n/dx f_n (GRAD) of a nodal field over a cell's
+// nodes (b0 the first, sy and sz the strides), summed axis by axis: rows, layers,
+// cell.  36 FMAs for value and gradient of a linear cell where weights and
+// products node by node take about 100.
+template <typename R, int OX, int OY, int OZ>
+struct CellWeights {
+    R wx[OX + 1], dx[OX + 1], wy[OY + 1], dy[OY + 1], wz[OZ + 1], dz[OZ + 1];
+};
+template <bool VAL, bool GRAD, typename R, int OX, int OY, int OZ>
+__device__ __forceinline__ void cell_field(const R *f, size_t b0, size_t sy, size_t sz,
+                                           const CellWeights<R, OX, OY, OZ> &w, R &val, R *g) {
+    R v = (R)0, gx = (R)0, gy = (R)0, gz = (R)0;
+#pragma unroll
+    for (int k = 0; k <= OZ; k++) {
+        R l = (R)0, lx = (R)0, ly = (R)0;
+#pragma unroll
+        for (int j = 0; j <= OY; j++) {
+            R r = (R)0, rx = (R)0;
+#pragma unroll
+            for (int i = 0; i <= OX; i++) {
+                const R q = ld(f + b0 + i + j * sy + k * sz);
+                r = fma(w.wx[i], q, r);
+                if (GRAD) rx = fma(w.dx[i], q, rx);
+            }
+            l = fma(w.wy[j], r, l);
+            if (GRAD) lx = fma(w.wy[j], rx, lx);
+            if (GRAD) ly = fma(w.dy[j], r, ly);
+        }
+        if (VAL) v = fma(w.wz[k], l, v);
+        if (GRAD) gx = fma(w.wz[k], lx, gx);
+        if (GRAD) gy = fma(w.wz[k], ly, gy);
+        if (GRAD) gz = fma(w.dz[k], l, gz);
+    }
+    if (VAL) val = v;
+    if (GRAD) g[0] = gx, g[1] = gy, g[2] = gz;
+}
+// the cell of a point, its node weights and its first node
+template <typename R, int OX, int OY, int OZ>
+__device__ __forceinline__ size_t cell_weights(const KGeom<R> &g, const R *x, CellWeights<R, OX, OY, OZ> &w) {
+    R t0, t1, t2;
+    const int cx = fast_cell(x[0], g, 0, t0), cy = fast_cell(x[1], g, 1, t1), cz = fast_cell(x[2], g, 2, t2);
+    CellAxis<R, OX>(cx, g.nel[0], g.inv_dx[0]).eval(t0, w.wx, w.dx);
+    CellAxis<R, OY>(cy, g.nel[1], g.inv_dx[1]).eval(t1, w.wy, w.dy);
+    CellAxis<R, OZ>(cz, g.nel[2], g.inv_dx[2]).eval(t2, w.wz, w.dz);
+    return node_id(g, cx, cy, cz);
+}
+
 // ------------------------------------------------------------- mpm_cells.cu
 // What a cell scatter sums: the eight P2G fields (plain, with the affine
 // momentum of TPIC / APIC, with the implicit solid's N m a in the force
