@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(CellShape<R, OX, OY, OZ>::THREADS, CellShape<R
     Sum *corner = reinterpret_cast<Sum *>(cell_smem);   // [FR][NE][CELLS]
     __shared__ Scales S;
     if (MUSL) load_scales_musl(a, S);
-    else load_scales(a, S);
+    else p2g_scales(a, S);   // read after the first barrier of a slab
     const int lc = threadIdx.x / P, part = threadIdx.x % P;
     const int kk = part % C::NZ, j0 = (part / C::NZ) * JP;
     const Particles<R> &Q = a.P;

@@ -173,10 +173,12 @@ __device__ __forceinline__ bool box_node_cells(const KGeom<float> &g, int n, int
 // The counters of the cell-P2G kernels: particles that left their sorted cell
 // and particles outside the grid.
 __device__ __forceinline__ void p2g_counters(const StepArgs<float> &a, int *sh_red, int misses, int oobs) {
-    int tot = block_reduce(misses + (oobs << 16), OpAddI(), sh_red);
-    if (threadIdx.x == 0 && tot) {
-        if (tot & 0xffff) atomicAdd(&a.ctl->tile_misses, (unsigned)(tot & 0xffff));
-        if (tot >> 16) atomicAdd(&a.ctl->err_oob, (unsigned)(tot >> 16));
+    // most CTAs have neither: one vote instead of two reductions
+    if (!__syncthreads_or(misses | oobs)) return;
+    const int nm = block_reduce(misses, OpAddI(), sh_red), no = block_reduce(oobs, OpAddI(), sh_red);
+    if (threadIdx.x == 0) {
+        if (nm) atomicAdd(&a.ctl->tile_misses, (unsigned)nm);
+        if (no) atomicAdd(&a.ctl->err_oob, (unsigned)no);
     }
 }
 
@@ -258,6 +260,49 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_p2g_cell(StepArgs<float>
                           ld(P.vol + p), v, s, fxg, fyg, fzg, acc, misses, oobs, p, A);
     }
     p2g_node_pass(a, S, corner, sh_red, lc, h, ox, oy, oz, acc, misses, oobs);
+}
+
+// One corner (i, j, h) = (e & 1, e >> 1 & 1, e >> 2) of a particle that left its
+// sorted cell: the terms of p2g_particle's scatter path.  Counts a particle
+// outside the grid once.
+template <bool AFF = false>
+__device__ __forceinline__ void p2g_miss(const StepArgs<float> &a, const Scales &S, int p, int e, int &oobs) {
+    const Particles<float> &P = a.P;
+    const float fxg = a.grav[0] * a.facl, fyg = a.grav[1] * a.facl, fzg = a.grav[2] * a.facl;
+    const int ci = e & 1, cj = (e >> 1) & 1, h = (e >> 2) & 1;
+    const float x0 = ld(P.x[0] + p), x1 = ld(P.x[1] + p), x2 = ld(P.x[2] + p), m = ld(P.m + p), vol = ld(P.vol + p);
+    const float vel[3] = {ld(P.v[0] + p), ld(P.v[1] + p), ld(P.v[2] + p)};
+    const float sg[6] = {ld(P.s[0] + p), ld(P.s[1] + p), ld(P.s[2] + p),
+                         ld(P.s[3] + p), ld(P.s[4] + p), ld(P.s[5] + p)};
+    bool oob = false;
+    const int px = cell_of(x0, a.g, 0, oob), py = cell_of(x1, a.g, 1, oob), pz = cell_of(x2, a.g, 2, oob);
+    oobs += oob && e == 0;
+    Axis<float, 1> ax, ay, az;
+    axis_eval<float, 1>(x0, a.g, 0, px, ax);
+    axis_eval<float, 1>(x1, a.g, 1, py, ay);
+    axis_eval<float, 1>(x2, a.g, 2, pz, az);
+    const float mfx = m * fxg, mfy = m * fyg, mfz = m * fzg;
+    const float wx = ci ? ax.w[1] : ax.w[0], dwx = ci ? ax.dw[1] : ax.dw[0];
+    const float wy = cj ? ay.w[1] : ay.w[0], dwy = cj ? ay.dw[1] : ay.dw[0];
+    const float wz = h ? az.w[1] : az.w[0], dwz = h ? az.dw[1] : az.dw[0];
+    const float wxy = wx * wy;
+    float vn[3] = {vel[0], vel[1], vel[2]};
+    if constexpr (AFF) {
+        float A[9];
+#pragma unroll
+        for (int q = 0; q < 9; q++) A[q] = ld(P.C[q] + p);
+        affine_velocity(vel, A, cp_coord<float, 1>(a.g, 0, px + ci) - x0, cp_coord<float, 1>(a.g, 1, py + cj) - x1,
+                        cp_coord<float, 1>(a.g, 2, pz + h) - x2, vn);
+    }
+    float q[NACC];
+    p2g_terms(wxy * wz, dwx * wy * wz, wx * dwy * wz, wxy * dwz, m, vol, vn, sg, mfx, mfy, mfz, q);
+    long long o[NACC];
+    fx_terms(q, S, o);
+    const size_t gn = node_id(a.g, px + ci, py + cj, pz + h);
+#pragma unroll
+    for (int f = 0; f < NACC; f++)
+        if (o[f]) atomic_add_i64(&a.acc[(size_t)f * a.g.nodec + gn], o[f]);
+    a.tileflag[tile_of_node(a.g, px + ci, py + cj, pz + h)] = 1;
 }
 
 // P2G in moment form.  Within a cell the linear weights are products of
@@ -343,7 +388,11 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_p2g_cell_mom(StepArgs<fl
     __shared__ float corner[NACC * 8][BRC];       // 32 KB
     __shared__ Scales S;
     __shared__ int sh_red[32];
-    load_scales(a, S);
+    __shared__ int n_miss[2];   // the brick's queue length, alternating
+    if (threadIdx.x == 0) n_miss[0] = 0;
+    int qi = 0;
+    p2g_scales(a, S);
+    __syncthreads();   // the queue length (the scales are read after a brick's barrier)
     int misses = 0, oobs = 0;   // over all of this CTA's bricks
     const int nbl = LIST ? *a.nblist : 1;
     for (int li = LIST ? (int)blockIdx.x : 0; li < nbl; li += LIST ? (int)gridDim.x : 1) {
@@ -381,13 +430,13 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_p2g_cell_mom(StepArgs<fl
             const float x0 = in.x[0], x1 = in.x[1], x2 = in.x[2], m = in.m, vol = in.vol;
             const float *vel = in.v, *sg = in.s;
             // offsets from the sorted cell's centre; a particle outside that
-            // cell (or outside the grid, or not finite) scatters in the
-            // deferred pass, which also counts the ones outside the grid
+            // cell (or outside the grid, or not finite) is queued in the
+            // brick's own range of a.miss and scatters after the cell sums
             const float u = cell_offset_u(x0, a.g, 0, cx), v = cell_offset_u(x1, a.g, 1, cy),
                         w = cell_offset_u(x2, a.g, 2, cz);
             if (!in_cell(u, v, w)) {
                 misses++;
-                a.miss[atomicAdd(&a.ctl->n_miss_p2g, 1u)] = p;
+                a.miss[cs[0] + atomicAdd(&n_miss[qi], 1)] = p;
                 continue;
             }
             const float uv = u * v, uw = u * w, vw = v * w;
@@ -425,8 +474,14 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_p2g_cell_mom(StepArgs<fl
         for (int ax = 0; ax < 3; ax++)
 #pragma unroll
             for (int c = 0; c < 4; c++) acc[5 + ax][c] = fmaf(acc[0][c], gv[ax], -T[ax][c]);
+        if (threadIdx.x == 0) n_miss[qi ^ 1] = 0;   // before the node pass's barrier
         p2g_node_pass<false>(a, S, corner, sh_red, lc, h, ox, oy, oz, acc, misses, oobs);
+        // the brick's queue, eight threads per particle (a launch of its own for the
+        // queues of all bricks cost 3 us per step, empty or not)
+        const int nm = n_miss[qi];
+        for (int g = threadIdx.x; g < 8 * nm; g += CELL_THREADS) p2g_miss(a, S, a.miss[cs[0] + (g >> 3)], g & 7, oobs);
         __syncthreads();   // shared memory is reused by the next brick
+        qi ^= 1;
     }
     p2g_counters(a, sh_red, misses, oobs);
 }
@@ -885,6 +940,68 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_cell(StepArgs<f
     }
 }
 
+// Corner e of a particle that left its sorted cell: every one of its eight
+// threads (consecutive lanes) gathers the particle's velocity, corner 0 writes it
+// and the shifting sums, and each re-projects its own corner.
+__device__ __forceinline__ void musl_miss(const StepArgs<float> &a, const Scales &S, int p, int e, long long &gacc,
+                                          float &vmax) {
+    const size_t N = (size_t)a.g.nodec;
+    const bool flip = (a.scheme == MPM_FLIP);
+    const Particles<float> &P = a.P;
+    const float x0 = ld(P.x[0] + p), x1 = ld(P.x[1] + p), x2 = ld(P.x[2] + p);
+    const float m = ld(P.m + p), vol = ld(P.vol + p);
+    bool oob = false;
+    const int px = cell_of(x0, a.g, 0, oob), py = cell_of(x1, a.g, 1, oob), pz = cell_of(x2, a.g, 2, oob);
+    Axis<float, 1> ax, ay, az;
+    axis_eval<float, 1>(x0, a.g, 0, px, ax);
+    axis_eval<float, 1>(x1, a.g, 1, py, ay);
+    axis_eval<float, 1>(x2, a.g, 2, pz, az);
+    float v[3] = {0.0f, 0.0f, 0.0f}, gu[3] = {0.0f, 0.0f, 0.0f}, ws = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int ii = 0; ii < 2; ii++) {
+                const size_t gn = node_id(a.g, px + ii, py + j, pz + k);
+                const float wxy = ax.w[ii] * ay.w[j];
+                const float N_ = wxy * az.w[k];
+                const float wv = flip ? N_ * a.dt : N_;
+                const float en = ld(a.nei + gn);
+                ws += N_;
+#pragma unroll
+                for (int d = 0; d < 3; d++) v[d] += wv * ld(a.G + d * N + gn);
+                gu[0] += ax.dw[ii] * ay.w[j] * az.w[k] * en;
+                gu[1] += ax.w[ii] * ay.dw[j] * az.w[k] * en;
+                gu[2] += wxy * az.dw[k] * en;
+            }
+    const float rw = a.gnorm ? rcp_approx(ws) : 1.0f;   // divided by the weights it used, as musl_particle
+#pragma unroll
+    for (int d = 0; d < 3; d++) v[d] *= rw;
+    if (flip) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) v[d] += P.v[d][p];
+        __syncwarp(0xFFu << ((threadIdx.x & 31) & ~7u));   // read by all eight before corner 0 writes
+    }
+    if (e == 0) {
+        P.v[0][p] = v[0];
+        P.v[1][p] = v[1];
+        P.v[2][p] = v[2];
+        vmax = fmaxf(vmax, fmaxf(fabsf(v[0]), fmaxf(fabsf(v[1]), fabsf(v[2]))));
+        const float tv = 2.0f * vol;
+        const float g0 = gu[0] * tv, g1 = gu[1] * tv, g2 = gu[2] * tv;
+        gacc += fx(g0 * g0 + g1 * g1 + g2 * g2, S.gd);
+    }
+    const int ci = e & 1, cj = (e >> 1) & 1, h = (e >> 2) & 1;
+    const float Nm = (ci ? ax.w[1] : ax.w[0]) * (cj ? ay.w[1] : ay.w[0]) * (h ? az.w[1] : az.w[0]) * m;
+    const size_t gn = node_id(a.g, px + ci, py + cj, pz + h);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const long long q = fx(Nm * v[d], S.q);
+        if (q) atomic_add_i64(&a.acc2[d * N + gn], q);
+    }
+}
+
 // Gather + MUSL in moment form.  Inside one cell the linear interpolant of a
 // nodal field is a trilinear polynomial in the particle's offset (u, v, w)
 // from the cell centre (u in [-1/2, 1/2], as in k_p2g_cell_mom).  Each lane of
@@ -958,6 +1075,9 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_mom(StepArgs<fl
     __shared__ Scales S;
     __shared__ long long sh_l[32];
     __shared__ float sh_f[32];
+    __shared__ int n_miss[2];   // the brick's queue length, alternating
+    if (threadIdx.x == 0) n_miss[0] = 0;
+    int qi = 0;
     load_scales_musl(a, S);
     const int nbl = LIST ? *a.nblist : 1;
     const bool flip = (a.scheme == MPM_FLIP);
@@ -1010,8 +1130,8 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_mom(StepArgs<fl
             const float u = cell_offset_u(x0, a.g, 0, cx), v = cell_offset_u(x1, a.g, 1, cy),
                         w = cell_offset_u(x2, a.g, 2, cz);
             if (!in_cell(u, v, w)) {
-                // a particle outside its sorted cell: the deferred pass (k_musl_misses)
-                a.miss[atomicAdd(&a.ctl->n_miss_musl, 1u)] = p;
+                // a particle outside its sorted cell: queued as in k_p2g_cell_mom
+                a.miss[cs[0] + atomicAdd(&n_miss[qi], 1)] = p;
                 continue;
             }
             const float uv = u * v, uw = u * w, vw = v * w, uvw = uv * w;
@@ -1043,8 +1163,13 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_mom(StepArgs<fl
             for (int k = 0; k < 8; k++) M[d][k] += __shfl_xor_sync(pair, M[d][k], 1);
             moments_to_layer(M[d], h, acc[d]);
         }
+        if (threadIdx.x == 0) n_miss[qi ^ 1] = 0;   // before the node pass's barrier
         musl_node_pass<false>(a, S, corner, sh_l, sh_f, lc, h, ox, oy, oz, acc, gacc, vmax);
+        const int nm = n_miss[qi];
+        for (int g = threadIdx.x; g < 8 * nm; g += CELL_THREADS)
+            musl_miss(a, S, a.miss[cs[0] + (g >> 3)], g & 7, gacc, vmax);
         __syncthreads();   // shared memory is reused by the next brick
+        qi ^= 1;
     }
     musl_counters(a, sh_l, sh_f, gacc, vmax);
 }
@@ -1325,10 +1450,10 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_cell_staged(Ste
     musl_node_pass(a, S, corner, sh_l, sh_f, lc, h, ox, oy, oz, acc, gacc, vmax);
 }
 
-// Deferred passes for the particles that left their sorted cell since the
-// last re-sort: fixed-point atomics (order independent, so the results do
-// not depend on the queue order); the P2G with eight threads per queued
-// particle, the gather + MUSL with one.
+// Deferred passes of the corner-form kernels for the particles that left their
+// sorted cell since the last re-sort (the moment forms take theirs brick by
+// brick): fixed-point atomics (order independent, so the results do not depend
+// on the queue order), eight threads per queued particle, one per corner.
 template <bool AFF = false>
 __global__ void __launch_bounds__(256) k_p2g_misses(StepArgs<float> a) {
     pdl_wait();
@@ -1336,52 +1461,10 @@ __global__ void __launch_bounds__(256) k_p2g_misses(StepArgs<float> a) {
     __shared__ int sh_red[32];
     load_scales(a, S);
     const unsigned n = a.ctl->n_miss_p2g;
-    const float fxg = a.grav[0] * a.facl, fyg = a.grav[1] * a.facl, fzg = a.grav[2] * a.facl;
-    const Particles<float> &P = a.P;
     int oobs = 0;
-    // eight threads per deferred particle, one per corner (i, j, h): the
-    // corner's terms are those of p2g_particle's scatter path, and the int64
-    // sums make the result independent of which thread adds them
     for (size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x; g < 8 * (size_t)n;
-         g += (size_t)gridDim.x * blockDim.x) {
-        const int p = a.miss[g >> 3];
-        const int ci = g & 1, cj = (g >> 1) & 1, h = (g >> 2) & 1;
-        const float x0 = ld(P.x[0] + p), x1 = ld(P.x[1] + p), x2 = ld(P.x[2] + p), m = ld(P.m + p),
-                    vol = ld(P.vol + p);
-        const float vel[3] = {ld(P.v[0] + p), ld(P.v[1] + p), ld(P.v[2] + p)};
-        const float sg[6] = {ld(P.s[0] + p), ld(P.s[1] + p), ld(P.s[2] + p),
-                             ld(P.s[3] + p), ld(P.s[4] + p), ld(P.s[5] + p)};
-        bool oob = false;
-        const int px = cell_of(x0, a.g, 0, oob), py = cell_of(x1, a.g, 1, oob), pz = cell_of(x2, a.g, 2, oob);
-        oobs += oob && (g & 7) == 0;
-        Axis<float, 1> ax, ay, az;
-        axis_eval<float, 1>(x0, a.g, 0, px, ax);
-        axis_eval<float, 1>(x1, a.g, 1, py, ay);
-        axis_eval<float, 1>(x2, a.g, 2, pz, az);
-        const float mfx = m * fxg, mfy = m * fyg, mfz = m * fzg;
-        const float wz = h ? az.w[1] : az.w[0], dwz = h ? az.dw[1] : az.dw[0];
-        const float wxy = ax.w[ci] * ay.w[cj];
-        float vn[3] = {vel[0], vel[1], vel[2]};
-        if constexpr (AFF) {
-            float A[9];
-#pragma unroll
-            for (int e = 0; e < 9; e++) A[e] = ld(P.C[e] + p);
-            affine_velocity(vel, A, cp_coord<float, 1>(a.g, 0, px + ci) - x0, cp_coord<float, 1>(a.g, 1, py + cj) - x1,
-                            cp_coord<float, 1>(a.g, 2, pz + h) - x2, vn);
-        }
-        float q[NACC];
-        p2g_terms(wxy * wz, ax.dw[ci] * ay.w[cj] * wz, ax.w[ci] * ay.dw[cj] * wz, wxy * dwz, m, vol, vn, sg, mfx, mfy,
-                  mfz, q);
-        long long o[NACC];
-        fx_terms(q, S, o);
-        const size_t gn = node_id(a.g, px + ci, py + cj, pz + h);
-#pragma unroll
-        for (int f = 0; f < NACC; f++)
-            if (o[f]) atomic_add_i64(&a.acc[(size_t)f * a.g.nodec + gn], o[f]);
-        a.tileflag[tile_of_node(a.g, px + ci, py + cj, pz + h)] = 1;
-    }
-    // the particles outside the grid (every one of them is deferred by the
-    // moment-form P2G)
+         g += (size_t)gridDim.x * blockDim.x)
+        p2g_miss<AFF>(a, S, a.miss[g >> 3], (int)(g & 7), oobs);
     const int tot = block_reduce(oobs, OpAddI(), sh_red);
     if (threadIdx.x == 0 && tot) atomicAdd(&a.ctl->err_oob, (unsigned)tot);
 }
@@ -1393,88 +1476,28 @@ __global__ void __launch_bounds__(256) k_musl_misses(StepArgs<float> a) {
     __shared__ float sh_f[32];
     load_scales_musl(a, S);
     const unsigned n = a.ctl->n_miss_musl;
-    const size_t N = (size_t)a.g.nodec;
-    const bool flip = (a.scheme == MPM_FLIP);
-    const Particles<float> &P = a.P;
     long long gacc = 0;
     float vmax = 0.0f;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int p = a.miss[i];
-        const float x0 = ld(P.x[0] + p), x1 = ld(P.x[1] + p), x2 = ld(P.x[2] + p);
-        const float m = ld(P.m + p), vol = ld(P.vol + p);
-        bool oob = false;
-        const int px = cell_of(x0, a.g, 0, oob), py = cell_of(x1, a.g, 1, oob), pz = cell_of(x2, a.g, 2, oob);
-        Axis<float, 1> ax, ay, az;
-        axis_eval<float, 1>(x0, a.g, 0, px, ax);
-        axis_eval<float, 1>(x1, a.g, 1, py, ay);
-        axis_eval<float, 1>(x2, a.g, 2, pz, az);
-        float v[3] = {0.0f, 0.0f, 0.0f}, gu[3] = {0.0f, 0.0f, 0.0f}, ws = 0.0f;
-        for (int k = 0; k < 2; k++)
-            for (int j = 0; j < 2; j++)
-                for (int ii = 0; ii < 2; ii++) {
-                    const size_t gn = node_id(a.g, px + ii, py + j, pz + k);
-                    const float wxy = ax.w[ii] * ay.w[j];
-                    const float N_ = wxy * az.w[k];
-                    const float wv = flip ? N_ * a.dt : N_;
-                    const float e = ld(a.nei + gn);
-                    ws += N_;
-#pragma unroll
-                    for (int d = 0; d < 3; d++) v[d] += wv * ld(a.G + d * N + gn);
-                    gu[0] += ax.dw[ii] * ay.w[j] * az.w[k] * e;
-                    gu[1] += ax.w[ii] * ay.dw[j] * az.w[k] * e;
-                    gu[2] += wxy * az.dw[k] * e;
-                }
-        const float rw = a.gnorm ? rcp_approx(ws) : 1.0f;   // divided by the weights it used, as musl_particle
-#pragma unroll
-        for (int d = 0; d < 3; d++) v[d] *= rw;
-        if (flip) {
-#pragma unroll
-            for (int d = 0; d < 3; d++) v[d] += ld(P.v[d] + p);
-        }
-        P.v[0][p] = v[0];
-        P.v[1][p] = v[1];
-        P.v[2][p] = v[2];
-        vmax = fmaxf(vmax, fmaxf(fabsf(v[0]), fmaxf(fabsf(v[1]), fabsf(v[2]))));
-        const float tv = 2.0f * vol;
-        const float g0 = gu[0] * tv, g1 = gu[1] * tv, g2 = gu[2] * tv;
-        gacc += fx(g0 * g0 + g1 * g1 + g2 * g2, S.gd);
-        for (int k = 0; k < 2; k++)
-            for (int j = 0; j < 2; j++)
-                for (int ii = 0; ii < 2; ii++) {
-                    const float Nm = ax.w[ii] * ay.w[j] * az.w[k] * m;
-                    const size_t gn = node_id(a.g, px + ii, py + j, pz + k);
-                    for (int d = 0; d < 3; d++) {
-                        const long long q = fx(Nm * v[d], S.q);
-                        if (q) atomic_add_i64(&a.acc2[d * N + gn], q);
-                    }
-                }
-    }
-    const long long gsum = block_reduce(gacc, OpAddL(), sh_l);
-    const float vm = block_reduce(vmax, OpMaxF(), sh_f);
-    if (threadIdx.x == 0) {
-        if (gsum) atomicAdd(&a.ctl->geup_acc, (unsigned long long)gsum);
-        if (vm > 0.0f) atomic_max_pos(&a.ctl->nxt[a.parity ^ 1][B_VMAX], vm * 1.000001f);
-    }
+    for (size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x; g < 8 * (size_t)n;
+         g += (size_t)gridDim.x * blockDim.x)
+        musl_miss(a, S, a.miss[g >> 3], (int)(g & 7), gacc, vmax);
+    musl_counters(a, sh_l, sh_f, gacc, vmax);
 }
 
-// Launched before the P2G of every step: records the P2G scales (for result
-// downloads) and resets the per-step device counters.
+// Starts a step whose P2G kernel does not (p2g_scales), and records the P2G scales
+// for result downloads; one warp.
 template <typename R>
 __global__ void k_step_reset(StepArgs<R> a) {
     pdl_wait();
-    Scales s;
-    compute_scales(a, s);
+    begin_step_ctl(a);
     DevCtl *ctl = a.ctl;
-    ctl->p2g_inv[0] = s.m.inv;
-    ctl->p2g_inv[1] = s.v.inv;
-    ctl->p2g_inv[2] = s.p.inv;
-    ctl->p2g_inv[3] = s.f.inv;
-    ctl->sc_p2g = s;
-    ctl->n_miss_p2g = 0u;
-    ctl->n_miss_musl = 0u;
-    for (int k = 0; k < B_NB; k++) ctl->nxt[a.parity ^ 1][k] = 0u;
-    for (int k = 0; k < C_NC; k++) ctl->cur[k] = 0u;
-    ctl->geup_acc = 0ull;
+    if (threadIdx.x < 4) {
+        const Fix f = make_fix(bound_p2g(a, a.parity, threadIdx.x));
+        (&ctl->sc_p2g.m)[threadIdx.x] = f;
+        ctl->p2g_inv[threadIdx.x] = f.inv;
+    }
+    if (threadIdx.x == 4) ctl->n_miss_p2g = 0u;
+    if (threadIdx.x == 5) ctl->n_miss_musl = 0u;
 }
 
 // ================================================= any order, staging box
@@ -2001,6 +2024,7 @@ __global__ void __launch_bounds__(256) k_affine_musl(StepArgs<R> a) {
 }
 
 // ------------------------------------------------------------ grid pass 1
+constexpr int TILE_DIRECT = 608;                             // tiles up to which no list is made
 constexpr int GRID_THREADS = 256;                            // threads of a grid-pass CTA
 constexpr int GRID_NPT = TILE * TILE * TILE / GRID_THREADS;  // nodes of a tile per thread
 static_assert(GRID_NPT * GRID_THREADS == TILE * TILE * TILE, "a grid-pass CTA covers its tile exactly");
@@ -2047,6 +2071,14 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid1(StepArgs<R> a) {
         for (int k = 0; k < GRID_NPT; k++) {
             if (!in[k]) continue;
             const size_t n = nid[k];
+            if (!a.all_tiles) {
+                // cleared for the next step here, where their values are known:
+                // an untouched node of an active tile costs no store (F-bar:
+                // k_fbar_grid reads the nvof sums first; k_grid2 reads the mass)
+#pragma unroll
+                for (int f = 1; f < NACC; f++)
+                    if (q[k][f] != 0 && !(a.fbar && f == 1)) a.acc[f * N + n] = 0ull;
+            }
             const R mass = unfx(q[k][0], S.m, (R)0);
             R vof = unfx(q[k][1], S.v, (R)0);
             R nv[3], na[3];
@@ -2113,10 +2145,11 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid1(StepArgs<R> a) {
         if (threadIdx.x == 0) {
             a.ctl->eu_norm = tot;
             a.ctl->tile_counter = 0u;
-            Scales sm;
-            compute_scales(a, sm);
-            a.ctl->sc_musl = sm;
         }
+        // the gather's scales beside the P2G's (k_grid2 reads the mass scale), one per thread
+        if (threadIdx.x < 6)
+            (&a.ctl->sc_musl.m)[threadIdx.x] =
+                threadIdx.x < 4 ? (&S.m)[threadIdx.x] : make_fix(bound_musl(a, (int)threadIdx.x - 4));
     }
 }
 
@@ -2126,6 +2159,9 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid2(StepArgs<R> a) {
     pdl_wait();
     __shared__ Scales S;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
+        // both deferred passes are over
+        a.ctl->n_miss_p2g = 0u;
+        a.ctl->n_miss_musl = 0u;
         // b0 of DeltaCorrectionParticleShifting (material_point.cpp:219)
         double gd = (double)(long long)a.ctl->geup_acc * a.ctl->sc_musl.gd.inv;
         a.ctl->b0 = (!a.shifting || gd < (double)a.mtol) ? 0.0 : a.ctl->eu_norm / gd;
@@ -2175,12 +2211,11 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid2(StepArgs<R> a) {
         }
 #pragma unroll
         for (int c = 0; c < 3; c++) a.nvel2[c * N + n] = nv[c];
-        if (!a.all_tiles) {
+        if (!a.all_tiles) {   // the sums k_grid1 left
+            if (q[k][0] != 0) a.acc[n] = 0ull;
 #pragma unroll
-            for (int f = 0; f < NACC; f++)
-                if (!(a.fbar && f == 1)) a.acc[f * N + n] = 0ull;   // F-bar: k_fbar_grid reads nvof first
-#pragma unroll
-            for (int c = 0; c < 3; c++) a.acc2[c * N + n] = 0ull;
+            for (int c = 0; c < 3; c++)
+                if (q[k][1 + c] != 0) a.acc2[c * N + n] = 0ull;
         }
     }
     if (!a.all_tiles) {
@@ -3047,6 +3082,8 @@ __global__ void __launch_bounds__(UCH, 3) k_g2p_update_tma(StepArgs<float> a, in
 }
 
 // ------------------------------------------------------------- host side
+static bool begins_itself(const mpm_ctx *c);
+
 template <typename R>
 static StepArgs<R> make_args(mpm_ctx *c) {
     StepArgs<R> a;
@@ -3124,6 +3161,7 @@ static StepArgs<R> make_args(mpm_ctx *c) {
         a.rev_g2p = a.parity ^ 1;
     }
     a.implicit = c->nreal == 27 ? 1 : 0;
+    a.begin = begins_itself(c) ? 1 : 0;
     a.nump = (double)c->num;
     a.mmax = c->mmax;
     double gs = 0.0, gsum = 0.0;
@@ -3159,6 +3197,21 @@ static int list_grid(const mpm_ctx *c, int per_sm) {
     return std::min(c->g.nbricks, per_sm * num_sms());
 }
 
+// The moment P2G and the cell scatters of a fused explicit step start the step
+// themselves (p2g_scales).  A step whose nodal sums are downloaded records its
+// scales as well, and an implicit one may repeat its P2G: k_step_reset.
+static bool begins_itself(const mpm_ctx *c) {
+    if (c->write_nodal_dl || c->nreal == 27 || !c->cell_scatter) return false;
+    const bool linear32 = c->precision == 32 && c->g.order[0] == 1;
+    return linear32 ? !c->affine && c->tune.p2g_moments && c->tune.p2g_moments != 3 : true;
+}
+
+// The grid passes walk a list of the active tiles, which takes a launch to make;
+// a grid whose tiles' CTAs are resident together (4 per SM) launches one CTA per
+// tile instead, which asks its tile's flag: 17 -> 13 us for both at 27 tiles, 24
+// -> 20 at 576, but 34 -> 54 us at 4,913 (spinning block, 128^3 cells).
+static bool use_tile_list(const mpm_ctx *c) { return !c->write_nodal_dl && c->g.ntiles > TILE_DIRECT; }
+
 // which: 0 P2G, 1 G2P + MUSL, 2 G2P update
 template <typename R, int OX, int OY, int OZ>
 static mpm_status launch_particle_kernel(mpm_ctx *c, int which) {
@@ -3166,8 +3219,10 @@ static mpm_status launch_particle_kernel(mpm_ctx *c, int which) {
     constexpr int BOX = (BRX + OX) * (BRY + OY) * (BRZ + OZ);
     if (c->num == 0) return MPM_OK;
     if (which == 0) {
-        launch(c->pdl != 0, k_step_reset<R>, 1, 1, 0, c->stream, a);
-        c->launches++;
+        if (!begins_itself(c)) {
+            launch(c->pdl != 0, k_step_reset<R>, 1, 32, 0, c->stream, a);
+            c->launches++;
+        }
         timer_begin(c, K_P2G);
         if constexpr (sizeof(R) == 4 && OX == 1 && OY == 1 && OZ == 1) {
             if (use_cell_kernels(c)) {
@@ -3199,9 +3254,13 @@ static mpm_status launch_particle_kernel(mpm_ctx *c, int which) {
                 } else {
                     k_p2g_cell<2><<<c->g.nbricks, CELL_THREADS, 0, c->stream>>>(a);
                 }
-                launch(c->pdl != 0, k_p2g_misses<false>, 2 * num_sms(), 256, 0, c->stream, a);
+                c->launches++;
+                // the moment forms scatter the particles that left their cell themselves (k_p2g_brick does not)
+                if (!c->tune.p2g_moments || c->tune.p2g_moments == 3) {
+                    launch(c->pdl != 0, k_p2g_misses<false>, 2 * num_sms(), 256, 0, c->stream, a);
+                    c->launches++;
+                }
                 timer_end(c, K_P2G);
-                c->launches += 2;
                 return check_launch(c);
             }
         }
@@ -3259,9 +3318,12 @@ static mpm_status launch_particle_kernel(mpm_ctx *c, int which) {
                 } else {
                     k_g2p_musl_cell<3, false><<<c->g.nbricks, CELL_THREADS, 0, c->stream>>>(a);
                 }
-                launch(c->pdl != 0, k_musl_misses, 2 * num_sms(), 256, 0, c->stream, a);
+                c->launches++;
+                if (!c->tune.musl_moments) {
+                    launch(c->pdl != 0, k_musl_misses, 2 * num_sms(), 256, 0, c->stream, a);
+                    c->launches++;
+                }
                 timer_end(c, K_G2P_MUSL);
-                c->launches += 2;
                 return check_launch(c);
             }
         }
@@ -3311,7 +3373,7 @@ static mpm_status launch_particle_kernel(mpm_ctx *c, int which) {
                 }
             }
             if (!cell) k_fbar_scatter<R, OX, OY, OZ><<<pg, 256, 0, c->stream>>>(a);
-            if (!a.all_tiles)
+            if (use_tile_list(c))
                 k_fbar_grid<R, true><<<std::min(c->g.ntiles, 6 * num_sms()), 256, 0, c->stream>>>(a);
             else
                 k_fbar_grid<R, false><<<c->g.ntiles, 256, 0, c->stream>>>(a);
@@ -3370,7 +3432,7 @@ static mpm_status particle_kernel(mpm_ctx *c, int which) {
 template <typename R>
 static mpm_status grid_kernel(mpm_ctx *c, int which) {
     StepArgs<R> a = make_args<R>(c);
-    const bool list = !a.all_tiles;
+    const bool list = use_tile_list(c);
     // persistent grids of as many CTAs as reside per SM: 4 for the first pass
     // (64 registers with its batched loads), 6 for the second (40)
     const int lgrid1 = std::min(c->g.ntiles, 4 * num_sms()), lgrid = std::min(c->g.ntiles, 6 * num_sms());

@@ -50,6 +50,7 @@ struct StepArgs {
     // traversal directions of the particle kernels: each starts where the
     // previous particle pass ended, so its first bricks are still in L2
     int rev_p2g, rev_g2p, rev_upd;
+    int begin;                  // the P2G kernel starts the step itself (p2g_scales), no k_step_reset before it
     double nump;                // particle count as a bound factor
     double mmax;                // max particle mass
     double gshape;              // bound on |dN/dx|
@@ -80,25 +81,47 @@ __device__ __forceinline__ size_t node_id(const KGeom<R> &g, int gx, int gy, int
 // and shared; producer and consumer kernels derive them from the same
 // device-resident bounds, so they agree exactly.
 
+// the bound of P2G scale k (0 mass, 1 volume, 2 momentum, 3 force) of the step
+// of the given parity
 template <typename R>
-__device__ void compute_scales(const StepArgs<R> &a, Scales &s) {
-    const unsigned *nb = a.ctl->nxt[a.parity];
-    double gabs = fmax(fabs((double)a.grav[0]), fmax(fabs((double)a.grav[1]), fabs((double)a.grav[2])));
-    s.m = make_fix(a.nump * a.mmax);
-    s.v = make_fix(a.nump * (double)bits_f(nb[B_VOLMAX]));
-    s.p = make_fix(a.nump * a.mmax * (double)bits_f(nb[B_VMAX]));
-    s.f = a.implicit ? make_fix(a.nump * a.mmax * (double)bits_f(nb[B_AMAX]) * 1.0000001)
-                     : make_fix(a.nump * ((double)bits_f(nb[B_VOLSMAX]) * 3.0 * a.gshape +
-                                          a.mmax * gabs * fabs((double)a.facl)));
-    double vb = (double)bits_f(a.ctl->cur[C_GMAX]);
-    if (a.scheme == MPM_FLIP) vb = (double)bits_f(nb[B_VMAX]) + fabs((double)a.dt) * vb;
-    s.q = make_fix(a.nump * a.mmax * vb * 1.0000001);
-    double gb = 2.0 * (double)bits_f(nb[B_VOLMAX]) * a.gsum * (double)bits_f(a.ctl->cur[C_NEIMAX]);
-    s.gd = make_fix(a.nump * 3.0 * gb * gb * 1.0000001);
+__device__ double bound_p2g(const StepArgs<R> &a, int parity, int k) {
+    const volatile unsigned *nb = a.ctl->nxt[parity];
+    if (k == 0) return a.nump * a.mmax;
+    if (k == 1) return a.nump * (double)bits_f(nb[B_VOLMAX]);
+    if (k == 2) return a.nump * a.mmax * (double)bits_f(nb[B_VMAX]);
+    if (a.implicit) return a.nump * a.mmax * (double)bits_f(nb[B_AMAX]) * 1.0000001;
+    const double gabs = fmax(fabs((double)a.grav[0]), fmax(fabs((double)a.grav[1]), fabs((double)a.grav[2])));
+    return a.nump * ((double)bits_f(nb[B_VOLSMAX]) * 3.0 * a.gshape + a.mmax * gabs * fabs((double)a.facl));
 }
+// the bound of the gather's scales of this step: k = 0 the MUSL momentum, 1 the
+// shifting's |geup|^2, from the grid maxima of k_grid1
+template <typename R>
+__device__ double bound_musl(const StepArgs<R> &a, int k) {
+    const unsigned *nb = a.ctl->nxt[a.parity];
+    const volatile unsigned *cur = a.ctl->cur;
+    if (k == 0) {
+        double vb = (double)bits_f(cur[C_GMAX]);
+        if (a.scheme == MPM_FLIP) vb = (double)bits_f(nb[B_VMAX]) + fabs((double)a.dt) * vb;
+        return a.nump * a.mmax * vb * 1.0000001;
+    }
+    const double gb = 2.0 * (double)bits_f(nb[B_VOLMAX]) * a.gsum * (double)bits_f(cur[C_NEIMAX]);
+    return a.nump * 3.0 * gb * gb * 1.0000001;
+}
+// What a step resets before its first kernel records anything: the per-step
+// counters and the bounds for the next step (one warp, a slot per lane).
+template <typename R>
+__device__ __forceinline__ void begin_step_ctl(const StepArgs<R> &a) {
+    DevCtl *ctl = a.ctl;
+    const int lane = threadIdx.x & 31;
+    if (lane == 6) ctl->geup_acc = 0ull;
+    else if (lane >= 8 && lane < 8 + B_NB) ctl->nxt[a.parity ^ 1][lane - 8] = 0u;
+    else if (lane >= 16 && lane < 16 + C_NC) ctl->cur[lane - 16] = 0u;
+}
+static_assert(B_NB <= 8 && C_NC <= 16, "one lane per slot");
 
-// The scales of a step are computed once: the P2G ones by k_step_reset, the
-// gather/MUSL ones by the last CTA of k_grid1 (they depend on the grid
+// The scales of a step: the P2G ones by k_step_reset or, where the P2G kernel
+// starts the step itself, by each of its CTAs; the gather/MUSL ones by the last
+// CTA of k_grid1 (they depend on the grid
 // maxima it records).  Kernels copy them into shared memory.
 template <typename R>
 __device__ __forceinline__ void load_scales_from(const Scales *src, Scales &sh) {
@@ -109,6 +132,21 @@ __device__ __forceinline__ void load_scales_from(const Scales *src, Scales &sh) 
 template <typename R>
 __device__ __forceinline__ void load_scales(const StepArgs<R> &a, Scales &sh) {
     load_scales_from<R>(&a.ctl->sc_p2g, sh);
+}
+// The P2G kernel's scales, from its first warp (the caller's next barrier
+// publishes them).  With a.begin it is the step's first kernel: every CTA derives
+// the scales from the bounds of the step before, and CTA 0 records them and
+// resets what the later kernels record.  (A one-warp kernel for this before every
+// P2G cost 3 us of a 33 us step of 8,000 particles.)
+template <typename R>
+__device__ __forceinline__ void p2g_scales(const StepArgs<R> &a, Scales &sh) {
+    if (threadIdx.x >= 32) return;
+    if (threadIdx.x < 4) {
+        const Fix f = a.begin ? make_fix(bound_p2g(a, a.parity, threadIdx.x)) : (&a.ctl->sc_p2g.m)[threadIdx.x];
+        (&sh.m)[threadIdx.x] = f;
+        if (a.begin && blockIdx.x == 0) (&a.ctl->sc_p2g.m)[threadIdx.x] = f;
+    }
+    if (a.begin && blockIdx.x == 0) begin_step_ctl(a);
 }
 template <typename R>
 __device__ __forceinline__ void load_scales_musl(const StepArgs<R> &a, Scales &sh) {
