@@ -36,6 +36,7 @@
 // products and norms, the true residual b - A x (the FP32-stored matrix
 // applied in FP64 arithmetic), the Newton check and the nodal kinematics
 // stay FP64.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstdio>
@@ -78,6 +79,7 @@ struct ImpState {
     double *gqq = nullptr, *gbeta = nullptr;  // |A p|^2 of each kept direction, projection coefficients
     float *gqf = nullptr;                   // FP32 copies of the kept images (GM * 3 * nodec), for the dots
     float *gp32 = nullptr, *gq32 = nullptr;  // FP32 operator: the directions and images in FP32 (GM * 3 * nodec)
+    float *p32 = nullptr;                   // FP32 operator: the CG direction in FP32
     float *dfx = nullptr;                   // FP32 operator: x split into high and low FP32 parts (2 * 3 * nodec)
     unsigned *cnt = nullptr;                // block counters of the single-launch reductions (zero between launches)
     int fallbacks = 0;                      // solves that switched from the network to Jacobi
@@ -95,7 +97,7 @@ namespace mpm {
 
 constexpr int GM = 8;   // directions kept by the flexible GCR solver
 
-enum Scal { S_RR0 = 0, S_RR1, S_PAP, S_RR_INIT, S_RES, S_IDOF, S_EU, S_GD, S_ZQ, S_PR, S_RRC, S_DZZ, S_DZR, S_QR, S_QQ, S_NSCAL };
+enum Scal { S_RR0 = 0, S_RR1, S_PAP, S_RR_INIT, S_RES, S_IDOF, S_EU, S_GD, S_ZQ, S_PR, S_RRC, S_DZZ, S_DZR, S_QR, S_QQ, S_THR, S_ITER, S_DONE, S_ALPHA, S_BETA, S_NSCAL };
 
 struct ImpArgs {
     int nnc[3];
@@ -667,7 +669,7 @@ __device__ __forceinline__ int warp_sums(T (&v)[V]) {
 
 template <int V>
 __device__ __forceinline__ bool partials_last(const double (&vin)[V], int nv, double *part, unsigned *cnt) {
-    __shared__ double sh[V][8];
+    __shared__ double sh[V][8];   // CTAs of at most 8 warps
     __shared__ bool s_last;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     double v[V];
@@ -709,10 +711,10 @@ __global__ void k_finish(const double *part, int nblk, double *out, int slot) {
 // FP32 operator, FP64 for its true residual and in the FP64 mode); TV: the
 // vectors x and y (FP64, or FP32 for the flexible GCR directions of the FP32
 // operator).  RX, RY, RZ: the stencil radius per axis.
-template <typename TA, typename TC, int RX, int RY, int RZ, typename TV = double>
-__global__ void __launch_bounds__(256) k_imp_matvec(ImpArgs a, const TA *A, const TV *x, TV *y,
+template <typename TA, typename TC, int RX, int RY, int RZ, typename TV = double, typename TY = TV>
+__global__ void __launch_bounds__(256) k_imp_matvec(ImpArgs a, const TA *A, const TV *x, TY *y,
                                                     double *part, unsigned *cnt = nullptr, double *scal = nullptr,
-                                                    int slot = 0) {
+                                                    int slot = 0, int num = -1, const double *xd = nullptr) {
     using TA2 = typename std::conditional<sizeof(TA) == 8, double2, float2>::type;
     constexpr int SX = 2 * RX + 1, SY = 2 * RY + 1, NS = SX * SY * (2 * RZ + 1);
     __shared__ double sh[32];
@@ -756,8 +758,9 @@ __global__ void __launch_bounds__(256) k_imp_matvec(ImpArgs a, const TA *A, cons
         const unsigned char bf = a.bcflag[n];
         for (int c = 0; c < 3; c++) {
             const double v = (bf & (1 << c)) ? 0.0 : (double)acc[c];
-            y[c * N + n] = (TV)v;
-            dot += (double)x[c * N + n] * v;
+            y[c * N + n] = (TY)v;
+            if constexpr (sizeof(TV) != sizeof(TY)) dot += xd[c * N + n] * v;   // x is a copy of xd
+            else dot += (double)x[c * N + n] * v;
         }
     }
     if (part && cnt) {   // dot(x, y) reduced by the last block into scal[slot]
@@ -766,11 +769,92 @@ __global__ void __launch_bounds__(256) k_imp_matvec(ImpArgs a, const TA *A, cons
         const double t = last_sum(part, 0, sh);
         if (threadIdx.x == 0) {
             scal[slot] = t;
+            if (num >= 0) scal[S_ALPHA] = t != 0.0 ? scal[num] / t : 0.0;
             *cnt = 0u;
         }
     } else if (part) {
         const double t = block_sum(dot, sh);
         if (threadIdx.x == 0) part[blockIdx.x] = t;
+    }
+}
+
+// The same product with MV_G threads per control point, each of SL neighbouring
+// slots (an even number, so that its entries start on a pair), added in order
+// through shared memory (mv_split says when).
+// x in the precision TV of the arithmetic's input, y in TY; with `part`, the dot
+// product of xd (FP64) and y goes to scal[slot] and scal[num] divided by it to
+// S_ALPHA (num >= 0).  `done`: nothing to do when set.
+constexpr int MV_NODES = 32, MV_G = 7;
+template <typename TA, typename TC, int RX, int RY, int RZ, typename TV, typename TY>
+__global__ void __launch_bounds__(MV_NODES * MV_G)
+    k_imp_matvec_split(ImpArgs a, const TA *__restrict__ A, const TV *__restrict__ x, TY *__restrict__ y,
+                       const double *__restrict__ xd, double *part, unsigned *cnt, double *scal, int slot, int num,
+                       const double *done) {
+    using TA2 = typename std::conditional<sizeof(TA) == 8, double2, float2>::type;
+    constexpr int SX = 2 * RX + 1, SY = 2 * RY + 1, NS = SX * SY * (2 * RZ + 1);
+    constexpr int SL = 2 * ((NS + 2 * MV_G - 1) / (2 * MV_G));
+    static_assert(SL * MV_G >= NS, "every slot has a thread");
+    __shared__ TC sh[MV_G][3][MV_NODES];
+    __shared__ double shd[32];
+    pdl_wait();
+    if (done && *done != 0.0) return;   // uniform over the grid
+    const int lane = threadIdx.x % MV_NODES, grp = threadIdx.x / MV_NODES;
+    const size_t N = (size_t)a.nodec;
+    double dot = 0.0;
+    const int n = blockIdx.x * MV_NODES + lane;
+    TC acc[3] = {(TC)0, (TC)0, (TC)0};
+    if (n < a.nodec) {
+        int i, j, k;
+        node_ijk(n, a.nnc, i, j, k);
+#pragma unroll
+        for (int q = 0; q < SL; q++) {
+            const int s = grp * SL + q;
+            const int ii = i + s % SX - RX, jj = j + (s / SX) % SY - RY, kk = k + s / (SX * SY) - RZ;
+            if (s >= NS || ii < 0 || jj < 0 || kk < 0 || ii >= a.nnc[0] || jj >= a.nnc[1] || kk >= a.nnc[2]) continue;
+            const size_t col = ii + (size_t)a.nnc[0] * (jj + (size_t)a.nnc[1] * kk);
+            const TC x0 = (TC)x[col], x1 = (TC)x[N + col], x2 = (TC)x[2 * N + col];
+            TC e[9];
+            if ((q & 1) == 0) {
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    const TA2 v = __ldg(reinterpret_cast<const TA2 *>(A + aidx(s * 9 + 2 * t, n, a.qp)));
+                    e[2 * t] = (TC)v.x;
+                    e[2 * t + 1] = (TC)v.y;
+                }
+                e[8] = (TC)__ldg(A + aidx(s * 9 + 8, n, a.qp));
+            } else {
+                e[0] = (TC)__ldg(A + aidx(s * 9, n, a.qp));
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    const TA2 v = __ldg(reinterpret_cast<const TA2 *>(A + aidx(s * 9 + 1 + 2 * t, n, a.qp)));
+                    e[1 + 2 * t] = (TC)v.x;
+                    e[2 + 2 * t] = (TC)v.y;
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 3; r++) acc[r] = fma(e[3 * r + 2], x2, fma(e[3 * r + 1], x1, fma(e[3 * r], x0, acc[r])));
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) sh[grp][c][lane] = acc[c];
+    __syncthreads();
+    if (grp < 3 && n < a.nodec) {
+        TC v = sh[0][grp][lane];
+#pragma unroll
+        for (int q = 1; q < MV_G; q++) v += sh[q][grp][lane];
+        const double r = (a.bcflag[n] & (1 << grp)) ? 0.0 : (double)v;
+        y[grp * N + n] = (TY)r;
+        if (part) dot = xd[grp * N + n] * r;
+    }
+    if (part) {
+        const double v[1] = {dot};
+        if (!partials_last<1>(v, 1, part, cnt)) return;
+        const double t = last_sum(part, 0, shd);
+        if (threadIdx.x == 0) {
+            scal[slot] = t;
+            if (num >= 0) scal[S_ALPHA] = t != 0.0 ? scal[num] / t : 0.0;
+            *cnt = 0u;
+        }
     }
 }
 
@@ -897,19 +981,35 @@ __device__ __forceinline__ double block_div(double num, double den, bool zero = 
     return s_q;
 }
 
-// x += alpha p, r -= alpha Ap, then (last block) r.r;  alpha = rr_cur / pAp
-__global__ void k_cg_update(ImpArgs a, double *scal, int cur, double *x, double *r, const double *p,
-                            const double *Ap, double *part, unsigned *cnt) {
+// x += alpha p, r -= alpha Ap, then (last block) r.r and beta;  alpha = rr_cur / pAp
+// and beta = rr_new / rr_cur are divided once, by the block that reduced them.
+// stop: the pass belongs to a solve that ends itself: nothing to do once S_DONE is
+// set, and the last block sets it when r.r is below S_THR (or not a number) and
+// counts the iteration.  Every load is issued before the first store.
+__global__ void __launch_bounds__(256) k_cg_update(ImpArgs a, double *scal, int cur, double *x, double *r,
+                                                   const double *p, const double *Ap, double *part, unsigned *cnt,
+                                                   int stop) {
     __shared__ double sh[32];
+    pdl_wait();
+    if (stop && scal[S_DONE] != 0.0) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    const double alpha = block_div(scal[cur], scal[S_PAP]);
-    double dot = 0.0;
+    const size_t N = (size_t)a.nodec;
+    double xv[3], rv[3], pv[3], qv[3];
     if (n < a.nodec) {
-        const size_t N = (size_t)a.nodec;
+#pragma unroll
         for (int c = 0; c < 3; c++) {
             const size_t i = c * N + n;
-            x[i] += alpha * p[i];
-            const double v = r[i] - alpha * Ap[i];
+            xv[c] = x[i], rv[c] = r[i], pv[c] = p[i], qv[c] = Ap[i];
+        }
+    }
+    const double alpha = scal[S_ALPHA];
+    double dot = 0.0;
+    if (n < a.nodec) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const size_t i = c * N + n;
+            x[i] = xv[c] + alpha * pv[c];
+            const double v = rv[c] - alpha * qv[c];
             r[i] = v;
             dot += v * v;
         }
@@ -919,20 +1019,49 @@ __global__ void k_cg_update(ImpArgs a, double *scal, int cur, double *x, double 
     const double t = last_sum(part, 0, sh);
     if (threadIdx.x == 0) {
         scal[cur ^ 1] = t;
+        scal[S_BETA] = scal[cur] != 0.0 ? t / scal[cur] : 0.0;
         *cnt = 0u;
+        if (stop) {
+            scal[S_ITER] += 1.0;
+            if (!(t >= scal[S_THR])) scal[S_DONE] = 1.0;
+        }
     }
 }
 
-// p = r + beta p;  beta = rr_new / rr_cur
-__global__ void k_cg_dir(ImpArgs a, const double *scal, int cur, const double *r, double *p) {
+// p = r + beta p; p32: the copy of p that the FP32 operator multiplies (null: none)
+__global__ void __launch_bounds__(256) k_cg_dir(ImpArgs a, const double *scal, const double *r, double *p, float *p32,
+                                                int stop) {
+    pdl_wait();
+    if (stop && scal[S_DONE] != 0.0) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    const double beta = block_div(scal[cur ^ 1], scal[cur]);
-    if (n >= a.nodec) return;
     const size_t N = (size_t)a.nodec;
+    if (n >= a.nodec) return;
+    double rv[3], pv[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) rv[c] = r[c * N + n], pv[c] = p[c * N + n];
+    const double beta = scal[S_BETA];
+#pragma unroll
     for (int c = 0; c < 3; c++) {
         const size_t i = c * N + n;
-        p[i] = r[i] + beta * p[i];
+        const double v = rv[c] + beta * pv[c];
+        p[i] = v;
+        if (p32) p32[i] = (float)v;
     }
+}
+
+// (re)starts a solve from the residual r: p = r, the iteration count `it` and the
+// threshold that ends it
+__global__ void k_cg_start(ImpArgs a, double *scal, double thr, int it, const double *r, double *p, float *p32) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        scal[S_THR] = thr;
+        scal[S_ITER] = (double)it;
+        scal[S_DONE] = 0.0;
+    }
+    if (i >= 3 * a.nodec) return;
+    const double v = r[i];
+    p[i] = v;
+    if (p32) p32[i] = (float)v;
 }
 
 // RestorSolution: x = xs D (crsmat.cpp:214-230)
@@ -1436,6 +1565,7 @@ void implicit_free(mpm_ctx *c) {
     if (s->cnt) cudaFree(s->cnt);
     if (s->gqf) cudaFree(s->gqf);
     if (s->gp32) cudaFree(s->gp32);
+    if (s->p32) cudaFree(s->p32);
     if (s->dfx) cudaFree(s->dfx);
     if (s->gq32) cudaFree(s->gq32);
     if (s->h_scal) cudaFreeHost(s->h_scal);
@@ -1535,6 +1665,7 @@ mpm_status mpm_gpu_implicit_setup(mpm_ctx *c, int nr_flag, double spec_rad) {
     if (s->prec == 32) {
         CKI(cudaMalloc((void **)&s->gp32, sizeof(float) * GM * 3 * N));
         CKI(cudaMalloc((void **)&s->gq32, sizeof(float) * GM * 3 * N));
+        CKI(cudaMalloc((void **)&s->p32, sizeof(float) * 3 * N));
         if (!getenv("MPM_GB300_TRUE_RESIDUAL_FP64")) CKI(cudaMalloc((void **)&s->dfx, sizeof(float) * 2 * 3 * N));
     }
     CKI(cudaMalloc((void **)&s->cnt, sizeof(unsigned) * 8));
@@ -1544,7 +1675,7 @@ mpm_status mpm_gpu_implicit_setup(mpm_ctx *c, int nr_flag, double spec_rad) {
     CKI(cudaMalloc((void **)&s->nei, sizeof(double) * N));
     s->nblk = (int)((N + 255) / 256);
     int pblk = (int)((c->num + 127) / 128);
-    int nparts = 2 * (s->nblk > pblk ? s->nblk : pblk) + 2 * ((3 * (int)N + 255) / 256) + (GM + 2) * s->nblk + 64;
+    int nparts = 2 * (s->nblk > pblk ? s->nblk : pblk) + 2 * ((3 * (int)N + 255) / 256) + (GM + 2) * s->nblk + (int)((N + MV_NODES - 1) / MV_NODES) + 64;
     CKI(cudaMalloc((void **)&s->part, sizeof(double) * (size_t)nparts));
     CKI(cudaMalloc((void **)&s->scal, sizeof(double) * S_NSCAL));
     CKI(cudaMallocHost((void **)&s->h_scal, sizeof(double) * S_NSCAL));
@@ -1560,7 +1691,8 @@ static int nb_nodes(mpm_ctx *c) { return (c->g.nodec + 255) / 256; }
 // precision and stencil); hi: FP64 arithmetic whatever the storage (the
 // true residual and the Newton check of the FP32 operator).
 static void launch_matvec(mpm_ctx *c, const ImpArgs &a, int nb, const double *x, double *y, double *part,
-                          unsigned *cnt = nullptr, double *scal = nullptr, int slot = 0, bool hi = false) {
+                          unsigned *cnt = nullptr, double *scal = nullptr, int slot = 0, bool hi = false,
+                          int num = -1) {
     ImpState *s = c->imp;
     const int *o = c->g.order;
     auto go = [&](auto ta, auto tc) {
@@ -1568,11 +1700,11 @@ static void launch_matvec(mpm_ctx *c, const ImpArgs &a, int nb, const double *x,
         using TC = decltype(tc);
         const TA *A = (const TA *)s->A;
         if (o[0] == 1 && o[1] == 1 && o[2] == 1)
-            k_imp_matvec<TA, TC, 1, 1, 1><<<nb, 256, 0, c->stream>>>(a, A, x, y, part, cnt, scal, slot);
+            k_imp_matvec<TA, TC, 1, 1, 1><<<nb, 256, 0, c->stream>>>(a, A, x, y, part, cnt, scal, slot, num);
         else if (o[1] == 2)
-            k_imp_matvec<TA, TC, 2, 2, 2><<<nb, 256, 0, c->stream>>>(a, A, x, y, part, cnt, scal, slot);
+            k_imp_matvec<TA, TC, 2, 2, 2><<<nb, 256, 0, c->stream>>>(a, A, x, y, part, cnt, scal, slot, num);
         else
-            k_imp_matvec<TA, TC, 2, 1, 2><<<nb, 256, 0, c->stream>>>(a, A, x, y, part, cnt, scal, slot);
+            k_imp_matvec<TA, TC, 2, 1, 2><<<nb, 256, 0, c->stream>>>(a, A, x, y, part, cnt, scal, slot, num);
     };
     if (s->prec == 64) {
         go(double(), double());
@@ -1594,17 +1726,54 @@ static void launch_matvec(mpm_ctx *c, const ImpArgs &a, int nb, const double *x,
     }
 }
 
-// y = A x with FP32 vectors and FP32 arithmetic (FP32 operator only): the
-// matvec of the flexible GCR directions.
-static void launch_matvec_f32(mpm_ctx *c, const ImpArgs &a, int nb, const float *x, float *y) {
+// Whether a CG product runs with MV_G threads per control point.  It does where
+// one thread per point leaves the chip short of loads in flight: per product,
+// split against not, 11.7 against 19.6 us (FP32, 1,690 points), 18.6 against 22.1
+// (FP32, 46,305), 37.5 against 50.8 (FP64, 46,305), 18.7 against 32.1 (FP32
+// B-spline stencil, 24,000).  On a large grid the reduction of the dot product over eight times
+// as many CTAs costs more than that: 86 against 65 us (FP32) and 174 against 152
+// (FP64) at 274,625 points.
+static bool mv_split(const mpm_ctx *c) { return c->g.nodec <= 100000; }
+
+template <typename TA, typename TC, typename TV, typename TY>
+static void launch_split(mpm_ctx *c, const ImpArgs &a, const TV *x, TY *y, const double *xd, double *part,
+                         unsigned *cnt, double *scal, int slot, int num, const double *done) {
     const int *o = c->g.order;
-    const float *A = (const float *)c->imp->A;
-    if (o[0] == 1 && o[1] == 1 && o[2] == 1)
-        k_imp_matvec<float, float, 1, 1, 1, float><<<nb, 256, 0, c->stream>>>(a, A, x, y, nullptr);
-    else if (o[1] == 2)
-        k_imp_matvec<float, float, 2, 2, 2, float><<<nb, 256, 0, c->stream>>>(a, A, x, y, nullptr);
+    const unsigned nb = (unsigned)((c->g.nodec + MV_NODES - 1) / MV_NODES);
+    const TA *A = (const TA *)c->imp->A;
+    auto go = [&](auto k) { launch(true, k, nb, MV_NODES * MV_G, 0, c->stream, a, A, x, y, xd, part, cnt, scal, slot, num, done); };
+    if (o[0] == 1 && o[1] == 1 && o[2] == 1) go(k_imp_matvec_split<TA, TC, 1, 1, 1, TV, TY>);
+    else if (o[1] == 2) go(k_imp_matvec_split<TA, TC, 2, 2, 2, TV, TY>);
+    else go(k_imp_matvec_split<TA, TC, 2, 1, 2, TV, TY>);
+}
+
+// y = A x with FP32 vectors and FP32 arithmetic (FP32 operator only): the
+// matvec of the flexible GCR directions.  Without a dot product the split form is
+// the faster one on every grid (52.6 against 57.0 us at 274,625 points).
+static void launch_matvec_f32(mpm_ctx *c, const ImpArgs &a, const float *x, float *y) {
+    launch_split<float, float>(c, a, x, y, nullptr, nullptr, nullptr, nullptr, 0, -1, nullptr);
+}
+
+// Ap = A p and p.Ap (into S_PAP) of one CG iteration; the FP32 operator
+// multiplies the FP32 copy of p that k_cg_dir left
+static void launch_matvec_cg(mpm_ctx *c, const ImpArgs &a, int nb, int cur, const double *done) {
+    ImpState *s = c->imp;
+    const int *o = c->g.order;
+    if (!mv_split(c) && s->prec == 64)
+        launch_matvec(c, a, nb, s->p, s->Ap, s->part, s->cnt + 3, s->scal, S_PAP, false, cur);
+    else if (!mv_split(c)) {
+        auto go = [&](auto k) {
+            k<<<nb, 256, 0, c->stream>>>(a, (const float *)s->A, (const float *)s->p32, s->Ap, s->part, s->cnt + 3,
+                                         s->scal, S_PAP, cur, (const double *)s->p);
+        };
+        if (o[0] == 1 && o[1] == 1 && o[2] == 1) go(k_imp_matvec<float, float, 1, 1, 1, float, double>);
+        else if (o[1] == 2) go(k_imp_matvec<float, float, 2, 2, 2, float, double>);
+        else go(k_imp_matvec<float, float, 2, 1, 2, float, double>);
+    }
+    else if (s->prec == 64)
+        launch_split<double, double>(c, a, (const double *)s->p, s->Ap, s->p, s->part, s->cnt + 3, s->scal, S_PAP, cur, done);
     else
-        k_imp_matvec<float, float, 2, 1, 2, float><<<nb, 256, 0, c->stream>>>(a, A, x, y, nullptr);
+        launch_split<float, float>(c, a, (const float *)s->p32, s->Ap, s->p, s->part, s->cnt + 3, s->scal, S_PAP, cur, done);
 }
 
 // AssembleSystem: k_imp_assemble (per particle), k_imp_rhs_diag, k_imp_scale
@@ -1709,15 +1878,16 @@ static mpm_status capture_iters(mpm_ctx *c, cudaGraphExec_t *exec, F body) {
 }
 
 // one CG iteration on the scaled system; `it` fixes the residual-norm slot parity
-static void cg_iteration(mpm_ctx *c, const ImpArgs &a, int nb, int it) {
+static void cg_iteration(mpm_ctx *c, const ImpArgs &a, int nb, int it, int stop) {
     ImpState *s = c->imp;
     const int cur = (it & 1) ? S_RR1 : S_RR0;
     timer_begin(c, K_MATVEC);
-    launch_matvec(c, a, nb, s->p, s->Ap, s->part, s->cnt + 3, s->scal, S_PAP);
+    launch_matvec_cg(c, a, nb, cur, stop ? s->scal + S_DONE : nullptr);
     timer_end(c, K_MATVEC);
     timer_begin(c, K_KRYLOV);
-    k_cg_update<<<nb, 256, 0, c->stream>>>(a, s->scal, cur, s->xs, s->r, s->p, s->Ap, s->part, s->cnt + 4);
-    k_cg_dir<<<nb, 256, 0, c->stream>>>(a, s->scal, cur, s->r, s->p);
+    launch(true, k_cg_update, nb, 256, 0, c->stream, a, s->scal, cur, s->xs, s->r, (const double *)s->p,
+           (const double *)s->Ap, s->part, s->cnt + 4, stop);
+    launch(true, k_cg_dir, nb, 256, 0, c->stream, a, (const double *)s->scal, (const double *)s->r, s->p, s->p32, stop);
     timer_end(c, K_KRYLOV);
     c->launches += 3;
 }
@@ -1725,7 +1895,7 @@ static void cg_iteration(mpm_ctx *c, const ImpArgs &a, int nb, int it) {
 static mpm_status imp_cg(mpm_ctx *c, double eps, int kmax, int *iters) {
     ImpState *s = c->imp;
     ImpArgs a = imp_args(c);
-    const int nb = nb_nodes(c);
+    const int nb = nb_nodes(c), nb3 = (3 * c->g.nodec + 255) / 256;
     k_cg_scale_in<<<nb, 256, 0, c->stream>>>(a, s->x, s->b, s->adiag, s->xs, s->r);
     if (s->prec == 32)   // the scaled RHS, for the true residual of the FP32 operator
         CKI(cudaMemcpyAsync(s->bs, s->r, sizeof(double) * 3 * c->g.nodec, cudaMemcpyDeviceToDevice, c->stream));
@@ -1738,62 +1908,66 @@ static mpm_status imp_cg(mpm_ctx *c, double eps, int kmax, int *iters) {
     const double rr0 = s->h_scal[S_RR0];
     int it = 0;
     bool done = !(rr0 > 1.0e-300);
-    bool fine = false;   // close to the tolerance: one iteration at a time, checked after each
+    // the device ends the solve at the iteration that reaches the tolerance; what
+    // is left of the launched block then does nothing.  (Checked by the host, the
+    // last decades of the residual went one iteration and one wait at a time.)
+    if (!done) {
+        k_cg_start<<<nb3, 256, 0, c->stream>>>(a, s->scal, eps * rr0, 0, s->r, s->p, s->p32);
+        c->launches++;
+    }
     while (!done && it < kmax) {
-        if (graphs_on(c) && !fine && it % KCHECK == 0 && it + KCHECK <= kmax) {
+        bool ran = false;
+        if (graphs_on(c) && it % KCHECK == 0 && it + KCHECK <= kmax) {
+            const int64_t l0 = c->launches;
             if (!s->g_cg && capture_iters(c, &s->g_cg, [&] {
-                    for (int k = 0; k < KCHECK; k++) cg_iteration(c, a, nb, k);
+                    for (int k = 0; k < KCHECK; k++) cg_iteration(c, a, nb, k, 1);
                 }) != MPM_OK)
                 s->no_graph = true;
             if (s->g_cg) {
                 CKI(cudaGraphLaunch(s->g_cg, c->stream));
-                it += KCHECK;
-                if (it > KCHECK) c->launches += 5 * KCHECK;   // the capture counted the first block
-            } else {
-                continue;
+                if (c->launches == l0) c->launches += 3 * KCHECK;   // the capture counted the first block
+                ran = true;
             }
-        } else {
-            cg_iteration(c, a, nb, it);
-            it++;
         }
-        if (it % KCHECK == 0 || it == kmax || fine) {
+        if (!ran) {
+            const int end = std::min(kmax, it + KCHECK - it % KCHECK);
+            for (int k = it; k < end; k++) cg_iteration(c, a, nb, k, 1);
+        }
+        CKI(cudaMemcpyAsync(s->h_scal, s->scal, sizeof(double) * S_NSCAL, cudaMemcpyDeviceToHost, c->stream));
+        CKI(cudaStreamSynchronize(c->stream));
+        it = (int)s->h_scal[S_ITER];
+        const int cur = (it & 1) ? S_RR1 : S_RR0;
+        const double rr = s->h_scal[cur];
+        if (rr != rr) {
+            *iters = it;
+            return MPM_ERR_NONFINITE;
+        }
+        if (s->debug) fprintf(stderr, "mpm_gb300 cg: it %d |r|/|r0| %.3e\n", it, sqrt(rr / rr0));
+        if (rr < eps * rr0 && s->prec == 32) {
+            // FP32 operator: the recursive residual carries the rounding of
+            // the FP32 matvecs, so convergence is judged on the true
+            // residual bs - A x (FP64 arithmetic); if it is not below the
+            // tolerance, CG restarts from it (r, and p = r).  Keeping the
+            // old direction instead diverged: at this point the recursive
+            // residual, and with it p, has fallen far below the true
+            // residual, so alpha = r.r / p.Ap overshoots.
+            launch_matvec(c, a, nb, s->xs, s->z, nullptr, nullptr, nullptr, 0, true);
+            k_true_residual<<<nb, 256, 0, c->stream>>>(a, s->bs, s->z, s->r, s->part);
+            k_finish<<<1, 256, 0, c->stream>>>(s->part, nb, s->scal, cur);
+            k_cg_start<<<nb3, 256, 0, c->stream>>>(a, s->scal, eps * rr0, it, s->r, s->p, s->p32);
+            c->launches += 4;
             CKI(cudaMemcpyAsync(s->h_scal, s->scal, sizeof(double) * 2, cudaMemcpyDeviceToHost, c->stream));
             CKI(cudaStreamSynchronize(c->stream));
-            const double rr = s->h_scal[(it & 1) ? S_RR1 : S_RR0];
-            if (rr != rr) {
-                *iters = it;
-                return MPM_ERR_NONFINITE;
-            }
-            if (s->debug) fprintf(stderr, "mpm_gb300 cg: it %d |r|/|r0| %.3e\n", it, sqrt(rr / rr0));
-            if (rr < eps * rr0 && s->prec == 32) {
-                // FP32 operator: the recursive residual carries the rounding of
-                // the FP32 matvecs, so convergence is judged on the true
-                // residual bs - A x (FP64 arithmetic); if it is not below the
-                // tolerance, CG restarts from it (r, and p = r).  Keeping the
-                // old direction instead diverged: at this point the recursive
-                // residual, and with it p, has fallen far below the true
-                // residual, so alpha = r.r / p.Ap overshoots.
-                const int cur = (it & 1) ? S_RR1 : S_RR0;
-                launch_matvec(c, a, nb, s->xs, s->z, nullptr, nullptr, nullptr, 0, true);
-                k_true_residual<<<nb, 256, 0, c->stream>>>(a, s->bs, s->z, s->r, s->part);
-                k_finish<<<1, 256, 0, c->stream>>>(s->part, nb, s->scal, cur);
-                CKI(cudaMemcpyAsync(s->p, s->r, sizeof(double) * 3 * c->g.nodec, cudaMemcpyDeviceToDevice,
-                                    c->stream));
-                c->launches += 3;
-                CKI(cudaMemcpyAsync(s->h_scal, s->scal, sizeof(double) * 2, cudaMemcpyDeviceToHost, c->stream));
-                CKI(cudaStreamSynchronize(c->stream));
-                const double rrt = s->h_scal[cur];
-                if (s->debug) fprintf(stderr, "mpm_gb300 cg: it %d true |r|/|r0| %.3e\n", it, sqrt(rrt / rr0));
-                if (rrt < eps * rr0) done = true;
-                s->last_rel = sqrt(rrt / rr0);
-            } else {
-                if (rr < eps * rr0) done = true;
-                else if (rr < FINE_FACTOR * eps * rr0) fine = true;
-                s->last_rel = sqrt(rr / rr0);
-            }
+            const double rrt = s->h_scal[cur];
+            if (s->debug) fprintf(stderr, "mpm_gb300 cg: it %d true |r|/|r0| %.3e\n", it, sqrt(rrt / rr0));
+            if (rrt < eps * rr0) done = true;
+            s->last_rel = sqrt(rrt / rr0);
+        } else {
+            if (rr < eps * rr0) done = true;
+            s->last_rel = sqrt(rr / rr0);
         }
     }
-    k_cg_scale_out<<<(3 * c->g.nodec + 255) / 256, 256, 0, c->stream>>>(a, s->xs, s->adiag, s->x);
+    k_cg_scale_out<<<nb3, 256, 0, c->stream>>>(a, s->xs, s->adiag, s->x);
     c->launches++;
     *iters = it;
     if (!done) return MPM_ERR_KRYLOV_MAXIT;
@@ -1816,7 +1990,7 @@ static mpm_status gcr_iter(mpm_ctx *c, const ImpArgs &a, int nb, int u, int sl) 
         timer_end(c, K_PRECOND);
         if (st != MPM_OK) return st;
         timer_begin(c, K_MATVEC);
-        launch_matvec_f32(c, a, nb, p, q);
+        launch_matvec_f32(c, a, p, q);
         timer_end(c, K_MATVEC);
         timer_begin(c, K_KRYLOV);
         if (u > 0)
@@ -1955,7 +2129,17 @@ static mpm_status imp_fcg(mpm_ctx *c, double eps, int kmax, int *iters) {
                 it++;
             }
             if (it % check == 0 || it == kmax || fine) {
-                if (s->prec == 32) {
+                // between the checks the recursive residual tells whether the true one
+                // (a double-float product) is worth forming: within a window they
+                // differ by the rounding of a few FP32 products
+                bool form = s->prec == 32;
+                if (form && it % check != 0 && it != kmax) {
+                    CKI(cudaMemcpyAsync(s->h_scal, s->scal, sizeof(double) * S_NSCAL, cudaMemcpyDeviceToHost,
+                                        c->stream));
+                    CKI(cudaStreamSynchronize(c->stream));
+                    if (s->h_scal[S_RRC] >= 1.1 * eps * rr0) continue;
+                }
+                if (form) {
                     // FP32 operator: the recursive residual drifts from the true one
                     // by the rounding of the FP32 matvecs, so at every check it is
                     // replaced by the true residual bs - A x (FP64 arithmetic); the
@@ -2313,6 +2497,7 @@ static mpm_status cg_scaled(mpm_ctx *c, double eps, int kmax, mpm_nn *net, int s
     const double rr0 = s->h_scal[S_RR0];
     int it = 0, pairs = 0;
     bool done = !(rr0 > 1.0e-300);
+    k_cg_start<<<(3 * c->g.nodec + 255) / 256, 256, 0, c->stream>>>(a, s->scal, 0.0, 0, s->r, s->p, s->p32);
     while (!done && it < kmax) {
         const int cur = (it & 1) ? S_RR1 : S_RR0;
         if (net && it % stride == 0 && pairs < max_pairs) {
@@ -2321,9 +2506,7 @@ static mpm_status cg_scaled(mpm_ctx *c, double eps, int kmax, mpm_nn *net, int s
             if (st != MPM_OK) return st;
             pairs++;
         }
-        launch_matvec(c, a, nb, s->p, s->Ap, s->part, s->cnt + 3, s->scal, S_PAP);
-        k_cg_update<<<nb, 256, 0, c->stream>>>(a, s->scal, cur, s->xs, s->r, s->p, s->Ap, s->part, s->cnt + 4);
-        k_cg_dir<<<nb, 256, 0, c->stream>>>(a, s->scal, cur, s->r, s->p);
+        cg_iteration(c, a, nb, it, 0);
         it++;
         if (it % 8 == 0 || it == kmax) {
             CKI(cudaMemcpyAsync(s->h_scal, s->scal, sizeof(double) * 2, cudaMemcpyDeviceToHost, c->stream));
