@@ -80,8 +80,10 @@ struct ImpState {
     float *gqf = nullptr;                   // FP32 copies of the kept images (GM * 3 * nodec), for the dots
     float *gp32 = nullptr, *gq32 = nullptr;  // FP32 operator: the directions and images in FP32 (GM * 3 * nodec)
     float *p32 = nullptr;                   // FP32 operator: the CG direction in FP32
+    float *nf32 = nullptr;                  // FP32 copies of ndispl, nvel, naccel (3 N each) and nei (N) for the particles
     float *dfx = nullptr;                   // FP32 operator: x split into high and low FP32 parts (2 * 3 * nodec)
     unsigned *cnt = nullptr;                // block counters of the single-launch reductions (zero between launches)
+    bool isotropic = false;                 // every material's tangent is isotropic (models -1, 0, 1)
     int fallbacks = 0;                      // solves that switched from the network to Jacobi
     int nn_applications = 0;
     // CUDA graphs of 8 Krylov iterations (CG; FCG with the network; FCG with Jacobi)
@@ -364,25 +366,16 @@ __device__ __forceinline__ void tangent_mooney_rivlin(Tangent<R> &t, const R F[3
     t.beta = t.delta = (R)(-0.5) * c2p;
 }
 
-// One thread per particle (AssembleSystem, solve_solid_implicit.cpp:123-189):
-// UpdateDefGrad with alpha_f, the stress of the Newton iterate, the gradient
-// correction dN <- dN dF^-1, then the tangent blocks of each unordered node
-// pair once (K_ba = K_ab^T: every C here has the major symmetry) + lumped
-// mass, and the internal/external force into the RHS, with atomics.  R is
-// the particle precision and the precision of the arithmetic and of A; the
-// RHS is summed in FP64.
+// A particle's part of AssembleSystem (solve_solid_implicit.cpp:123-189):
+// UpdateDefGrad with alpha_f, the stress of the Newton iterate (written to
+// stress_k), the gradient correction dN <- dN dF^-1 and the tangent of its model.
 template <typename R, int OX, int OY, int OZ>
-__global__ void __launch_bounds__(128) k_imp_assemble(ImpArgs a, PView<R> P, const double *ndispl, R *stress_k,
-                                                      R *A, double *b) {
-    constexpr int NX = OX + 1, NY = OY + 1, NZ = OZ + 1, NE = NX * NY * NZ;
-    constexpr int SX = 2 * OX + 1, SY = 2 * OY + 1, NS = SX * SY * (2 * OZ + 1);
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= a.num) return;
+__device__ __forceinline__ void imp_particle(const ImpArgs &a, const PView<R> &P, const R *ndispl, R *stress_k,
+                                             int p, int *nid, R *Nw, R (*dN)[3], R *sk, R &vol, Tangent<R> &t) {
+    constexpr int NE = (OX + 1) * (OY + 1) * (OZ + 1);
     const size_t N = (size_t)a.nodec, NP = (size_t)a.num;
     const KGeom<R> g = kgeom<R>(a);
     const R x[3] = {P.x[0][p], P.x[1][p], P.x[2][p]};
-    int nid[NE];
-    R Nw[NE], dN[NE][3];
     bool oob = false;
     shape_nodes<R, OX, OY, OZ>(a, g, x, Nw, dN, nid, oob);
     // ComputeDeltaDefGrad with alpha_f (material_point.cpp:127-151): d = I + Dm
@@ -428,14 +421,12 @@ __global__ void __launch_bounds__(128) k_imp_assemble(ImpArgs a, PView<R> P, con
         for (int r = 0; r < 3; r++)
             for (int c = 0; c < 3; c++) Fn[r][c] = Hn[r][c] + (r == c ? (R)1 : (R)0);
     }
-    const R vol = J * P.vol0[p];
+    vol = J * P.vol0[p];
     // UpdateConstitutiveModel on the Newton stress (constitutive_model.cpp:16-305)
-    R sk[6];
     for (int k = 0; k < 6; k++) sk[k] = stress_k[k * NP + p];
     const int mid = P.matid[p];
     const int model = a.iprop[mid];
     const R E = (R)a.matprop[3 * mid], nu = (R)a.matprop[3 * mid + 1], m3 = (R)a.matprop[3 * mid + 2];
-    Tangent<R> t;
     t.general = false;
     t.lam = t.mu = (R)0;
     if (model == 0) {
@@ -501,6 +492,19 @@ __global__ void __launch_bounds__(128) k_imp_assemble(ImpArgs a, PView<R> P, con
         for (int c = 0; c < 3; c++) tq[c] = dN[q][0] * di[0][c] + dN[q][1] * di[1][c] + dN[q][2] * di[2][c];
         for (int c = 0; c < 3; c++) dN[q][c] = tq[c];
     }
+}
+
+// The tangent blocks of each unordered node pair of one particle once (K_ba =
+// K_ab^T: every C here has the major symmetry) + lumped mass, and the
+// internal/external force into the RHS, with atomics; the RHS is summed in FP64.
+template <typename R, int OX, int OY, int OZ>
+__device__ __forceinline__ void imp_scatter(const ImpArgs &a, const PView<R> &P, int p, const int *nid, const R *Nw,
+                                            const R (*dN)[3], const R *sk, R vol, const Tangent<R> &t, R *A,
+                                            double *b) {
+    constexpr int NX = OX + 1, NY = OY + 1, NZ = OZ + 1, NE = NX * NY * NZ;
+    constexpr int SX = 2 * OX + 1, SY = 2 * OY + 1, NS = SX * SY * (2 * OZ + 1);
+    const size_t N = (size_t)a.nodec;
+    const R af = (R)a.af;
     const R sg[3][3] = {{sk[0], sk[5], sk[4]}, {sk[5], sk[1], sk[3]}, {sk[4], sk[3], sk[2]}};
     const R m = P.m[p];
     const R fx = (R)(a.grav[0] * a.facl), fy = (R)(a.grav[1] * a.facl), fz = (R)(a.grav[2] * a.facl);
@@ -581,6 +585,184 @@ __global__ void __launch_bounds__(128) k_imp_assemble(ImpArgs a, PView<R> P, con
         atomicAdd(&b[na], (double)f0);
         atomicAdd(&b[N + na], (double)f1);
         atomicAdd(&b[2 * N + na], (double)f2);
+    }
+}
+
+// One thread per particle: its part, then its pairs with atomics.  R is the
+// particle precision and the precision of the arithmetic and of A.
+template <typename R, int OX, int OY, int OZ>
+__global__ void __launch_bounds__(128) k_imp_assemble(ImpArgs a, PView<R> P, const R *ndispl, R *stress_k,
+                                                      R *A, double *b) {
+    constexpr int NE = (OX + 1) * (OY + 1) * (OZ + 1);
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= a.num) return;
+    int nid[NE];
+    R Nw[NE], dN[NE][3], sk[6], vol;
+    Tangent<R> t;
+    imp_particle<R, OX, OY, OZ>(a, P, ndispl, stress_k, p, nid, Nw, dN, sk, vol, t);
+    imp_scatter<R, OX, OY, OZ>(a, P, p, nid, Nw, dN, sk, vol, t, A, b);
+}
+
+// The assembly of an FP32 operator whose materials are isotropic (models -1, 0,
+// 1), cell by cell.  A particle adds 576 numbers to the matrix (8 nodes) and its
+// cell's other particles add to the same ones: with an atomic each, the assembly
+// waited for the memory system (1,728,000 particles: 1.1e9 atomics, 2.07 ms).
+// Here a CTA takes CELLS cells of a brick: its threads form their particles'
+// parts in shared memory, then BG threads per cell and row node sum that node's
+// blocks with NB column nodes over the cell's particles in registers and add
+// each once, two entries per reduction.  What is left is bound by registers and
+// latency (72 sums a thread): 16 cells and 128 particles per CTA, three CTAs per
+// SM held to 168 registers, beat 32 cells in one CTA (592 to 741 us) and two or
+// four threads per row node (790 to 1018).  The class with scaling and RHS, per
+// Newton iteration: 1,728,000 particles 2217 -> 592 us, 232,320 372 -> 150, quadratic
+// B-splines (87,808) 870 -> 439.
+// A particle outside its sorted cell scatters with atomics of its own.
+template <int OX, int OY, int OZ>
+struct AsmShape {
+    static constexpr int NX = OX + 1, NY = OY + 1, NZ = OZ + 1, NE = NX * NY * NZ;
+    static constexpr int SX = 2 * OX + 1, SY = 2 * OY + 1, NS = SX * SY * (2 * OZ + 1);
+    static constexpr int BG = NE == 8 ? 1 : 3, NB = NE / BG;
+    static constexpr int CELLS = NE == 8 ? 16 : NE == 18 ? 8 : 4;
+    static constexpr int THREADS = CELLS * NE * BG;
+    static constexpr int CH = NE == 8 ? 128 : 64, ST = CH + 1;          // particles per round; row stride
+    static constexpr int F_N = 3 * NE, F_L = 4 * NE, F_M = F_L + 1, F_S = F_L + 2, F_MASS = F_L + 8, NFLD = F_L + 9;
+    static constexpr size_t SMEM = sizeof(float) * NFLD * ST;
+    static_assert((CELLS & (CELLS - 1)) == 0, "binary search");
+    static_assert(NE % BG == 0 && THREADS >= CH, "one particle per thread and round");
+};
+
+__device__ __forceinline__ void red2(float *p, float x, float y) {
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(x), "f"(y) : "memory");
+}
+// a double sum as an unevaluated pair of FP32 numbers (two-sum)
+__device__ __forceinline__ void pair_add(float &s, float &e, float q) {
+    const float t = __fadd_rn(s, q), u = __fsub_rn(t, s);
+    e += __fadd_rn(__fsub_rn(s, __fsub_rn(t, u)), __fsub_rn(q, u));
+    s = t;
+}
+
+template <int OX, int OY, int OZ>
+__global__ void __launch_bounds__(AsmShape<OX, OY, OZ>::THREADS, (OX == 1 ? 3 : 1))
+    k_imp_assemble_cells(ImpArgs a, PView<float> P, const float *ndispl, float *stress_k, float *A, double *b,
+                         const int *cstart, const int *blist, const int *nblist, int nbx, int nby) {
+    using C = AsmShape<OX, OY, OZ>;
+    constexpr int NX = C::NX, NY = C::NY, NE = C::NE, NB = C::NB, ST = C::ST;
+    extern __shared__ float sm[];   // [NFLD][ST]
+    constexpr int SLABS = BRC / C::CELLS;
+    const int item = blockIdx.x;
+    if (item >= *nblist * SLABS) return;
+    const int br = blist[item / SLABS], c0 = (item % SLABS) * C::CELLS;
+    const int *cs = cstart + (size_t)br * (BRC + 1) + c0;
+    const int P0 = cs[0], P1 = cs[C::CELLS];
+    if (P0 == P1) return;
+    const int lc = threadIdx.x / (NE * C::BG), rem = threadIdx.x % (NE * C::BG), na = rem % NE, b0 = (rem / NE) * NB;
+    const int cell = c0 + lc;
+    const int cx = (br % nbx) * BRX + cell % BRX, cy = ((br / nbx) % nby) * BRY + (cell / BRX) % BRY,
+              cz = (br / (nbx * nby)) * BRZ + cell / (BRX * BRY);
+    const int p0 = cs[lc], p1 = cs[lc + 1];
+    const float afg = a.nr_flag ? (float)a.af : 0.0f, amb = (float)(a.am * a.nb[3]);
+    const float gv[3] = {(float)(a.grav[0] * a.facl), (float)(a.grav[1] * a.facl), (float)(a.grav[2] * a.facl)};
+    float K[NB][3][3], f[3] = {0.0f, 0.0f, 0.0f}, fe[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int q = 0; q < NB; q++)
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int j = 0; j < 3; j++) K[q][i][j] = 0.0f;
+    for (int r0 = P0; r0 < P1; r0 += C::CH) {
+        const int l = threadIdx.x, p = r0 + l;
+        if (l < C::CH && p < P1) {
+            int nid[NE];
+            float Nw[NE], dN[NE][3], sk[6], vol;
+            Tangent<float> t;
+            imp_particle<float, OX, OY, OZ>(a, P, ndispl, stress_k, p, nid, Nw, dN, sk, vol, t);
+            // its sorted cell is the one whose range holds p; its own cell's first node is nid[0]
+            int q = 0;
+#pragma unroll
+            for (int h = C::CELLS / 2; h >= 1; h /= 2)
+                if (cs[q + h] <= p) q += h;
+            const int oc = c0 + q;
+            const int ox = (br % nbx) * BRX + oc % BRX, oy = ((br / nbx) % nby) * BRY + (oc / BRX) % BRY,
+                      oz = (br / (nbx * nby)) * BRZ + oc / (BRX * BRY);
+            const bool mine = nid[0] == ox + a.nnc[0] * (oy + a.nnc[1] * oz);
+            if (!mine) imp_scatter<float, OX, OY, OZ>(a, P, p, nid, Nw, dN, sk, vol, t, A, b);
+            const float on = mine ? 1.0f : 0.0f, afv = (float)a.af * vol;
+#pragma unroll
+            for (int e = 0; e < NE; e++) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) sm[(3 * e + c) * ST + l] = mine ? dN[e][c] : 0.0f;
+                sm[(C::F_N + e) * ST + l] = mine ? Nw[e] : 0.0f;
+            }
+            sm[C::F_L * ST + l] = mine ? t.lam * afv : 0.0f;
+            sm[C::F_M * ST + l] = mine ? t.mu * afv : 0.0f;
+#pragma unroll
+            for (int e = 0; e < 6; e++) sm[(C::F_S + e) * ST + l] = mine ? vol * sk[e] : 0.0f;
+            sm[C::F_MASS * ST + l] = on * P.m[p];
+        }
+        __syncthreads();
+        const int q1 = min(p1, r0 + C::CH);
+        for (int pp = max(p0, r0); pp < q1; pp++) {
+            const float *s = sm + (pp - r0);
+            const float av[3] = {s[(3 * na) * ST], s[(3 * na + 1) * ST], s[(3 * na + 2) * ST]};
+            const float lam = s[C::F_L * ST], mu = s[C::F_M * ST], m = s[C::F_MASS * ST], N_ = s[(C::F_N + na) * ST];
+            const float S[6] = {s[C::F_S * ST], s[(C::F_S + 1) * ST], s[(C::F_S + 2) * ST],
+                                s[(C::F_S + 3) * ST], s[(C::F_S + 4) * ST], s[(C::F_S + 5) * ST]};
+            // vol sigma a: the force of node a and, times alpha_f, the geometric term
+            const float Sa[3] = {S[0] * av[0] + S[5] * av[1] + S[4] * av[2], S[5] * av[0] + S[1] * av[1] + S[3] * av[2],
+                                 S[4] * av[0] + S[3] * av[1] + S[2] * av[2]};
+            float L[3], M[3], T[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                L[c] = lam * av[c];
+                M[c] = mu * av[c];
+                T[c] = fmaf(afg, Sa[c], M[c]);
+            }
+#pragma unroll
+            for (int q = 0; q < NB; q++) {
+                const float bv[3] = {s[(3 * (b0 + q)) * ST], s[(3 * (b0 + q) + 1) * ST], s[(3 * (b0 + q) + 2) * ST]};
+                const float dg = T[0] * bv[0] + T[1] * bv[1] + T[2] * bv[2];
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        float v = fmaf(L[i], bv[j], K[q][i][j]);
+                        if (i == j) v += dg;
+                        K[q][i][j] = fmaf(M[j], bv[i], v);
+                    }
+            }
+            const float emd = amb * N_ * m;
+#pragma unroll
+            for (int q = 0; q < NB; q++)
+                if (b0 + q == na) K[q][0][0] += emd, K[q][1][1] += emd, K[q][2][2] += emd;
+            if (b0 == 0) {
+                const float Nm = N_ * m;
+#pragma unroll
+                for (int c = 0; c < 3; c++) pair_add(f[c], fe[c], fmaf(Nm, gv[c], -Sa[c]));
+            }
+        }
+        __syncthreads();   // shared memory is reused by the next round
+    }
+    if (p0 == p1) return;
+    const int ia = na % NX, ja = (na / NX) % NY, ka = na / (NX * NY);
+    const int node = (cx + ia) + a.nnc[0] * ((cy + ja) + a.nnc[1] * (cz + ka));
+#pragma unroll
+    for (int q = 0; q < NB; q++) {
+        const int nb = b0 + q;
+        const int sl = (nb % NX - ia + OX) + C::SX * (((nb / NX) % NY - ja + OY) + C::SY * (nb / (NX * NY) - ka + OZ));
+        const float *v = &K[q][0][0];
+        float *row = A + aidx(9 * sl, node, a.qp);   // entry 9 sl: the first of a pair when sl is even
+        const bool odd = sl & 1;
+        // the other half of a pair is the next address, the next pair 64 on
+        float *pr = odd ? row + 63 : row;
+        atomicAdd(odd ? row : pr + 4 * 64, odd ? v[0] : v[8]);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            red2(pr + 64 * u, odd ? v[2 * u + 1] : v[2 * u], odd ? v[2 * u + 2] : v[2 * u + 1]);
+    }
+    if (b0 == 0) {
+        const size_t N = (size_t)a.nodec;
+#pragma unroll
+        for (int c = 0; c < 3; c++) atomicAdd(&b[c * N + node], (double)f[c] + (double)fe[c]);
     }
 }
 
@@ -1126,11 +1308,14 @@ __global__ void k_imp_nei(ImpArgs a, const double *nvof, double *nei, double *pa
 // already committed: F, J, vol, stress, displacement/acceleration/velocity
 // gathers and the shifting gradient; CommitParticleKinematics without the shift.
 template <typename R, int OX, int OY, int OZ>
-__global__ void __launch_bounds__(128) k_imp_g2p(ImpArgs a, PView<R> P, const double *ndispl, const double *nvel,
-                                                 const double *naccel, const double *nei, R *geup, double *part,
-                                                 DevCtl *ctl, int parity) {
+__global__ void __launch_bounds__(128) k_imp_g2p(ImpArgs a, PView<R> P, const R *__restrict__ ndispl,
+                                                 const R *__restrict__ nvel, const R *__restrict__ naccel,
+                                                 const R *__restrict__ nei, R *geup, double *part, DevCtl *ctl,
+                                                 int parity) {
     constexpr int NE = (OX + 1) * (OY + 1) * (OZ + 1);
     __shared__ double sh[32];
+    __shared__ float sh_m[4][4];   // the four bounds of the block's warps
+    float bnd[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // |a|, |v|, vol, vol |sigma|
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     double gd = 0.0;
     if (p < a.num) {
@@ -1216,7 +1401,7 @@ __global__ void __launch_bounds__(128) k_imp_g2p(ImpArgs a, PView<R> P, const do
                 for (int c = 0; c < 3; c++) {
                     disp[c] += Nw[q] * (R)ndispl[c * N + nid[q]];
                     acc[c] += Nw[q] * (R)naccel[c * N + nid[q]];
-                    vel[c] += Nw[q] * (R)nvel[c * N + nid[q]];
+                    if (!flip) vel[c] += Nw[q] * (R)nvel[c * N + nid[q]];
                 }
         }
         // shifting gradient at the old position with the new volume (material_point.cpp:192-216)
@@ -1239,13 +1424,38 @@ __global__ void __launch_bounds__(128) k_imp_g2p(ImpArgs a, PView<R> P, const do
             amax = fmaxf(amax, (float)fabs(acc[c]));
             vmax = fmaxf(vmax, (float)fabs(vc));
         }
-        const float rs = (float)fmax(fabs((double)sk[0]) + fabs((double)sk[5]) + fabs((double)sk[4]),
-                                     fmax(fabs((double)sk[5]) + fabs((double)sk[1]) + fabs((double)sk[3]),
-                                          fabs((double)sk[4]) + fabs((double)sk[3]) + fabs((double)sk[2])));
-        atomic_max_pos(&ctl->nxt[parity ^ 1][B_AMAX], amax * 1.000001f);
-        atomic_max_pos(&ctl->nxt[parity ^ 1][B_VMAX], vmax * 1.000001f);
-        atomic_max_pos(&ctl->nxt[parity ^ 1][B_VOLMAX], (float)fabs((double)vol) * 1.000001f);
-        atomic_max_pos(&ctl->nxt[parity ^ 1][B_VOLSMAX], (float)fabs((double)vol) * rs * 1.000001f);
+        const float f0 = fabsf((float)sk[0]), f1 = fabsf((float)sk[1]), f2 = fabsf((float)sk[2]),
+                    f3 = fabsf((float)sk[3]), f4 = fabsf((float)sk[4]), f5 = fabsf((float)sk[5]);
+        bnd[0] = amax;
+        bnd[1] = vmax;
+        bnd[2] = fabsf((float)vol);
+        bnd[3] = bnd[2] * fmaxf(f0 + f5 + f4, fmaxf(f5 + f1 + f3, f4 + f3 + f2));
+    }
+    // the block's bounds: one atomic each (one per particle took half of this pass)
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float v = __shfl_xor_sync(0xffffffffu, bnd[k], o);
+            bnd[k] = (v > bnd[k] || v != v) ? v : bnd[k];   // keeps a NaN, which atomic_max_pos turns into the largest bound
+        }
+        if (lane == 0) sh_m[k][wid] = bnd[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        constexpr int slot[4] = {B_AMAX, B_VMAX, B_VOLMAX, B_VOLSMAX};
+        float v = 0.0f;
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
+            const float u = sh_m[threadIdx.x][w];
+            v = (u > v || u != u) ? u : v;
+            if (u != u) break;
+        }
+        int sl = slot[0];
+#pragma unroll
+        for (int k = 1; k < 4; k++)
+            if ((int)threadIdx.x == k) sl = slot[k];
+        atomic_max_pos(&ctl->nxt[parity ^ 1][sl], v * 1.000001f);
     }
     const double t = block_sum(gd, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = t;
@@ -1566,6 +1776,7 @@ void implicit_free(mpm_ctx *c) {
     if (s->gqf) cudaFree(s->gqf);
     if (s->gp32) cudaFree(s->gp32);
     if (s->p32) cudaFree(s->p32);
+    if (s->nf32) cudaFree(s->nf32);
     if (s->dfx) cudaFree(s->dfx);
     if (s->gq32) cudaFree(s->gq32);
     if (s->h_scal) cudaFreeHost(s->h_scal);
@@ -1615,15 +1826,19 @@ mpm_status mpm_gpu_implicit_setup(mpm_ctx *c, int nr_flag, double spec_rad) {
                         (o[0] == 2 && o[1] == 1 && o[2] == 2);
         if (!ok) return MPM_ERR_UNSUPPORTED;
     }
+    bool isotropic = true;
     {
         std::vector<int> ip(c->nmat);
         CKI(cudaMemcpy(ip.data(), c->d_iprop, sizeof(int) * c->nmat, cudaMemcpyDeviceToHost));
-        for (int m : ip)
+        for (int m : ip) {
             if (m > 3) return MPM_ERR_UNSUPPORTED;   // no tangent for the fluid model
+            isotropic = isotropic && m <= 1;
+        }
     }
     implicit_free(c);
     ImpState *s = new ImpState();
     c->imp = s;
+    s->isotropic = isotropic;
     s->debug = getenv("MPM_GB300_KRYLOV_TRACE") != nullptr;
     s->gcr = getenv("MPM_GB300_FCG_ONLY") == nullptr;
     if (const char *w = getenv("MPM_GB300_GCR_WINDOW")) {
@@ -1666,6 +1881,7 @@ mpm_status mpm_gpu_implicit_setup(mpm_ctx *c, int nr_flag, double spec_rad) {
         CKI(cudaMalloc((void **)&s->gp32, sizeof(float) * GM * 3 * N));
         CKI(cudaMalloc((void **)&s->gq32, sizeof(float) * GM * 3 * N));
         CKI(cudaMalloc((void **)&s->p32, sizeof(float) * 3 * N));
+        CKI(cudaMalloc((void **)&s->nf32, sizeof(float) * 10 * N));
         if (!getenv("MPM_GB300_TRUE_RESIDUAL_FP64")) CKI(cudaMalloc((void **)&s->dfx, sizeof(float) * 2 * 3 * N));
     }
     CKI(cudaMalloc((void **)&s->cnt, sizeof(unsigned) * 8));
@@ -1776,20 +1992,56 @@ static void launch_matvec_cg(mpm_ctx *c, const ImpArgs &a, int nb, int cur, cons
         launch_split<float, float>(c, a, (const float *)s->p32, s->Ap, s->p, s->part, s->cnt + 3, s->scal, S_PAP, cur, done);
 }
 
+// FP32 copies of nodal fields, so that the FP32 particles' gathers convert each
+// node's value once instead of once per particle and node (a conversion takes a
+// slot of the FP64 pipe)
+__global__ void k_to_f32(const double *__restrict__ x, float *__restrict__ y, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) y[i] = (float)x[i];
+}
+// `n` values of a nodal field in the particle precision: the field itself, or its
+// copy at `at` of the FP32 copies
+template <typename R>
+static const R *nodal_of(mpm_ctx *c, const double *x, size_t at, size_t n) {
+    if constexpr (sizeof(R) == 8) {
+        return x;
+    } else {
+        float *y = c->imp->nf32 + at;
+        k_to_f32<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(x, y, (int)n);
+        c->launches++;
+        return y;
+    }
+}
+
 // AssembleSystem: k_imp_assemble (per particle), k_imp_rhs_diag, k_imp_scale
 template <typename R>
 static void launch_assemble(mpm_ctx *c, const ImpArgs &a) {
     ImpState *s = c->imp;
     const PView<R> P = pview<R>(c);
     R *A = (R *)s->A, *sk = (R *)s->stress_k;
+    const R *nd = nodal_of<R>(c, s->ndispl, 0, 3 * (size_t)c->g.nodec);
     const int pb = (int)((c->num + 127) / 128);
     const int *o = c->g.order;
-    if (o[0] == 1 && o[1] == 1 && o[2] == 1)
-        k_imp_assemble<R, 1, 1, 1><<<pb, 128, 0, c->stream>>>(a, P, s->ndispl, sk, A, s->b);
+    bool cells = false;
+    if constexpr (sizeof(R) == 4) {
+        cells = s->isotropic && c->cell_scatter;
+        auto go = [&](auto shape, auto k) {
+            using C = decltype(shape);
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+            k<<<c->g.nbricks * (BRC / C::CELLS), C::THREADS, C::SMEM, c->stream>>>(
+                a, P, nd, sk, A, s->b, c->d_cstart, c->d_blist, c->d_nblist, c->g.nbrick[0], c->g.nbrick[1]);
+        };
+        if (cells && o[0] == 1) go(AsmShape<1, 1, 1>(), k_imp_assemble_cells<1, 1, 1>);
+        else if (cells && o[1] == 2) go(AsmShape<2, 2, 2>(), k_imp_assemble_cells<2, 2, 2>);
+        else if (cells) go(AsmShape<2, 1, 2>(), k_imp_assemble_cells<2, 1, 2>);
+    }
+    if (cells) {
+    } else if (o[0] == 1 && o[1] == 1 && o[2] == 1)
+        k_imp_assemble<R, 1, 1, 1><<<pb, 128, 0, c->stream>>>(a, P, nd, sk, A, s->b);
     else if (o[1] == 2)
-        k_imp_assemble<R, 2, 2, 2><<<pb, 128, 0, c->stream>>>(a, P, s->ndispl, sk, A, s->b);
+        k_imp_assemble<R, 2, 2, 2><<<pb, 128, 0, c->stream>>>(a, P, nd, sk, A, s->b);
     else
-        k_imp_assemble<R, 2, 1, 2><<<pb, 128, 0, c->stream>>>(a, P, s->ndispl, sk, A, s->b);
+        k_imp_assemble<R, 2, 1, 2><<<pb, 128, 0, c->stream>>>(a, P, nd, sk, A, s->b);
     k_imp_rhs_diag<R><<<nb_nodes(c), 256, 0, c->stream>>>(a, A, s->nmass, s->naccel_k, s->naccel, s->b, s->adiag);
     k_imp_scale<R><<<nb_nodes(c), 256, 0, c->stream>>>(a, A, s->adiag);
 }
@@ -1800,15 +2052,18 @@ static void launch_g2p(mpm_ctx *c, const ImpArgs &a, int parity, int pb) {
     ImpState *s = c->imp;
     const PView<R> P = pview<R>(c);
     R *geup = (R *)s->geup;
+    const size_t N = (size_t)c->g.nodec;
+    const R *nd = nodal_of<R>(c, s->ndispl, 0, 3 * N), *nv = nodal_of<R>(c, s->nvel, 3 * N, 3 * N),
+            *na = nodal_of<R>(c, s->naccel, 6 * N, 3 * N), *ne = nodal_of<R>(c, s->nei, 9 * N, N);
     const int *o = c->g.order;
     if (o[0] == 1 && o[1] == 1 && o[2] == 1)
-        k_imp_g2p<R, 1, 1, 1><<<pb, 128, 0, c->stream>>>(a, P, s->ndispl, s->nvel, s->naccel, s->nei, geup, s->part,
+        k_imp_g2p<R, 1, 1, 1><<<pb, 128, 0, c->stream>>>(a, P, nd, nv, na, ne, geup, s->part,
                                                           c->d_ctl, parity);
     else if (o[1] == 2)
-        k_imp_g2p<R, 2, 2, 2><<<pb, 128, 0, c->stream>>>(a, P, s->ndispl, s->nvel, s->naccel, s->nei, geup, s->part,
+        k_imp_g2p<R, 2, 2, 2><<<pb, 128, 0, c->stream>>>(a, P, nd, nv, na, ne, geup, s->part,
                                                           c->d_ctl, parity);
     else
-        k_imp_g2p<R, 2, 1, 2><<<pb, 128, 0, c->stream>>>(a, P, s->ndispl, s->nvel, s->naccel, s->nei, geup, s->part,
+        k_imp_g2p<R, 2, 1, 2><<<pb, 128, 0, c->stream>>>(a, P, nd, nv, na, ne, geup, s->part,
                                                           c->d_ctl, parity);
     k_finish<<<1, 256, 0, c->stream>>>(s->part, pb, s->scal, S_GD);
     k_imp_shift<R><<<pb, 128, 0, c->stream>>>(a, P, geup, s->scal);
