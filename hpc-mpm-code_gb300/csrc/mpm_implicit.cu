@@ -78,6 +78,8 @@ struct ImpState {
     double *gp = nullptr, *gq = nullptr;    // flexible GCR: GM directions and their images (GM * 3 * nodec)
     double *gqq = nullptr, *gbeta = nullptr;  // |A p|^2 of each kept direction, projection coefficients
     float *gqf = nullptr;                   // FP32 copies of the kept images (GM * 3 * nodec), for the dots
+    size_t gst = 0;                         // values per direction slot: 3 * nodec, up to a multiple of four
+    int64_t gcr_launches = 0;               // launches in g_gcr
     float *gp32 = nullptr, *gq32 = nullptr;  // FP32 operator: the directions and images in FP32 (GM * 3 * nodec)
     float *p32 = nullptr;                   // FP32 operator: the CG direction in FP32
     float *nf32 = nullptr;                  // FP32 copies of ndispl, nvel, naccel (3 N each) and nei (N) for the particles
@@ -99,7 +101,7 @@ namespace mpm {
 
 constexpr int GM = 8;   // directions kept by the flexible GCR solver
 
-enum Scal { S_RR0 = 0, S_RR1, S_PAP, S_RR_INIT, S_RES, S_IDOF, S_EU, S_GD, S_ZQ, S_PR, S_RRC, S_DZZ, S_DZR, S_QR, S_QQ, S_THR, S_ITER, S_DONE, S_ALPHA, S_BETA, S_NSCAL };
+enum Scal { S_RR0 = 0, S_RR1, S_PAP, S_RR_INIT, S_RES, S_IDOF, S_EU, S_GD, S_ZQ, S_PR, S_RRC, S_DZZ, S_DZR, S_THR, S_ITER, S_DONE, S_ALPHA, S_BETA, S_NSCAL };
 
 struct ImpArgs {
     int nnc[3];
@@ -873,6 +875,29 @@ __device__ __forceinline__ bool partials_last(const double (&vin)[V], int nv, do
     return s_last;
 }
 
+// in the last block: thread j < nv gets the total of value j over all blocks.  All
+// values are read at once (a reduction per value waited for memory once each).
+template <int V>
+__device__ __forceinline__ double last_sums(const double *part, int nv) {
+    __shared__ double sh[V][8];   // CTAs of at most 8 warps
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double t[V];
+#pragma unroll
+    for (int j = 0; j < V; j++) t[j] = 0.0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x)
+#pragma unroll
+        for (int j = 0; j < V; j++)
+            if (j < nv) t[j] += __ldcg(part + (size_t)j * gridDim.x + i);
+    const int jv = warp_sums<V>(t);
+    if ((lane & (32 / V - 1)) == 0) sh[jv][wid] = t[0];
+    __syncthreads();
+    double s = 0.0;
+    if ((int)threadIdx.x < nv)
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += sh[threadIdx.x][w];
+    return s;
+}
+
 // in the last block: the total of value j over all blocks (thread 0)
 __device__ __forceinline__ double last_sum(const double *part, int j, double *sh32) {
     double acc = 0.0;
@@ -888,15 +913,12 @@ __global__ void k_finish(const double *part, int nblk, double *out, int slot) {
     if (threadIdx.x == 0) out[slot] = t;
 }
 
-// y = A x with BC rows zeroed (MatVecMult + BCResidualSet), optional dot(x, y).
-// TA: storage of A; TC: arithmetic (FP32 in the Krylov iterations of the
-// FP32 operator, FP64 for its true residual and in the FP64 mode); TV: the
-// vectors x and y (FP64, or FP32 for the flexible GCR directions of the FP32
-// operator).  RX, RY, RZ: the stencil radius per axis.
-template <typename TA, typename TC, int RX, int RY, int RZ, typename TV = double, typename TY = TV>
-__global__ void __launch_bounds__(256) k_imp_matvec(ImpArgs a, const TA *A, const TV *x, TY *y,
-                                                    double *part, unsigned *cnt = nullptr, double *scal = nullptr,
-                                                    int slot = 0, int num = -1, const double *xd = nullptr) {
+// y = A x with BC rows zeroed (MatVecMult + BCResidualSet), optionally the block
+// sums of dot(x, y) in part.  TA: storage of A; TC: arithmetic.  RX, RY, RZ: the
+// stencil radius per axis.
+template <typename TA, typename TC, int RX, int RY, int RZ>
+__global__ void __launch_bounds__(256) k_imp_matvec(ImpArgs a, const TA *A, const double *x, double *y,
+                                                    double *part) {
     using TA2 = typename std::conditional<sizeof(TA) == 8, double2, float2>::type;
     constexpr int SX = 2 * RX + 1, SY = 2 * RY + 1, NS = SX * SY * (2 * RZ + 1);
     __shared__ double sh[32];
@@ -940,21 +962,11 @@ __global__ void __launch_bounds__(256) k_imp_matvec(ImpArgs a, const TA *A, cons
         const unsigned char bf = a.bcflag[n];
         for (int c = 0; c < 3; c++) {
             const double v = (bf & (1 << c)) ? 0.0 : (double)acc[c];
-            y[c * N + n] = (TY)v;
-            if constexpr (sizeof(TV) != sizeof(TY)) dot += xd[c * N + n] * v;   // x is a copy of xd
-            else dot += (double)x[c * N + n] * v;
+            y[c * N + n] = v;
+            if (part) dot += x[c * N + n] * v;
         }
     }
-    if (part && cnt) {   // dot(x, y) reduced by the last block into scal[slot]
-        const double v[1] = {dot};
-        if (!partials_last<1>(v, 1, part, cnt)) return;
-        const double t = last_sum(part, 0, sh);
-        if (threadIdx.x == 0) {
-            scal[slot] = t;
-            if (num >= 0) scal[S_ALPHA] = t != 0.0 ? scal[num] / t : 0.0;
-            *cnt = 0u;
-        }
-    } else if (part) {
+    if (part) {
         const double t = block_sum(dot, sh);
         if (threadIdx.x == 0) part[blockIdx.x] = t;
     }
@@ -962,7 +974,7 @@ __global__ void __launch_bounds__(256) k_imp_matvec(ImpArgs a, const TA *A, cons
 
 // The same product with MV_G threads per control point, each of SL neighbouring
 // slots (an even number, so that its entries start on a pair), added in order
-// through shared memory (mv_split says when).
+// through shared memory.
 // x in the precision TV of the arithmetic's input, y in TY; with `part`, the dot
 // product of xd (FP64) and y goes to scal[slot] and scal[num] divided by it to
 // S_ALPHA (num >= 0).  `done`: nothing to do when set.
@@ -977,7 +989,6 @@ __global__ void __launch_bounds__(MV_NODES * MV_G)
     constexpr int SL = 2 * ((NS + 2 * MV_G - 1) / (2 * MV_G));
     static_assert(SL * MV_G >= NS, "every slot has a thread");
     __shared__ TC sh[MV_G][3][MV_NODES];
-    __shared__ double shd[32];
     pdl_wait();
     if (done && *done != 0.0) return;   // uniform over the grid
     const int lane = threadIdx.x % MV_NODES, grp = threadIdx.x / MV_NODES;
@@ -1031,7 +1042,7 @@ __global__ void __launch_bounds__(MV_NODES * MV_G)
     if (part) {
         const double v[1] = {dot};
         if (!partials_last<1>(v, 1, part, cnt)) return;
-        const double t = last_sum(part, 0, shd);
+        const double t = last_sums<1>(part, 1);
         if (threadIdx.x == 0) {
             scal[slot] = t;
             if (num >= 0) scal[S_ALPHA] = t != 0.0 ? scal[num] / t : 0.0;
@@ -1163,6 +1174,70 @@ __device__ __forceinline__ double block_div(double num, double den, bool zero = 
     return s_q;
 }
 
+// Four neighbouring values of a vector of m (a direction's slot starts on 16 bytes),
+// zero past its end.
+__device__ __forceinline__ void ld4(float (&v)[4], const float *p, int i, int m) {
+    if (i + 4 <= m) {
+        const float4 q = *reinterpret_cast<const float4 *>(p + i);
+        v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++) v[e] = i + e < m ? p[i + e] : 0.0f;
+    }
+}
+__device__ __forceinline__ void ld4(double (&v)[4], const double *p, int i, int m) {
+    if (i + 4 <= m) {
+        const double2 a = *reinterpret_cast<const double2 *>(p + i), b = *reinterpret_cast<const double2 *>(p + i + 2);
+        v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++) v[e] = i + e < m ? p[i + e] : 0.0;
+    }
+}
+__device__ __forceinline__ void st4(float *p, const float (&v)[4], int i, int m) {
+    if (i + 4 <= m) {
+        *reinterpret_cast<float4 *>(p + i) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (i + e < m) p[i + e] = v[e];
+    }
+}
+__device__ __forceinline__ void st4(double *p, const double (&v)[4], int i, int m) {
+    if (i + 4 <= m) {
+        *reinterpret_cast<double2 *>(p + i) = make_double2(v[0], v[1]);
+        *reinterpret_cast<double2 *>(p + i + 2) = make_double2(v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (i + e < m) p[i + e] = v[e];
+    }
+}
+
+// p.Ap to S_PAP and alpha = scal[cur] / p.Ap to S_ALPHA, where the product does not
+// form it (mv_dot)
+__global__ void __launch_bounds__(256) k_cg_dot(const double *p, const double *Ap, int m, double *part, unsigned *cnt,
+                                                double *scal, int cur, const double *done) {
+    pdl_wait();
+    if (done && *done != 0.0) return;   // uniform over the grid
+    const int i = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    double v[1] = {0.0};
+    if (i < m) {
+        double x[4], y[4];
+        ld4(x, p, i, m);
+        ld4(y, Ap, i, m);
+#pragma unroll
+        for (int e = 0; e < 4; e++) v[0] = fma(x[e], y[e], v[0]);
+    }
+    if (!partials_last<1>(v, 1, part, cnt)) return;
+    const double t = last_sums<1>(part, 1);
+    if (threadIdx.x == 0) {
+        scal[S_PAP] = t;
+        scal[S_ALPHA] = t != 0.0 ? scal[cur] / t : 0.0;
+        *cnt = 0u;
+    }
+}
+
 // x += alpha p, r -= alpha Ap, then (last block) r.r and beta;  alpha = rr_cur / pAp
 // and beta = rr_new / rr_cur are divided once, by the block that reduced them.
 // stop: the pass belongs to a solve that ends itself: nothing to do once S_DONE is
@@ -1171,7 +1246,6 @@ __device__ __forceinline__ double block_div(double num, double den, bool zero = 
 __global__ void __launch_bounds__(256) k_cg_update(ImpArgs a, double *scal, int cur, double *x, double *r,
                                                    const double *p, const double *Ap, double *part, unsigned *cnt,
                                                    int stop) {
-    __shared__ double sh[32];
     pdl_wait();
     if (stop && scal[S_DONE] != 0.0) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1198,7 +1272,7 @@ __global__ void __launch_bounds__(256) k_cg_update(ImpArgs a, double *scal, int 
     }
     const double v[1] = {dot};
     if (!partials_last<1>(v, 1, part, cnt)) return;
-    const double t = last_sum(part, 0, sh);
+    const double t = last_sums<1>(part, 1);
     if (threadIdx.x == 0) {
         scal[cur ^ 1] = t;
         scal[S_BETA] = scal[cur] != 0.0 ? t / scal[cur] : 0.0;
@@ -1612,43 +1686,47 @@ __global__ void k_set_modulus(double *matprop, int nmat, double E) {
 // slot of the direction kept j + 1 iterations before the one in `slot` (ring of w)
 __device__ __forceinline__ int gcr_prev(int slot, int j, int w) { return (slot - 1 - j + 2 * w) % w; }
 
-// partial dots q . Q_j with the `used` previous images (j = 0 the newest)
-// Per-block partial sums of nv (<= V) values into part[j * gridDim.x + b];
-// true in the last block to finish (the blocks count themselves on *cnt),
-// which then reduces the partials in block order (last_sum), so the sums
-// are reproducible without a separate reduction launch.
-// flexible GCR: the dots q . Q_j of the new image with the kept ones, then
-// (last block) beta_j = (q . Q_j) / (Q_j . Q_j).  beta only has to be close:
-// the same beta_j update both the direction and its image (k_gcr_axpy, in
-// FP64), so A p = q holds whatever their accuracy and only the
-// orthogonality of the kept images is at FP32 level.  So the dots run in
-// FP32 on FP32 copies of the kept images (the FP64 pipe is this part's
+// The three passes of a flexible GCR iteration after the product q = A p.  Each is
+// a pass over vectors that mostly sit in L2 (17, 46 and 42 MB at 274,625 nodes, FP32)
+// and a reduction that its last block finishes; what they took was the chain of
+// loads per thread and the last block's one reduction per value.  So a thread
+// takes four neighbouring values with every load issued before the first use, the
+// last block reads all partials at once, and each pass is launched while its
+// predecessor drains.  Dots, axpy and update, 1,728,000 particles: 18.4 + 24.4 + 19.8 ->
+// 11.0 + 21.4 + 15.8 us (the last with the network's input pass, 8.0 before).
+//
+// beta_j = (q . Q_j) / (Q_j . Q_j) with the `used` previous images (j = 0 the
+// newest; W >= the window w).  beta only has to be close: the same beta_j update
+// both the direction and its image (k_gcr_axpy), so A p = q holds whatever their
+// accuracy and only the orthogonality of the kept images is at FP32 level.  So the
+// dots run in FP32 on FP32 copies of the kept images (the FP64 pipe is this part's
 // scarce resource), and the block partials are summed in FP64.
-template <typename T>
-__global__ void __launch_bounds__(256) k_gcr_dots(ImpArgs a, const T *Q, const float *Qf, int slot, int used,
+template <typename T, int W>
+__global__ void __launch_bounds__(256) k_gcr_dots(const T *Q, const float *Qf, size_t st, int m, int slot, int used,
                                                   int w, double *part, unsigned *cnt, const double *qq,
                                                   double *beta) {
-    __shared__ double sh[32];
-    __shared__ double shw[GM][8];
+    __shared__ double shw[W][8];
     __shared__ bool s_last;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t N = (size_t)a.nodec, st = 3 * N;
-    float d[GM];
+    pdl_wait();
+    const int i = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    float d[W];
 #pragma unroll
-    for (int j = 0; j < GM; j++) d[j] = 0.0f;
-    if (n < a.nodec) {
-        const T *q = Q + (size_t)slot * st;
-        const float q0 = (float)q[n], q1 = (float)q[N + n], q2 = (float)q[2 * N + n];
+    for (int j = 0; j < W; j++) d[j] = 0.0f;
+    if (i < m) {
+        T q[4];
+        float qj[W][4];
+        ld4(q, Q + (size_t)slot * st, i, m);
 #pragma unroll
-        for (int j = 0; j < GM; j++)
-            if (j < used) {
-                const float *qj = Qf + (size_t)gcr_prev(slot, j, w) * st;
-                d[j] = q0 * qj[n] + q1 * qj[N + n] + q2 * qj[2 * N + n];
-            }
+        for (int j = 0; j < W; j++)   // past `used`: any slot, the dot is not used
+            ld4(qj[j], Qf + (size_t)(j < used ? gcr_prev(slot, j, w) : slot) * st, i, m);
+#pragma unroll
+        for (int j = 0; j < W; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) d[j] += (float)q[e] * qj[j][e];
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int jv = warp_sums<GM>(d);
-    if ((lane & (32 / GM - 1)) == 0) shw[jv][wid] = (double)d[0];
+    const int jv = warp_sums<W>(d);
+    if ((lane & (32 / W - 1)) == 0) shw[jv][wid] = (double)d[0];
     __syncthreads();
     if ((int)threadIdx.x < used) {
         double t = 0.0;
@@ -1661,89 +1739,146 @@ __global__ void __launch_bounds__(256) k_gcr_dots(ImpArgs a, const T *Q, const f
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    for (int j = 0; j < used; j++) {
-        const double t = last_sum(part, j, sh);
-        if (threadIdx.x == 0) {
-            const double dq = qq[gcr_prev(slot, j, w)];
-            beta[j] = dq > 0.0 ? t / dq : 0.0;
-        }
+    const double t = last_sums<W>(part, used);
+    if ((int)threadIdx.x < used) {
+        const double dq = qq[gcr_prev(slot, threadIdx.x, w)];
+        beta[threadIdx.x] = dq > 0.0 ? t / dq : 0.0;
     }
     if (threadIdx.x == 0) *cnt = 0u;
 }
 
-// p -= sum beta_j P_j, q -= sum beta_j Q_j in the precision T of the
-// directions (FP64: an FP32 copy of q is kept for the dots; FP32: the images
-// themselves are what the dots read, Qf is null); then (last block) q.r and
-// q.q in FP64
-template <typename T>
-__global__ void __launch_bounds__(256) k_gcr_axpy(ImpArgs a, T *P, T *Q, float *Qf, int slot, int used,
-                                                  int w, const double *beta, const double *r, double *part,
-                                                  unsigned *cnt, double *scal) {
-    __shared__ double sh[32];
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t N = (size_t)a.nodec, st = 3 * N;
+// p -= sum beta_j P_j, q -= sum beta_j Q_j in the precision T of the directions
+// (FP64: an FP32 copy of q is kept for the dots; FP32: the images themselves are
+// what the dots read, Qf is null); then (last block) q.r, q.q (kept as the slot's)
+// and alpha = q.r / q.q.
+// rr: r.r after the coming update, r.r - (q.r)^2 / q.q, goes to S_RRC (the update
+// then needs no reduction and can feed the network).  It is used where r is
+// replaced by the true residual every few iterations (the FP32 operator): within
+// those r.r falls by far less than the 2^52 that the difference could lose.
+template <typename T, int W>
+__global__ void __launch_bounds__(256) k_gcr_axpy(T *P, T *Q, float *Qf, size_t st, int m, int slot, int used, int w,
+                                                  const double *beta, const double *r, double *qqs, double *part,
+                                                  unsigned *cnt, double *scal, int rr) {
+    pdl_wait();
+    const int i = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     double v[2] = {0.0, 0.0};
-    if (n < a.nodec) {
+    if (i < m) {
         T *p = P + (size_t)slot * st, *q = Q + (size_t)slot * st;
-        T bj[GM];
+        T pv[4], qv[4], pj[W][4], qj[W][4], bj[W];
+        double rv[4];
+        ld4(pv, p, i, m);
+        ld4(qv, q, i, m);
+        ld4(rv, r, i, m);
 #pragma unroll
-        for (int j = 0; j < GM; j++) bj[j] = j < used ? (T)beta[j] : (T)0;
-        for (int c = 0; c < 3; c++) {
-            const size_t i = c * N + n;
-            T pv = p[i], qv = q[i];
+        for (int j = 0; j < W; j++) {
+            const size_t o = (size_t)(j < used ? gcr_prev(slot, j, w) : slot) * st;
+            ld4(pj[j], P + o, i, m);
+            ld4(qj[j], Q + o, i, m);
+            bj[j] = j < used ? (T)beta[j] : (T)0;
+        }
 #pragma unroll
-            for (int j = 0; j < GM; j++)
-                if (j < used) {
-                    const size_t o = (size_t)gcr_prev(slot, j, w) * st + i;
-                    pv -= bj[j] * P[o];
-                    qv -= bj[j] * Q[o];
+        for (int j = 0; j < W; j++)
+            if (j < used)
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    pv[e] -= bj[j] * pj[j][e];
+                    qv[e] -= bj[j] * qj[j][e];
                 }
-            p[i] = pv;
-            q[i] = qv;
-            if (Qf) Qf[(size_t)slot * st + i] = (float)qv;   // the copy k_gcr_dots reads
-            v[0] += (double)qv * r[i];
-            v[1] += (double)qv * (double)qv;
+        st4(p, pv, i, m);
+        st4(q, qv, i, m);
+        if (Qf) {   // the copy k_gcr_dots reads
+            float qf[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) qf[e] = (float)qv[e];
+            st4(Qf + (size_t)slot * st, qf, i, m);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const double qd = (double)qv[e];
+            v[0] = fma(qd, rv[e], v[0]);
+            v[1] = fma(qd, qd, v[1]);
         }
     }
     if (!partials_last<2>(v, 2, part, cnt)) return;
-    const double qr = last_sum(part, 0, sh);
-    const double qq = last_sum(part, 1, sh);
+    __shared__ double s_t[2];
+    const double t = last_sums<2>(part, 2);
+    if (threadIdx.x < 2) s_t[threadIdx.x] = t;
+    __syncthreads();
     if (threadIdx.x == 0) {
-        scal[S_QR] = qr;
-        scal[S_QQ] = qq;
+        const double qr = s_t[0], qq = s_t[1], alpha = qq > 0.0 ? qr / qq : 0.0;
+        scal[S_ALPHA] = alpha;
+        qqs[slot] = qq;
+        if (rr) {
+            const double left = scal[S_RRC] - alpha * qr;
+            scal[S_RRC] = left < 0.0 ? 0.0 : left;   // keeps a NaN
+        }
         *cnt = 0u;
     }
 }
 
-// alpha = q.r / q.q; x += alpha p; r -= alpha q; keeps q.q of the slot; then
-// (last block) r.r
+// x += alpha p; r -= alpha q; then (last block) r.r
 template <typename T>
-__global__ void __launch_bounds__(256) k_gcr_update(ImpArgs a, double *scal, double *x, double *r, const T *P,
-                                                    const T *Q, int slot, double *qq, double *part,
-                                                    unsigned *cnt) {
-    __shared__ double sh[32];
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t N = (size_t)a.nodec, st = 3 * N;
-    const double dqq = scal[S_QQ];
-    const double alpha = block_div(scal[S_QR], dqq, !(dqq > 0.0));
-    if (blockIdx.x == 0 && threadIdx.x == 0) qq[slot] = dqq;
+__global__ void __launch_bounds__(256) k_gcr_update(double *scal, double *x, double *r, const T *P, const T *Q,
+                                                    size_t st, int m, int slot, double *part, unsigned *cnt) {
+    pdl_wait();
+    const int i = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    const double alpha = scal[S_ALPHA];
     double v[1] = {0.0};
-    if (n < a.nodec) {
-        const T *p = P + (size_t)slot * st, *q = Q + (size_t)slot * st;
-        for (int c = 0; c < 3; c++) {
-            const size_t i = c * N + n;
-            x[i] += alpha * (double)p[i];
-            const double w = r[i] - alpha * (double)q[i];
-            r[i] = w;
-            v[0] += w * w;
+    if (i < m) {
+        T p[4], q[4];
+        double xv[4], rv[4];
+        ld4(p, P + (size_t)slot * st, i, m);
+        ld4(q, Q + (size_t)slot * st, i, m);
+        ld4(xv, x, i, m);
+        ld4(rv, r, i, m);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            xv[e] += alpha * (double)p[e];
+            rv[e] -= alpha * (double)q[e];
+            v[0] += rv[e] * rv[e];
         }
+        st4(x, xv, i, m);
+        st4(r, rv, i, m);
     }
     if (!partials_last<1>(v, 1, part, cnt)) return;
-    const double rr = last_sum(part, 0, sh);
+    const double rr = last_sums<1>(part, 1);
     if (threadIdx.x == 0) {
         scal[S_RRC] = rr;
         *cnt = 0u;
     }
+}
+
+// The same for the FP32 operator, whose r.r k_gcr_axpy left: no reduction, and the
+// new residual goes straight into the network's input (feed; the next iteration's
+// first pass, k_input_r, is then not needed).
+__global__ void __launch_bounds__(256) k_gcr_update_feed(const double *scal, double *x, double *r,
+                                                         const float *__restrict__ P, const float *__restrict__ Q,
+                                                         size_t st, int nodec, int slot, int feed, nn::Input in) {
+    __shared__ double s_inv;
+    pdl_wait();
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t N = (size_t)nodec;
+    if (threadIdx.x == 0) s_inv = nn::inv_rms(scal[S_RRC], nodec);
+    __syncthreads();
+    if (n >= nodec) return;
+    const double alpha = scal[S_ALPHA], inv = s_inv;
+    const float *p = P + (size_t)slot * st + n, *q = Q + (size_t)slot * st + n;
+    double xv[3], rv[3];
+    float pv[3], qv[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        pv[c] = p[c * N];
+        qv[c] = q[c * N];
+        xv[c] = x[c * N + n];
+        rv[c] = r[c * N + n];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        x[c * N + n] = xv[c] + alpha * (double)pv[c];
+        rv[c] -= alpha * (double)qv[c];
+        r[c * N + n] = rv[c];
+    }
+    if (feed) nn::store_input(in, n, (float)(rv[0] * inv), (float)(rv[1] * inv), (float)(rv[2] * inv));
 }
 
 __global__ void k_imp_reset_next(DevCtl *ctl, int parity) {
@@ -1872,14 +2007,15 @@ mpm_status mpm_gpu_implicit_setup(mpm_ctx *c, int nr_flag, double spec_rad) {
     double **vec3[] = {&s->adiag, &s->b,    &s->x,       &s->r, &s->p,  &s->Ap,    &s->xs, &s->ndispl,
                        &s->nvel,  &s->naccel, &s->naccel_k, &s->z, &s->bs, &s->xstar, &s->ev};
     for (double **v : vec3) CKI(cudaMalloc((void **)v, sizeof(double) * 3 * N));
-    CKI(cudaMalloc((void **)&s->gp, sizeof(double) * GM * 3 * N));
-    CKI(cudaMalloc((void **)&s->gq, sizeof(double) * GM * 3 * N));
+    s->gst = (3 * N + 3) & ~(size_t)3;
+    CKI(cudaMalloc((void **)&s->gp, sizeof(double) * GM * s->gst));
+    CKI(cudaMalloc((void **)&s->gq, sizeof(double) * GM * s->gst));
     CKI(cudaMalloc((void **)&s->gqq, sizeof(double) * GM));
     CKI(cudaMalloc((void **)&s->gbeta, sizeof(double) * GM));
-    CKI(cudaMalloc((void **)&s->gqf, sizeof(float) * GM * 3 * N));
+    CKI(cudaMalloc((void **)&s->gqf, sizeof(float) * GM * s->gst));
     if (s->prec == 32) {
-        CKI(cudaMalloc((void **)&s->gp32, sizeof(float) * GM * 3 * N));
-        CKI(cudaMalloc((void **)&s->gq32, sizeof(float) * GM * 3 * N));
+        CKI(cudaMalloc((void **)&s->gp32, sizeof(float) * GM * s->gst));
+        CKI(cudaMalloc((void **)&s->gq32, sizeof(float) * GM * s->gst));
         CKI(cudaMalloc((void **)&s->p32, sizeof(float) * 3 * N));
         CKI(cudaMalloc((void **)&s->nf32, sizeof(float) * 10 * N));
         if (!getenv("MPM_GB300_TRUE_RESIDUAL_FP64")) CKI(cudaMalloc((void **)&s->dfx, sizeof(float) * 2 * 3 * N));
@@ -1906,9 +2042,8 @@ static int nb_nodes(mpm_ctx *c) { return (c->g.nodec + 255) / 256; }
 // y = A x on the context's stream (k_imp_matvec for the context's matrix
 // precision and stencil); hi: FP64 arithmetic whatever the storage (the
 // true residual and the Newton check of the FP32 operator).
-static void launch_matvec(mpm_ctx *c, const ImpArgs &a, int nb, const double *x, double *y, double *part,
-                          unsigned *cnt = nullptr, double *scal = nullptr, int slot = 0, bool hi = false,
-                          int num = -1) {
+static void launch_matvec(mpm_ctx *c, const ImpArgs &a, int nb, const double *x, double *y,
+                          double *part = nullptr, bool hi = false) {
     ImpState *s = c->imp;
     const int *o = c->g.order;
     auto go = [&](auto ta, auto tc) {
@@ -1916,11 +2051,11 @@ static void launch_matvec(mpm_ctx *c, const ImpArgs &a, int nb, const double *x,
         using TC = decltype(tc);
         const TA *A = (const TA *)s->A;
         if (o[0] == 1 && o[1] == 1 && o[2] == 1)
-            k_imp_matvec<TA, TC, 1, 1, 1><<<nb, 256, 0, c->stream>>>(a, A, x, y, part, cnt, scal, slot, num);
+            k_imp_matvec<TA, TC, 1, 1, 1><<<nb, 256, 0, c->stream>>>(a, A, x, y, part);
         else if (o[1] == 2)
-            k_imp_matvec<TA, TC, 2, 2, 2><<<nb, 256, 0, c->stream>>>(a, A, x, y, part, cnt, scal, slot, num);
+            k_imp_matvec<TA, TC, 2, 2, 2><<<nb, 256, 0, c->stream>>>(a, A, x, y, part);
         else
-            k_imp_matvec<TA, TC, 2, 1, 2><<<nb, 256, 0, c->stream>>>(a, A, x, y, part, cnt, scal, slot, num);
+            k_imp_matvec<TA, TC, 2, 1, 2><<<nb, 256, 0, c->stream>>>(a, A, x, y, part);
     };
     if (s->prec == 64) {
         go(double(), double());
@@ -1942,14 +2077,15 @@ static void launch_matvec(mpm_ctx *c, const ImpArgs &a, int nb, const double *x,
     }
 }
 
-// Whether a CG product runs with MV_G threads per control point.  It does where
-// one thread per point leaves the chip short of loads in flight: per product,
-// split against not, 11.7 against 19.6 us (FP32, 1,690 points), 18.6 against 22.1
-// (FP32, 46,305), 37.5 against 50.8 (FP64, 46,305), 18.7 against 32.1 (FP32
-// B-spline stencil, 24,000).  On a large grid the reduction of the dot product over eight times
-// as many CTAs costs more than that: 86 against 65 us (FP32) and 174 against 152
-// (FP64) at 274,625 points.
-static bool mv_split(const mpm_ctx *c) { return c->g.nodec <= 100000; }
+// Whether a CG product forms p.Ap itself.  MV_G threads per control point give it
+// eight times as many CTAs as a pass over vectors has, and on a large grid their
+// partials cost more than a pass of its own over p and Ap: per product, with its own dot
+// against a separate one, 18.8 against 17.1 us (FP32) and 38.1 against 35.3 (FP64) at
+// 46,305 points, 86 against 63.4 (FP32) at 274,625; but 10.9 against 12.6 at 1,690 and
+// 18.8 against 19.6 at 24,000 (B-spline stencil).
+// (One thread per point: 19.6 us FP32 at 1,690 points, 22.1 at 46,305, 65 at
+// 274,625; FP64 50.8 and 153 where the split takes 35.3 and 143.)
+static bool mv_dot(const mpm_ctx *c) { return c->g.nodec <= 32768; }
 
 template <typename TA, typename TC, typename TV, typename TY>
 static void launch_split(mpm_ctx *c, const ImpArgs &a, const TV *x, TY *y, const double *xd, double *part,
@@ -1975,21 +2111,18 @@ static void launch_matvec_f32(mpm_ctx *c, const ImpArgs &a, const float *x, floa
 static void launch_matvec_cg(mpm_ctx *c, const ImpArgs &a, int nb, int cur, const double *done) {
     ImpState *s = c->imp;
     const int *o = c->g.order;
-    if (!mv_split(c) && s->prec == 64)
-        launch_matvec(c, a, nb, s->p, s->Ap, s->part, s->cnt + 3, s->scal, S_PAP, false, cur);
-    else if (!mv_split(c)) {
-        auto go = [&](auto k) {
-            k<<<nb, 256, 0, c->stream>>>(a, (const float *)s->A, (const float *)s->p32, s->Ap, s->part, s->cnt + 3,
-                                         s->scal, S_PAP, cur, (const double *)s->p);
-        };
-        if (o[0] == 1 && o[1] == 1 && o[2] == 1) go(k_imp_matvec<float, float, 1, 1, 1, float, double>);
-        else if (o[1] == 2) go(k_imp_matvec<float, float, 2, 2, 2, float, double>);
-        else go(k_imp_matvec<float, float, 2, 1, 2, float, double>);
-    }
-    else if (s->prec == 64)
-        launch_split<double, double>(c, a, (const double *)s->p, s->Ap, s->p, s->part, s->cnt + 3, s->scal, S_PAP, cur, done);
+    const bool dot = mv_dot(c);
+    double *part = dot ? s->part : nullptr;
+    if (s->prec == 64)
+        launch_split<double, double>(c, a, (const double *)s->p, s->Ap, s->p, part, s->cnt + 3, s->scal, S_PAP, cur, done);
     else
-        launch_split<float, float>(c, a, (const float *)s->p32, s->Ap, s->p, s->part, s->cnt + 3, s->scal, S_PAP, cur, done);
+        launch_split<float, float>(c, a, (const float *)s->p32, s->Ap, s->p, part, s->cnt + 3, s->scal, S_PAP, cur, done);
+    if (!dot) {
+        const int m = 3 * c->g.nodec;
+        launch(true, k_cg_dot, (m + 1023) / 1024, 256, 0, c->stream, (const double *)s->p, (const double *)s->Ap, m,
+               s->part, s->cnt + 3, s->scal, cur, done);
+        c->launches++;
+    }
 }
 
 // FP32 copies of nodal fields, so that the FP32 particles' gathers convert each
@@ -2154,7 +2287,7 @@ static mpm_status imp_cg(mpm_ctx *c, double eps, int kmax, int *iters) {
     k_cg_scale_in<<<nb, 256, 0, c->stream>>>(a, s->x, s->b, s->adiag, s->xs, s->r);
     if (s->prec == 32)   // the scaled RHS, for the true residual of the FP32 operator
         CKI(cudaMemcpyAsync(s->bs, s->r, sizeof(double) * 3 * c->g.nodec, cudaMemcpyDeviceToDevice, c->stream));
-    launch_matvec(c, a, nb, s->xs, s->Ap, nullptr, nullptr, nullptr, 0, true);
+    launch_matvec(c, a, nb, s->xs, s->Ap, nullptr, true);
     k_cg_init<<<nb, 256, 0, c->stream>>>(a, s->Ap, s->r, s->p, s->part);
     k_finish<<<1, 256, 0, c->stream>>>(s->part, nb, s->scal, S_RR0);
     c->launches += 4;
@@ -2206,7 +2339,7 @@ static mpm_status imp_cg(mpm_ctx *c, double eps, int kmax, int *iters) {
             // old direction instead diverged: at this point the recursive
             // residual, and with it p, has fallen far below the true
             // residual, so alpha = r.r / p.Ap overshoots.
-            launch_matvec(c, a, nb, s->xs, s->z, nullptr, nullptr, nullptr, 0, true);
+            launch_matvec(c, a, nb, s->xs, s->z, nullptr, true);
             k_true_residual<<<nb, 256, 0, c->stream>>>(a, s->bs, s->z, s->r, s->part);
             k_finish<<<1, 256, 0, c->stream>>>(s->part, nb, s->scal, cur);
             k_cg_start<<<nb3, 256, 0, c->stream>>>(a, s->scal, eps * rr0, it, s->r, s->p, s->p32);
@@ -2232,49 +2365,67 @@ static mpm_status imp_cg(mpm_ctx *c, double eps, int kmax, int *iters) {
 // One flexible GCR iteration on the scaled system: z = M(r) into direction
 // slot `sl`, q = A z, orthogonalised against the `u` previous images, then
 // x += alpha z, r -= alpha q with alpha = q.r / q.q.
-static mpm_status gcr_iter(mpm_ctx *c, const ImpArgs &a, int nb, int u, int sl) {
+// fed: the network's input already holds r; feed: leave the new r there.
+static mpm_status gcr_iter(mpm_ctx *c, const ImpArgs &a, int nb, int u, int sl, bool fed = false, bool feed = false) {
     ImpState *s = c->imp;
-    const size_t st3 = 3 * (size_t)c->g.nodec;
+    const size_t st = s->gst;
+    const int m = 3 * c->g.nodec, nq = (m + 1023) / 1024;
+    const bool pdl = !c->timer.on;
+    auto dots = [&](auto k, auto *Q, const float *Qf) {
+        launch(pdl, k, nq, 256, 0, c->stream, Q, Qf, st, m, sl, u, s->gm, s->part, s->cnt, (const double *)s->gqq,
+               s->gbeta);
+    };
+    auto axpy = [&](auto k, auto *P, auto *Q, float *Qf, int rr) {
+        launch(pdl, k, nq, 256, 0, c->stream, P, Q, Qf, st, m, sl, u, s->gm, (const double *)s->gbeta,
+               (const double *)s->r, s->gqq, s->part, s->cnt + 1, s->scal, rr);
+    };
     if (s->gp32 && mpm_nn_fp32_output(s->net)) {
         // FP32 operator: directions and images in FP32 (the FP32 matvec computes
         // them in FP32 anyway; x, r and the true residual stay FP64)
-        float *p = s->gp32 + (size_t)sl * st3, *q = s->gq32 + (size_t)sl * st3;
+        float *p = s->gp32 + (size_t)sl * st, *q = s->gq32 + (size_t)sl * st;
         timer_begin(c, K_PRECOND);
-        mpm_status st = mpm_nn_apply_precond_f32(s->net, c->stream, s->r, s->scal + S_RRC, s->adiag, a.bcflag, a.mtol,
-                                                 p);
+        mpm_status e = mpm_nn_apply_precond_f32(s->net, c->stream, s->r, s->scal + S_RRC, s->adiag, a.bcflag, a.mtol,
+                                                p, fed, pdl);
         timer_end(c, K_PRECOND);
-        if (st != MPM_OK) return st;
+        if (e != MPM_OK) return e;
         timer_begin(c, K_MATVEC);
         launch_matvec_f32(c, a, p, q);
         timer_end(c, K_MATVEC);
         timer_begin(c, K_KRYLOV);
-        if (u > 0)
-            k_gcr_dots<float><<<nb, 256, 0, c->stream>>>(a, s->gq32, s->gq32, sl, u, s->gm, s->part, s->cnt, s->gqq,
-                                                         s->gbeta);
-        k_gcr_axpy<float><<<nb, 256, 0, c->stream>>>(a, s->gp32, s->gq32, nullptr, sl, u, s->gm, s->gbeta, s->r,
-                                                     s->part, s->cnt + 1, s->scal);
-        k_gcr_update<float><<<nb, 256, 0, c->stream>>>(a, s->scal, s->xs, s->r, s->gp32, s->gq32, sl, s->gqq,
-                                                       s->part, s->cnt + 2);
+        const float *Q = s->gq32;
+        if (s->gm <= 4) {
+            if (u > 0) dots(k_gcr_dots<float, 4>, Q, Q);
+            axpy(k_gcr_axpy<float, 4>, s->gp32, s->gq32, nullptr, 1);
+        } else {
+            if (u > 0) dots(k_gcr_dots<float, GM>, Q, Q);
+            axpy(k_gcr_axpy<float, GM>, s->gp32, s->gq32, nullptr, 1);
+        }
+        launch(pdl, k_gcr_update_feed, nb, 256, 0, c->stream, (const double *)s->scal, s->xs, s->r,
+               (const float *)s->gp32, (const float *)s->gq32, st, c->g.nodec, sl, feed ? 1 : 0,
+               mpm_nn_input(s->net));
         timer_end(c, K_KRYLOV);
-        c->launches += 9 + 3 + (u > 0 ? 1 : 0);
+        c->launches += 7 + (fed ? 0 : 1) + 3 + (u > 0 ? 1 : 0);
         return MPM_OK;
     }
     timer_begin(c, K_PRECOND);
-    mpm_status st = mpm_nn_apply_precond(s->net, c->stream, s->r, s->scal + S_RRC, s->adiag, a.bcflag, a.mtol,
-                                         s->gp + (size_t)sl * st3);
+    mpm_status e = mpm_nn_apply_precond(s->net, c->stream, s->r, s->scal + S_RRC, s->adiag, a.bcflag, a.mtol,
+                                        s->gp + (size_t)sl * st);
     timer_end(c, K_PRECOND);
-    if (st != MPM_OK) return st;
+    if (e != MPM_OK) return e;
     timer_begin(c, K_MATVEC);
-    launch_matvec(c, a, nb, s->gp + (size_t)sl * st3, s->gq + (size_t)sl * st3, nullptr);
+    launch_matvec(c, a, nb, s->gp + (size_t)sl * st, s->gq + (size_t)sl * st);
     timer_end(c, K_MATVEC);
     timer_begin(c, K_KRYLOV);
-    if (u > 0)
-        k_gcr_dots<double><<<nb, 256, 0, c->stream>>>(a, s->gq, s->gqf, sl, u, s->gm, s->part, s->cnt, s->gqq,
-                                                      s->gbeta);
-    k_gcr_axpy<double><<<nb, 256, 0, c->stream>>>(a, s->gp, s->gq, s->gqf, sl, u, s->gm, s->gbeta, s->r, s->part,
-                                                  s->cnt + 1, s->scal);
-    k_gcr_update<double><<<nb, 256, 0, c->stream>>>(a, s->scal, s->xs, s->r, s->gp, s->gq, sl, s->gqq, s->part,
-                                                    s->cnt + 2);
+    const double *Q = s->gq;
+    if (s->gm <= 4) {
+        if (u > 0) dots(k_gcr_dots<double, 4>, Q, s->gqf);
+        axpy(k_gcr_axpy<double, 4>, s->gp, s->gq, s->gqf, 0);
+    } else {
+        if (u > 0) dots(k_gcr_dots<double, GM>, Q, s->gqf);
+        axpy(k_gcr_axpy<double, GM>, s->gp, s->gq, s->gqf, 0);
+    }
+    launch(pdl, k_gcr_update<double>, nq, 256, 0, c->stream, s->scal, s->xs, s->r, (const double *)s->gp,
+           (const double *)s->gq, st, m, sl, s->part, s->cnt + 2);
     timer_end(c, K_KRYLOV);
     c->launches += 9 + 3 + (u > 0 ? 1 : 0);
     return MPM_OK;
@@ -2293,7 +2444,7 @@ static mpm_status imp_fcg(mpm_ctx *c, double eps, int kmax, int *iters) {
     const size_t N = (size_t)c->g.nodec;
     k_cg_scale_in<<<nb, 256, 0, c->stream>>>(a, s->x, s->b, s->adiag, s->xs, s->r);
     CKI(cudaMemcpyAsync(s->bs, s->r, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, c->stream));
-    launch_matvec(c, a, nb, s->xs, s->Ap, nullptr, nullptr, nullptr, 0, true);
+    launch_matvec(c, a, nb, s->xs, s->Ap, nullptr, true);
     k_true_residual<<<nb, 256, 0, c->stream>>>(a, s->bs, s->Ap, s->r, s->part);
     k_finish<<<1, 256, 0, c->stream>>>(s->part, nb, s->scal, S_RR0);
     k_finish<<<1, 256, 0, c->stream>>>(s->part, nb, s->scal, S_RRC);
@@ -2361,23 +2512,27 @@ static mpm_status imp_fcg(mpm_ctx *c, double eps, int kmax, int *iters) {
         int used = 0, slot = 0;
         double rr_win = rr0;
         bool fine = false;   // close to the tolerance: one iteration at a time, checked after each
-        auto gcr_iteration = [&](int u, int sl) -> mpm_status { return gcr_iter(c, a, nb, u, sl); };
+        bool fed = false;    // the network's input holds the current residual
         while (!done && use_nn && it < kmax) {
             if (graphs_on(c) && !fine && used == s->gm && slot == 0 && it % check == 0 && it + check <= kmax) {
                 const int64_t l0 = c->launches;
                 if (!s->g_gcr && capture_iters(c, &s->g_gcr, [&] {
-                        for (int k = 0; k < check; k++) gcr_iteration(s->gm, k % s->gm);
+                        for (int k = 0; k < check; k++)
+                            gcr_iter(c, a, nb, s->gm, k % s->gm, k > 0, k + 1 < check);
+                        s->gcr_launches = c->launches - l0;
                     }) != MPM_OK)
                     s->no_graph = true;
                 if (!s->g_gcr) continue;
                 s->g_net = s->net;
                 CKI(cudaGraphLaunch(s->g_gcr, c->stream));
-                if (c->launches == l0) c->launches += 18 * check;
+                if (c->launches == l0) c->launches += s->gcr_launches;
+                fed = false;
                 s->nn_applications += check;
                 it += check;
             } else {
-                mpm_status st = gcr_iteration(used, slot);
+                mpm_status st = gcr_iter(c, a, nb, used, slot, fed, true);
                 if (st != MPM_OK) return st;
+                fed = s->gp32 && mpm_nn_fp32_output(s->net);
                 s->nn_applications++;
                 used = used < s->gm ? used + 1 : s->gm;
                 slot = (slot + 1) % s->gm;
@@ -2394,12 +2549,13 @@ static mpm_status imp_fcg(mpm_ctx *c, double eps, int kmax, int *iters) {
                     CKI(cudaStreamSynchronize(c->stream));
                     if (s->h_scal[S_RRC] >= 1.1 * eps * rr0) continue;
                 }
+                fed = false;
                 if (form) {
                     // FP32 operator: the recursive residual drifts from the true one
                     // by the rounding of the FP32 matvecs, so at every check it is
                     // replaced by the true residual bs - A x (FP64 arithmetic); the
                     // kept directions and their images stay valid
-                    launch_matvec(c, a, nb, s->xs, s->z, nullptr, nullptr, nullptr, 0, true);
+                    launch_matvec(c, a, nb, s->xs, s->z, nullptr, true);
                     k_true_residual<<<nb, 256, 0, c->stream>>>(a, s->bs, s->z, s->r, s->part);
                     k_finish<<<1, 256, 0, c->stream>>>(s->part, nb, s->scal, S_RRC);
                     c->launches += 3;
@@ -2415,7 +2571,7 @@ static mpm_status imp_fcg(mpm_ctx *c, double eps, int kmax, int *iters) {
                 if (rr < eps * rr0 && s->prec == 32) {
                     done = true;   // rr is the true residual
                 } else if (rr < eps * rr0) {
-                    launch_matvec(c, a, nb, s->xs, s->z, nullptr, nullptr, nullptr, 0, true);
+                    launch_matvec(c, a, nb, s->xs, s->z, nullptr, true);
                     k_true_residual<<<nb, 256, 0, c->stream>>>(a, s->bs, s->z, s->r, s->part);
                     k_finish<<<1, 256, 0, c->stream>>>(s->part, nb, s->scal, S_RRC);
                     c->launches += 3;
@@ -2490,7 +2646,7 @@ static mpm_status imp_fcg(mpm_ctx *c, double eps, int kmax, int *iters) {
                         use_nn ? "network" : "jacobi");
             if (rr < eps * rr0) {
                 // confirm on the true residual
-                launch_matvec(c, a, nb, s->xs, s->z, nullptr, nullptr, nullptr, 0, true);
+                launch_matvec(c, a, nb, s->xs, s->z, nullptr, true);
                 k_true_residual<<<nb, 256, 0, c->stream>>>(a, s->bs, s->z, s->r, s->part);
                 k_finish<<<1, 256, 0, c->stream>>>(s->part, nb, s->scal, S_RRC);
                 c->launches += 3;
@@ -2544,7 +2700,7 @@ static mpm_status imp_residuals(mpm_ctx *c, double *ref, double *absr) {
     ImpArgs a = imp_args(c);
     const int nb = nb_nodes(c);
     k_imp_prepare_residual<<<nb, 256, 0, c->stream>>>(a, s->x, s->adiag, s->b, s->xs);
-    launch_matvec(c, a, nb, s->xs, s->Ap, nullptr, nullptr, nullptr, 0, true);
+    launch_matvec(c, a, nb, s->xs, s->Ap, nullptr, true);
     k_imp_residual<<<nb, 256, 0, c->stream>>>(a, s->Ap, s->adiag, s->b, s->part);
     k_finish<<<1, 256, 0, c->stream>>>(s->part, nb, s->scal, S_RES);
     k_finish<<<1, 256, 0, c->stream>>>(s->part + nb, nb, s->scal, S_IDOF);
@@ -2707,7 +2863,7 @@ mpm_status mpm_gpu_implicit_matvec(mpm_ctx *c, const double *x, double *y) {
     CKI(cudaMemcpyAsync(s->xs, x, sizeof(double) * 3 * N, cudaMemcpyHostToDevice, c->stream));
     ImpArgs a = imp_args(c);
     timer_begin(c, K_MATVEC);
-    launch_matvec(c, a, nb_nodes(c), s->xs, s->Ap, nullptr, nullptr, nullptr, 0, true);
+    launch_matvec(c, a, nb_nodes(c), s->xs, s->Ap, nullptr, true);
     timer_end(c, K_MATVEC);
     c->launches++;
     CKI(cudaMemcpyAsync(y, s->Ap, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, c->stream));
@@ -2793,6 +2949,9 @@ static mpm_status gcr_record(mpm_ctx *c, mpm_nn *rec, int npairs) {
         if (st != MPM_OK) return st;
         st = gcr_iter(c, a, nb, used, slot);
         if (st != MPM_OK) return st;
+        // the pairs are scaled by the residual's own norm
+        k_dot3<<<nb, 256, 0, c->stream>>>(a, s->r, s->r, s->part);
+        k_finish<<<1, 256, 0, c->stream>>>(s->part, nb, s->scal, S_RRC);
         used = used < s->gm ? used + 1 : s->gm;
         slot = (slot + 1) % s->gm;
     }

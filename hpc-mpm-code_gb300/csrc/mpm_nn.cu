@@ -27,6 +27,7 @@
 
 #include <cuda.h>
 
+#include "mpm_device.cuh"
 #include "mpm_nn.cuh"
 #include "mpm_tc.cuh"
 
@@ -115,13 +116,6 @@ __device__ __forceinline__ void unpack8(const uint4 &u, float *f) {
     }
 }
 
-__device__ __forceinline__ uint4 pack8(const float *f) {
-    uint4 u;
-    __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&u);
-#pragma unroll
-    for (int i = 0; i < 4; i++) h[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-    return u;
-}
 
 // ------------------------------------------------------------------ conv
 struct ConvArgs {
@@ -411,6 +405,13 @@ __global__ void __launch_bounds__(128) k_conv_halo(ConvArgs a, const __grid_cons
             bulk_g2s(smem + NBUF * HB + o, reinterpret_cast<const unsigned char *>(a.w) + o, WB - o < WCH ? WB - o : WCH,
                      &wbar);
     }
+    // Launched while its predecessor drains: the tensor memory, barriers and weights
+    // above depend on nothing the predecessor writes (forward does not launch the
+    // first convolution early after new weights).  The trigger lies behind the
+    // allocation, so a successor's blocks never take tensor memory that a block of
+    // this grid still has to get.
+    pdl_wait();
+    pdl_trigger();
     const uint32_t taddr = tslot;
     const int ntx = (a.lout.n[0] + H::TX - 1) / H::TX, nty = (a.lout.n[1] + H::TY - 1) / H::TY;
     const int64_t per_b = (int64_t)ntx * nty * a.lout.n[2];
@@ -729,7 +730,7 @@ __device__ __forceinline__ double block_rms(const double *rr, int64_t nodec, boo
     __shared__ double s_rms;
     if (threadIdx.x == 0) {
         const double ms = rr[0] / (3.0 * (double)nodec);
-        s_rms = ms > 0.0 ? (inverse ? 1.0 / sqrt(ms) : sqrt(ms)) : 0.0;
+        s_rms = inverse ? inv_rms(rr[0], nodec) : ms > 0.0 ? sqrt(ms) : 0.0;
     }
     __syncthreads();
     return s_rms;
@@ -737,23 +738,20 @@ __device__ __forceinline__ double block_rms(const double *rr, int64_t nodec, boo
 
 // x0 from an FP64 component-major residual, scaled by 1 / sqrt(rr / (3 nodec)),
 // and the system's feature channels
-__global__ void k_input_r(const double *r, const double *rr, const bf16 *feat, int64_t nodec, int linear, bf16 *x0) {
+__global__ void k_input_r(const double *r, const double *rr, int64_t nodec, Input in) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const double inv = block_rms(rr, nodec, true);
     if (n >= nodec) return;
-    float f[8] = {(float)(r[n] * inv), (float)(r[nodec + n] * inv), (float)(r[2 * nodec + n] * inv),
-                  __bfloat162float(feat[3 * n]), __bfloat162float(feat[3 * n + 1]), __bfloat162float(feat[3 * n + 2]),
-                  0, 0};
-    if (linear)
-        for (int c = 0; c < 3; c++) f[3 + c] *= f[c];   // r * phi keeps the map linear in r
-    uint4 *o = reinterpret_cast<uint4 *>(x0 + n * 16);
-    o[0] = pack8(f);
-    o[1] = make_uint4(0, 0, 0, 0);
+    store_input(in, n, (float)(r[n] * inv), (float)(r[nodec + n] * inv), (float)(r[2 * nodec + n] * inv));
 }
 
 // out = relu(up(coarse) + skip), C channels, one thread per (fine row, 8 channels)
 template <int C>
 __global__ void k_up_add_relu(const bf16 *coarse, const bf16 *skip, bf16 *out, Lvl lf, Lvl lc, int64_t rows, int act) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t item = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (item >= rows * (C / 8)) return;
     const int64_t row = item / (C / 8);
@@ -864,6 +862,7 @@ template <typename TZ>
 __global__ void k_output_up(const bf16 *c1, const bf16 *e0, const float *w5, const double *rr, Lvl lf, Lvl lc,
                             const double *adiag, const unsigned char *bcflag, double mtol, const double *r, TZ *z) {
     __shared__ float sw5[48];
+    pdl_wait();
     const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (threadIdx.x < 48) sw5[threadIdx.x] = w5[threadIdx.x];
     const double s = block_rms(rr, lf.v, false);
@@ -1232,7 +1231,7 @@ bool make_halo_maps(const bf16 *in, const Lvl &L, int batch, HaloMaps &m) {
 }
 
 template <int K, int N, int MODE>
-cudaError_t launch_conv_halo(mpm_nn *net, cudaStream_t st, const ConvArgs &a) {
+cudaError_t launch_conv_halo(mpm_nn *net, cudaStream_t st, const ConvArgs &a, bool pdl) {
     constexpr size_t smem = halo_smem<K, N, MODE>();
     static_assert(smem <= 227u * 1024, "shared memory");
     HaloMaps maps;
@@ -1250,13 +1249,14 @@ cudaError_t launch_conv_halo(mpm_nn *net, cudaStream_t st, const ConvArgs &a) {
     const int per_sm = std::max<int>(1, std::min<int>(4, (int)(225000 / (smem + 1024))));
     const int grid = (int)std::min<int64_t>(ntile, (int64_t)net->nsm * per_sm);
     if (grid <= 0) return cudaSuccess;
-    k_conv_halo<K, N, MODE><<<grid, 128, smem, st>>>(a, maps);
+    launch(pdl, k_conv_halo<K, N, MODE>, grid, 128, smem, st, a, maps);
     return cudaGetLastError();
 }
 
 template <int K, int N, int MODE>
 cudaError_t launch_conv(mpm_nn *net, cudaStream_t st, const bf16 *in, bf16 *out, const bf16 *w, const float *bias,
-                        const bf16 *add, const bf16 *mask, int relu, const Lvl &lin, const Lvl &lout, int batch) {
+                        const bf16 *add, const bf16 *mask, int relu, const Lvl &lin, const Lvl &lout, int batch,
+                        bool pdl = false) {
     constexpr size_t smem = conv_smem<K, N>();
     static bool attr_set = false;
     if (!attr_set) {
@@ -1278,7 +1278,7 @@ cudaError_t launch_conv(mpm_nn *net, cudaStream_t st, const bf16 *in, bf16 *out,
     a.rows = (int64_t)batch * lout.v;
     a.err = net->err;
     if constexpr (MODE == S1 || MODE == S2) {
-        if (net->halo) return launch_conv_halo<K, N, MODE>(net, st, a);
+        if (net->halo) return launch_conv_halo<K, N, MODE>(net, st, a, pdl);
     }
     const int64_t ntile = (a.rows + 127) / 128;
     const int per_sm = std::max<int>(1, std::min<int>(4, (int)(220000 / smem)));
@@ -1336,7 +1336,8 @@ cudaError_t prep_weights(mpm_nn *net, cudaStream_t st) {
 }
 
 // forward of `batch` samples whose x0 is already in place
-cudaError_t forward(mpm_nn *net, cudaStream_t st, int batch, bool make_d0 = true) {
+cudaError_t forward(mpm_nn *net, cudaStream_t st, int batch, bool make_d0 = true, bool pdl = false) {
+    const bool fresh = net->weights_dirty;
     cudaError_t e = prep_weights(net, st);
     if (e != cudaSuccess) return e;
     const Lvl &L0 = net->L[0], &L1 = net->L[1], &L2 = net->L[2];
@@ -1344,21 +1345,22 @@ cudaError_t forward(mpm_nn *net, cudaStream_t st, int batch, bool make_d0 = true
     const int act = net->linear ? 0 : 1;
     auto bias = [&](int l) -> const float * { return net->linear ? nullptr : P + b_offset(l); };
     if ((e = launch_conv<16, 16, S1>(net, st, net->x0, net->e0, net->wf[0], bias(0), nullptr, nullptr, act, L0, L0,
-                                     batch)) != cudaSuccess)
+                                     batch, pdl && !fresh)) != cudaSuccess)
         return e;
     if ((e = launch_conv<16, 32, S2>(net, st, net->e0, net->e1, net->wf[1], bias(1), nullptr, nullptr, act, L0, L1,
-                                     batch)) != cudaSuccess)
+                                     batch, pdl)) != cudaSuccess)
         return e;
     if ((e = launch_conv<32, 64, S2>(net, st, net->e1, net->e2, net->wf[2], bias(2), nullptr, nullptr, act, L1, L2,
-                                     batch)) != cudaSuccess)
+                                     batch, pdl)) != cudaSuccess)
         return e;
     if ((e = launch_conv<64, 32, S1>(net, st, net->e2, net->c2, net->wf[3], bias(3), nullptr, nullptr, 0, L2, L2,
-                                     batch)) != cudaSuccess)
+                                     batch, pdl)) != cudaSuccess)
         return e;
     const int64_t r1 = (int64_t)batch * L1.v, r0 = (int64_t)batch * L0.v;
-    k_up_add_relu<32><<<blocks(r1 * 4), 256, 0, st>>>(net->c2, net->e1, net->d1, L1, L2, r1, act);
+    launch(pdl, k_up_add_relu<32>, blocks(r1 * 4), 256, 0, st, (const bf16 *)net->c2, (const bf16 *)net->e1, net->d1, L1,
+           L2, r1, act);
     if ((e = launch_conv<32, 16, S1>(net, st, net->d1, net->c1, net->wf[4], bias(4), nullptr, nullptr, 0, L1, L1,
-                                     batch)) != cudaSuccess)
+                                     batch, pdl)) != cudaSuccess)
         return e;
     if (make_d0) k_up_add_relu<16><<<blocks(r0 * 2), 256, 0, st>>>(net->c1, net->e0, net->d0, L0, L1, r0, act);
     return cudaGetLastError();
@@ -1722,10 +1724,12 @@ int mpm_nn_grid_matches(const mpm_nn *net, const int nodes[3]) {
     return net && net->L[0].n[0] == nodes[0] && net->L[0].n[1] == nodes[1] && net->L[0].n[2] == nodes[2];
 }
 
+nn::Input mpm_nn_input(const mpm_nn *net) { return {net->x0, net->feat, net->linear}; }
+
 mpm_status mpm_nn_apply_precond(mpm_nn *net, cudaStream_t st, const double *r, const double *rr, const double *adiag,
                                 const unsigned char *bcflag, double mtol, double *z) {
     const int64_t nodec = net->L[0].v;
-    k_input_r<<<blocks(nodec), 256, 0, st>>>(r, rr, net->feat, nodec, net->linear, net->x0);
+    k_input_r<<<blocks(nodec), 256, 0, st>>>(r, rr, nodec, mpm_nn_input(net));
     if (net->linear && !net->symmetric) {
         CKN(forward(net, st, 1, false));
         k_output_up<double><<<blocks(nodec), 256, 0, st>>>(net->c1, net->e0, net->p + w5_offset(), rr, net->L[0],
@@ -1753,13 +1757,15 @@ mpm_status mpm_nn_apply_precond(mpm_nn *net, cudaStream_t st, const double *r, c
 int mpm_nn_fp32_output(const mpm_nn *net) { return net && net->linear && !net->symmetric; }
 
 mpm_status mpm_nn_apply_precond_f32(mpm_nn *net, cudaStream_t st, const double *r, const double *rr,
-                                    const double *adiag, const unsigned char *bcflag, double mtol, float *z) {
+                                    const double *adiag, const unsigned char *bcflag, double mtol, float *z, bool fed,
+                                    bool pdl) {
     if (!mpm_nn_fp32_output(net)) return MPM_ERR_UNSUPPORTED;
     const int64_t nodec = net->L[0].v;
-    k_input_r<<<blocks(nodec), 256, 0, st>>>(r, rr, net->feat, nodec, net->linear, net->x0);
-    CKN(forward(net, st, 1, false));
-    k_output_up<float><<<blocks(nodec), 256, 0, st>>>(net->c1, net->e0, net->p + w5_offset(), rr, net->L[0],
-                                                      net->L[1], adiag, bcflag, mtol, net->additive ? r : nullptr, z);
+    if (!fed) launch(pdl, k_input_r, blocks(nodec), 256, 0, st, r, rr, nodec, mpm_nn_input(net));
+    CKN(forward(net, st, 1, false, pdl));
+    launch(pdl, k_output_up<float>, blocks(nodec), 256, 0, st, (const bf16 *)net->c1, (const bf16 *)net->e0,
+           (const float *)(net->p + w5_offset()), rr, net->L[0], net->L[1], adiag, bcflag, mtol,
+           net->additive ? r : (const double *)nullptr, z);
     CKN(cudaGetLastError());
     return MPM_OK;
 }

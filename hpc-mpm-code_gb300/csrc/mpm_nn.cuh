@@ -46,6 +46,37 @@ int64_t b_offset(int l);
 int64_t w5_offset();
 int64_t b5_offset();
 
+__device__ __forceinline__ uint4 pack8(const float *f) {
+    uint4 u;
+    __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&u);
+#pragma unroll
+    for (int i = 0; i < 4; i++) h[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+    return u;
+}
+
+// The network's input of one system: x0 and the feature channels.
+struct Input {
+    __nv_bfloat16 *x0;
+    const __nv_bfloat16 *feat;
+    int linear;
+};
+
+__device__ __forceinline__ double inv_rms(double rr, int64_t nodec) {
+    const double ms = rr / (3.0 * (double)nodec);
+    return ms > 0.0 ? 1.0 / sqrt(ms) : 0.0;
+}
+
+// the input row of node n from its scaled residual
+__device__ __forceinline__ void store_input(const Input &in, int64_t n, float r0, float r1, float r2) {
+    float f[8] = {r0, r1, r2, __bfloat162float(in.feat[3 * n]), __bfloat162float(in.feat[3 * n + 1]),
+                  __bfloat162float(in.feat[3 * n + 2]), 0, 0};
+    if (in.linear)
+        for (int c = 0; c < 3; c++) f[3 + c] *= f[c];   // r * phi keeps the map linear in r
+    uint4 *o = reinterpret_cast<uint4 *>(in.x0 + n * 16);
+    o[0] = pack8(f);
+    o[1] = make_uint4(0, 0, 0, 0);
+}
+
 }  // namespace nn
 }  // namespace mpm
 
@@ -57,8 +88,12 @@ mpm_status mpm_nn_apply_precond(mpm_nn *net, cudaStream_t st, const double *r, c
                                 const unsigned char *bcflag, double mtol, double *z);
 // The same with z in FP32, for the network's default mode (linear, not
 // symmetrised: true from mpm_nn_fp32_output); MPM_ERR_UNSUPPORTED otherwise.
+// fed: the input row of every node was already stored (store_input on
+// mpm_nn_input); pdl: launched while the stream's predecessors drain.
 mpm_status mpm_nn_apply_precond_f32(mpm_nn *net, cudaStream_t st, const double *r, const double *rr,
-                                    const double *adiag, const unsigned char *bcflag, double mtol, float *z);
+                                    const double *adiag, const unsigned char *bcflag, double mtol, float *z,
+                                    bool fed = false, bool pdl = false);
+mpm::nn::Input mpm_nn_input(const mpm_nn *net);
 int mpm_nn_fp32_output(const mpm_nn *net);
 // Feature channels of the system about to be solved (phi, FP64 component-major).
 mpm_status mpm_nn_set_feature(mpm_nn *net, cudaStream_t st, const double *phi);
