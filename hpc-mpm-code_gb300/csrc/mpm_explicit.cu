@@ -1053,22 +1053,27 @@ __device__ __forceinline__ float trilinear_eval(const float *c, float u, float v
     return fmaf(c[7], uvw, r);
 }
 
-// the inputs of one particle of the moment-form gather (v: FLIP only)
+// the inputs of one particle of the moment-form gather
 struct MuslIn {
-    float x[3], m, vol, v[3];
+    float x[3], m, vol;
 };
-__device__ __forceinline__ void musl_fetch(const Particles<float> &P, int p, bool flip, MuslIn &o) {
+__device__ __forceinline__ void musl_fetch(const Particles<float> &P, int p, MuslIn &o) {
     o.x[0] = ld(P.x[0] + p);
     o.x[1] = ld(P.x[1] + p);
     o.x[2] = ld(P.x[2] + p);
     o.m = ld(P.m + p);
     o.vol = ld(P.vol + p);
-    o.v[0] = flip ? ld(P.v[0] + p) : 0.0f;
-    o.v[1] = flip ? ld(P.v[1] + p) : 0.0f;
-    o.v[2] = flip ? ld(P.v[2] + p) : 0.0f;
 }
 
-template <int MINB, bool LIST>
+// FLIP adds to the particle's own velocity, which the same pass overwrites.  A load
+// of a sector that this SM has just stored to waits for the store, and the cells'
+// lanes came to every sector eight times: 34 us against 10.6 for PIC at 243,675
+// particles (27 per cell).  So the old velocities of up to VCH of the brick's
+// particles are brought into shared memory first, coalesced: 34 -> 11.5 us (577,600
+// particles, 64 per cell: 117 -> 39; 72,200, 8 per cell: 10.8 -> 11.1).
+constexpr int VCH = 4096;   // 48 KB: a full brick of 32 particles per cell
+
+template <int MINB, bool LIST, bool FLIP>
 __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_mom(StepArgs<float> a) {
     pdl_wait();
     __shared__ float corner[3 * 8][BRC];
@@ -1080,7 +1085,7 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_mom(StepArgs<fl
     int qi = 0;
     load_scales_musl(a, S);
     const int nbl = LIST ? *a.nblist : 1;
-    const bool flip = (a.scheme == MPM_FLIP);
+    extern __shared__ float vold[];   // FLIP: [3][VCH]
     const unsigned pair = 3u << ((threadIdx.x & 31) & ~1u);
     long long gacc = 0;   // over all of this CTA's bricks
     float vmax = 0.0f;
@@ -1096,7 +1101,7 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_mom(StepArgs<fl
         const Particles<float> &P = a.P;
         // the first particle's loads are in flight with the cell's nodal values
         MuslIn nx;
-        if (p0 + h < p1) musl_fetch(P, p0 + h, flip, nx);
+        if (p0 + h < p1) musl_fetch(P, p0 + h, nx);
         float Gc[3][8], Ec[8];
         {
             MuslCell C;
@@ -1105,7 +1110,7 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_mom(StepArgs<fl
             for (int d = 0; d < 3; d++) trilinear_coeffs(C.G[d], h, pair, Gc[d]);
             trilinear_coeffs(C.E, h, pair, Ec);
         }
-        if (flip) {
+        if (FLIP) {
             // FLIP gathers the nodal acceleration: v += dt sum N a
 #pragma unroll
             for (int d = 0; d < 3; d++)
@@ -1122,11 +1127,23 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_mom(StepArgs<fl
         for (int d = 0; d < 3; d++)
 #pragma unroll
             for (int k = 0; k < 8; k++) M[d][k] = 0.0f;
-        for (int p = p0 + h; p < p1; p += 2) {
+        int p = p0 + h;
+        for (int c0 = cs[0], P1 = cs[BRC]; c0 < P1; c0 += VCH) {
+        const int q1 = FLIP ? min(p1, c0 + VCH) : p1;
+        if (FLIP) {
+            if (c0 != cs[0]) __syncthreads();   // every lane is done with the chunk before
+            const int nv = min(VCH, P1 - c0);
+#pragma unroll 4
+            for (int i = threadIdx.x; i < nv; i += CELL_THREADS)
+#pragma unroll
+                for (int d = 0; d < 3; d++) vold[d * VCH + i] = P.v[d][c0 + i];
+            __syncthreads();
+        }
+        for (; p < q1; p += 2) {
             // this particle's inputs, and the next one's loads issued before the work on this one
             const float x0 = nx.x[0], x1 = nx.x[1], x2 = nx.x[2], m = nx.m, vol = nx.vol;
-            float vel[3] = {nx.v[0], nx.v[1], nx.v[2]};
-            if (p + 2 < p1) musl_fetch(P, p + 2, flip, nx);
+            float vel[3];
+            if (p + 2 < p1) musl_fetch(P, p + 2, nx);
             const float u = cell_offset_u(x0, a.g, 0, cx), v = cell_offset_u(x1, a.g, 1, cy),
                         w = cell_offset_u(x2, a.g, 2, cz);
             if (!in_cell(u, v, w)) {
@@ -1138,7 +1155,7 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_mom(StepArgs<fl
 #pragma unroll
             for (int d = 0; d < 3; d++) {
                 const float g = trilinear_eval(Gc[d], u, v, w, uv, uw, vw, uvw);
-                vel[d] = flip ? vel[d] + g : g;
+                vel[d] = FLIP ? vold[d * VCH + p - c0] + g : g;
             }
             P.v[0][p] = vel[0];
             P.v[1][p] = vel[1];
@@ -1155,6 +1172,8 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_mom(StepArgs<fl
 #pragma unroll
                 for (int k = 0; k < 8; k++) M[d][k] = fmaf(q, mono[k], M[d][k]);
             }
+        }
+        if (!FLIP) break;   // no chunks
         }
         float acc[3][4];
 #pragma unroll
@@ -3295,10 +3314,15 @@ static mpm_status launch_particle_kernel(mpm_ctx *c, int which) {
         timer_begin(c, K_G2P_MUSL);
         if constexpr (sizeof(R) == 4 && OX == 1 && OY == 1 && OZ == 1) {
             if (use_cell_kernels(c)) {
-                if (c->tune.musl_moments == 2) {
-                    launch(c->pdl != 0, k_g2p_musl_mom<2, true>, list_grid(c, 2), CELL_THREADS, 0, c->stream, a);
-                } else if (c->tune.musl_moments) {
-                    k_g2p_musl_mom<3, true><<<list_grid(c, 3), CELL_THREADS, 0, c->stream>>>(a);
+                if (c->tune.musl_moments) {
+                    const int ctas = c->tune.musl_moments == 2 ? 2 : 3;
+                    auto go = [&](auto k, size_t smem) {
+                        if (smem) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                        launch(c->pdl != 0, k, list_grid(c, ctas), CELL_THREADS, smem, c->stream, a);
+                    };
+                    constexpr size_t V = sizeof(float) * 3 * VCH;
+                    if (ctas == 2) c->scheme == MPM_FLIP ? go(k_g2p_musl_mom<2, true, true>, V) : go(k_g2p_musl_mom<2, true, false>, 0);
+                    else c->scheme == MPM_FLIP ? go(k_g2p_musl_mom<3, true, true>, V) : go(k_g2p_musl_mom<3, true, false>, 0);
                 } else if (c->tune.musl_staged == 2) {
                     k_musl_brick<<<c->g.nbricks, BCH, 0, c->stream>>>(a);
                 } else if (c->tune.musl_staged) {
