@@ -269,7 +269,8 @@ __global__ void __launch_bounds__(CellShape<R, OX, OY, OZ>::THREADS, CellShape<R
     using Sum = typename C::Sum;
     Sum *corner = reinterpret_cast<Sum *>(cell_smem);   // [FR][NE][CELLS]
     __shared__ Scales S;
-    if (MUSL) load_scales_musl(a, S);
+    if (KIND == CELL_MUSL_AFF) affine_scales(a, S);
+    else if (MUSL) load_scales_musl(a, S);
     else p2g_scales(a, S);   // read after the first barrier of a slab
     const int lc = threadIdx.x / P, part = threadIdx.x % P;
     const int kk = part % C::NZ, j0 = (part / C::NZ) * JP;
@@ -546,7 +547,7 @@ __global__ void __launch_bounds__(256) k_gather(StepArgs<R> a) {
     __shared__ Scales S;
     __shared__ long long sh_l[32];
     __shared__ float sh_f[32];
-    load_scales_musl(a, S);
+    musl_scales(a, S);
     const size_t N = (size_t)a.g.nodec, sy = (size_t)a.g.nnc[0], sz = sy * (size_t)a.g.nnc[1];
     const Particles<R> &P = a.P;
     const bool flip = a.scheme == MPM_FLIP, shift = a.shifting != 0;

@@ -175,6 +175,24 @@ __device__ __forceinline__ long long fx(double c, const Fix &f) { return __doubl
 __device__ __forceinline__ float unfx(long long q, const Fix &f, float) { return (__ll2float_rn(q) * f.i1) * f.i2; }
 __device__ __forceinline__ double unfx(long long q, const Fix &f, double) { return (double)q * f.inv; }
 
+// __ll2float_rn for |q| < 2^63 without the 64-bit conversion, which takes a slot of
+// the FP64 pipe (a warp's conversion holds it for 64 cycles; these 20 instructions
+// are issued in 25).  |q| = A 2^k + B with A, B below 2^24, so one FMA rounds it:
+// k = 17 when |q| < 2^41; above, B's last bit (2^16, at most a quarter of the
+// result's last place) stands for every bit below it.
+__device__ __forceinline__ float ll2f(long long q) {
+    const unsigned long long m = q < 0 ? 0ull - (unsigned long long)q : (unsigned long long)q;
+    const unsigned h = (unsigned)(m >> 32), l = (unsigned)m;
+    const bool big = h >= 512u;
+    const unsigned a = big ? h & ~0x7Fu : (unsigned)(m >> 17);
+    const unsigned b = big ? ((h & 0x7Fu) << 16) | (l >> 16) | ((l & 0xFFFFu) != 0u ? 1u : 0u) : l & 0x1FFFFu;
+    const float fb = __uint_as_float(0x4B000000u | b) - 8388608.0f;   // b < 2^23
+    const float r = fmaf((float)a, big ? 4294967296.0f : 131072.0f, big ? fb * 65536.0f : fb);
+    return q < 0 ? -r : r;
+}
+__device__ __forceinline__ float unfx_int(long long q, const Fix &f, float) { return (ll2f(q) * f.i1) * f.i2; }
+__device__ __forceinline__ double unfx_int(long long q, const Fix &f, double) { return (double)q * f.inv; }
+
 __device__ __forceinline__ void atomic_add_i64(unsigned long long *p, long long v) {
     atomicAdd(p, (unsigned long long)v);
 }

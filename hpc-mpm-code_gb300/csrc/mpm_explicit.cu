@@ -230,6 +230,8 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_p2g_cell(StepArgs<float>
     __shared__ float corner[NACC * 8][BRC];       // 32 KB
     __shared__ Scales S;
     __shared__ int sh_red[32];
+    pdl_wait();
+    p2g_scales(a, S);   // before an empty brick leaves: CTA 0 starts the step
     const int b = blockIdx.x;
     const int lc = threadIdx.x >> 1, h = threadIdx.x & 1;
     const int *cs = a.cstart + (size_t)b * (BRC + 1);
@@ -238,7 +240,7 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_p2g_cell(StepArgs<float>
     brick_origin(b, a.nbrick, ox, oy, oz);
     const int cx = ox + (lc % BRX), cy = oy + (lc / BRX) % BRY, cz = oz + lc / (BRX * BRY);
     const int p0 = cs[lc], p1 = cs[lc + 1];
-    load_scales(a, S);
+    __syncthreads();
     const float fxg = a.grav[0] * a.facl, fyg = a.grav[1] * a.facl, fzg = a.grav[2] * a.facl;
     const Particles<float> &P = a.P;
     float acc[NACC][4];
@@ -903,7 +905,7 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_cell(StepArgs<f
     __shared__ Scales S;
     __shared__ long long sh_l[32];
     __shared__ float sh_f[32];
-    load_scales_musl(a, S);
+    musl_scales(a, S);
     const int nbl = LIST ? *a.nblist : 1;
     for (int li = LIST ? (int)blockIdx.x : 0; li < nbl; li += LIST ? (int)gridDim.x : 1) {
         const int b = LIST ? a.blist[a.rev_g2p ? nbl - 1 - li : li] : (int)blockIdx.x;
@@ -1083,7 +1085,7 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_mom(StepArgs<fl
     __shared__ int n_miss[2];   // the brick's queue length, alternating
     if (threadIdx.x == 0) n_miss[0] = 0;
     int qi = 0;
-    load_scales_musl(a, S);
+    musl_scales(a, S);
     const int nbl = LIST ? *a.nblist : 1;
     extern __shared__ float vold[];   // FLIP: [3][VCH]
     const unsigned pair = 3u << ((threadIdx.x & 31) & ~1u);
@@ -1229,7 +1231,7 @@ __global__ void __launch_bounds__(BCH) k_musl_brick(StepArgs<float> a) {
         box[2][l] = ld(a.G + 2 * N + gn);
         box[3][l] = ld(a.nei + gn);
     }
-    load_scales_musl(a, S);   // also publishes scs and box
+    musl_scales(a, S, true);   // also publishes scs and box
     const Particles<float> &P = a.P;
     const bool flip = (a.scheme == MPM_FLIP);
     const int lc = tid;
@@ -1427,7 +1429,7 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_g2p_musl_cell_staged(Ste
     brick_origin(b, a.nbrick, ox, oy, oz);
     const int cx = ox + (lc % BRX), cy = oy + (lc / BRX) % BRY, cz = oz + lc / (BRX * BRY);
     const int p0 = cs[lc], p1 = cs[lc + 1];
-    load_scales_musl(a, S);
+    musl_scales(a, S, true);
     MuslCell C;
     musl_load_cell(a, cx, cy, cz, h, p1 > p0, C);
     float acc[3][4];
@@ -1633,7 +1635,7 @@ __global__ void __launch_bounds__(256) k_g2p_musl_box(StepArgs<R> a) {
     int ox, oy, oz;
     brick_origin(w.tile, a.nbrick, ox, oy, oz);
     for (int i = threadIdx.x; i < 3 * BOX; i += blockDim.x) sacc[i] = 0ull;
-    load_scales_musl(a, S);
+    musl_scales(a, S, true);
     const size_t N = (size_t)a.g.nodec;
     const Particles<R> &P = a.P;
     const bool flip = (a.scheme == MPM_FLIP);
@@ -1773,10 +1775,11 @@ __device__ __forceinline__ void apic_axis(const KGeom<R> &g, int d, int c, R x, 
 
 template <typename R, int OX, int OY, int OZ>
 __global__ void __launch_bounds__(256) k_affine_gather(StepArgs<R> a) {
+    pdl_wait();
     __shared__ Scales S;
     __shared__ long long sh_l[32];
     __shared__ float sh_f[32];
-    load_scales_musl(a, S);
+    musl_scales(a, S);
     const size_t N = (size_t)a.g.nodec;
     const Particles<R> &P = a.P;
     const bool apic = (a.scheme == MPM_APIC);
@@ -1895,6 +1898,8 @@ __global__ void __launch_bounds__(256) k_affine_gather(StepArgs<R> a) {
 __global__ void __launch_bounds__(CELL_THREADS, 3) k_affine_musl_cell(StepArgs<float> a) {
     __shared__ float corner[3 * 8][BRC];
     __shared__ Scales S;
+    pdl_wait();
+    affine_scales(a, S);   // before an empty brick leaves: CTA 0 records the scale
     const int b = blockIdx.x;
     const int lc = threadIdx.x >> 1, h = threadIdx.x & 1;
     const int *cs = a.cstart + (size_t)b * (BRC + 1);
@@ -1902,7 +1907,7 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_affine_musl_cell(StepArgs<f
     int ox, oy, oz;
     brick_origin(b, a.nbrick, ox, oy, oz);
     const int cx = ox + (lc % BRX), cy = oy + (lc / BRX) % BRY, cz = oz + lc / (BRX * BRY);
-    load_scales_musl(a, S);
+    __syncthreads();
     const size_t N = (size_t)a.g.nodec;
     const Particles<float> &P = a.P;
     float acc[3][4];
@@ -1969,22 +1974,18 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_affine_musl_cell(StepArgs<f
     }
 }
 
-template <typename R>
-__global__ void k_affine_scale(StepArgs<R> a) {
-    a.ctl->sc_musl.q = make_fix(a.nump * a.mmax * (double)bits_f(a.ctl->nxt[a.parity ^ 1][B_VMAX]) * 1.0000001);
-}
-
 template <typename R, int OX, int OY, int OZ>
 __global__ void __launch_bounds__(256) k_affine_musl(StepArgs<R> a) {
     constexpr int BX = BRX + OX, BY = BRY + OY, BZ = BRZ + OZ, BOX = BX * BY * BZ;
     extern __shared__ unsigned long long sacc[];   // 3 * BOX
     __shared__ Scales S;
+    affine_scales(a, S);   // before a CTA without work leaves: CTA 0 records the scale
     if ((int)blockIdx.x >= *a.nwork) return;
     const WorkItem w = a.work[blockIdx.x];
     int ox, oy, oz;
     brick_origin(w.tile, a.nbrick, ox, oy, oz);
     for (int i = threadIdx.x; i < 3 * BOX; i += blockDim.x) sacc[i] = 0ull;
-    load_scales_musl(a, S);
+    __syncthreads();
     const size_t N = (size_t)a.g.nodec;
     const Particles<R> &P = a.P;
     for (int p = w.begin + threadIdx.x; p < w.end; p += blockDim.x) {
@@ -2053,14 +2054,13 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid1(StepArgs<R> a) {
     pdl_wait();
     __shared__ double sh_d[32];
     __shared__ float sh_f[32];
-    __shared__ bool s_last;
     __shared__ Scales S;
     float gmax = 0.0f, neimax = 0.0f;
+    float eu = 0.0f, eue = 0.0f;   // the thread's sum of nei^2 as an unevaluated pair
     load_scales(a, S);
     const int ntl = LIST ? *a.ntlist : 1;
     for (int lt = LIST ? (int)blockIdx.x : 0; lt < ntl; lt += LIST ? (int)gridDim.x : 1) {
     const int t = LIST ? a.tlist[lt] : (int)blockIdx.x;
-    float eu = 0.0f;
     const bool active = LIST || a.all_tiles || a.tileflag[t];
     if (active) {
         int tx, ty, tz;
@@ -2090,7 +2090,11 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid1(StepArgs<R> a) {
         for (int k = 0; k < GRID_NPT; k++) {
             if (!in[k]) continue;
             const size_t n = nid[k];
-            if (!a.all_tiles) {
+            long long any = 0;
+#pragma unroll
+            for (int f = 0; f < NACC; f++) any |= q[k][f];
+            const bool set = any != 0;   // most nodes of a tile at the body's surface are not
+            if (!a.all_tiles && set) {
                 // cleared for the next step here, where their values are known:
                 // an untouched node of an active tile costs no store (F-bar:
                 // k_fbar_grid reads the nvof sums first; k_grid2 reads the mass)
@@ -2098,16 +2102,18 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid1(StepArgs<R> a) {
                 for (int f = 1; f < NACC; f++)
                     if (q[k][f] != 0 && !(a.fbar && f == 1)) a.acc[f * N + n] = 0ull;
             }
-            const R mass = unfx(q[k][0], S.m, (R)0);
-            R vof = unfx(q[k][1], S.v, (R)0);
-            R nv[3], na[3];
-            const R im = (mass > a.mtol) ? recip<R>(mass) : (R)0;   // one reciprocal per node
+            R vof = (R)0, nv[3] = {(R)0, (R)0, (R)0}, na[3] = {(R)0, (R)0, (R)0};
+            if (set) {
+                const R mass = unfx_int(q[k][0], S.m, (R)0);
+                vof = unfx_int(q[k][1], S.v, (R)0);
+                const R im = (mass > a.mtol) ? recip<R>(mass) : (R)0;   // one reciprocal per node
 #pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const R pc = unfx(q[k][2 + c], S.p, (R)0);
-                const R fc = unfx(q[k][5 + c], S.f, (R)0);
-                nv[c] = pc * im;
-                na[c] = fc * im;
+                for (int c = 0; c < 3; c++) {
+                    const R pc = unfx_int(q[k][2 + c], S.p, (R)0);
+                    const R fc = unfx_int(q[k][5 + c], S.f, (R)0);
+                    nv[c] = pc * im;
+                    na[c] = fc * im;
+                }
             }
             if (vof < a.mtol) vof = (R)0;
             const unsigned char bf = bfl[k];
@@ -2132,43 +2138,41 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid1(StepArgs<R> a) {
                 a.G[c * N + n] = gv;
                 gmax = fmaxf(gmax, fabsf((float)gv));
             }
-            R e = vof - (R)nvl[k];
-            e = e > (R)0 ? e : (R)0;
+            R e = (R)0;
+            if (set) {
+                e = vof - (R)nvl[k];
+                e = e > (R)0 ? e : (R)0;
+            }
             a.nei[n] = e;
-            eu += (float)e * (float)e;
+            {
+                const float e2 = (float)e * (float)e, t2 = __fadd_rn(eu, e2), u2 = __fsub_rn(t2, eu);
+                eue += __fadd_rn(__fsub_rn(eu, __fsub_rn(t2, u2)), __fsub_rn(e2, u2));
+                eu = t2;
+            }
             neimax = fmaxf(neimax, (float)e);
         }
     }
-    // deterministic sum of nei^2: per-tile partials (by list position in list
-    // mode), reduced in order by the last CTA
-    double ebl = block_reduce((double)eu, OpAddD(), sh_d);
-    if (threadIdx.x == 0) a.eu_part[LIST ? lt : t] = ebl;
-    __syncthreads();
     }
-    float gm = block_reduce(gmax, OpMaxF(), sh_f);
-    float nm = block_reduce(neimax, OpMaxF(), sh_f);
+    // the block's sum and maxima behind one barrier
+    double e2 = (double)eu + (double)eue;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        e2 += __shfl_down_sync(0xffffffffu, e2, o);
+        gmax = fmaxf(gmax, __shfl_down_sync(0xffffffffu, gmax, o));
+        neimax = fmaxf(neimax, __shfl_down_sync(0xffffffffu, neimax, o));
+    }
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (lane == 0) sh_d[wid] = e2, sh_f[wid] = gmax, sh_f[16 + wid] = neimax;
+    __syncthreads();
     if (threadIdx.x == 0) {
-        if (gm > 0.0f) atomic_max_pos(&a.ctl->cur[C_GMAX], gm * 1.000001f);
-        if (nm > 0.0f) atomic_max_pos(&a.ctl->cur[C_NEIMAX], nm * 1.000001f);
-        __threadfence();
-        unsigned prev = atomicAdd(&a.ctl->tile_counter, 1u);
-        s_last = (prev == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (s_last) {
-        __threadfence();
-        double acc = 0.0;
-        const int npart = LIST ? *a.ntlist : (int)gridDim.x;
-        for (int i = threadIdx.x; i < npart; i += blockDim.x) acc += ((volatile double *)a.eu_part)[i];
-        double tot = block_reduce(acc, OpAddD(), sh_d);
-        if (threadIdx.x == 0) {
-            a.ctl->eu_norm = tot;
-            a.ctl->tile_counter = 0u;
+        for (int w = 1; w < GRID_THREADS / 32; w++) {
+            e2 += sh_d[w];
+            gmax = fmaxf(gmax, sh_f[w]);
+            neimax = fmaxf(neimax, sh_f[16 + w]);
         }
-        // the gather's scales beside the P2G's (k_grid2 reads the mass scale), one per thread
-        if (threadIdx.x < 6)
-            (&a.ctl->sc_musl.m)[threadIdx.x] =
-                threadIdx.x < 4 ? (&S.m)[threadIdx.x] : make_fix(bound_musl(a, (int)threadIdx.x - 4));
+        a.eu_part[blockIdx.x] = e2;   // added in order by k_grid2
+        if (gmax > 0.0f) atomic_max_pos(&a.ctl->cur[C_GMAX], gmax * 1.000001f);
+        if (neimax > 0.0f) atomic_max_pos(&a.ctl->cur[C_NEIMAX], neimax * 1.000001f);
     }
 }
 
@@ -2177,17 +2181,25 @@ template <typename R, bool LIST>
 __global__ void __launch_bounds__(GRID_THREADS) k_grid2(StepArgs<R> a) {
     pdl_wait();
     __shared__ Scales S;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        // both deferred passes are over
-        a.ctl->n_miss_p2g = 0u;
-        a.ctl->n_miss_musl = 0u;
-        // b0 of DeltaCorrectionParticleShifting (material_point.cpp:219)
-        double gd = (double)(long long)a.ctl->geup_acc * a.ctl->sc_musl.gd.inv;
-        a.ctl->b0 = (!a.shifting || gd < (double)a.mtol) ? 0.0 : a.ctl->eu_norm / gd;
+    if (blockIdx.x == gridDim.x - 1) {
+        // one CTA beside the tiles': sum nei^2 in the order of k_grid1's CTAs, then b0 of
+        // DeltaCorrectionParticleShifting (material_point.cpp:219)
+        __shared__ double sh_d[32];
+        double acc = 0.0;
+        for (int i = threadIdx.x; i < a.eu_parts; i += blockDim.x) acc += a.eu_part[i];
+        const double eu = block_reduce(acc, OpAddD(), sh_d);
+        if (threadIdx.x == 0) {
+            const double gd = (double)(long long)a.ctl->geup_acc * a.ctl->sc_musl.gd.inv;
+            a.ctl->b0 = (!a.shifting || gd < (double)a.mtol) ? 0.0 : eu / gd;
+            // both deferred passes are over
+            a.ctl->n_miss_p2g = 0u;
+            a.ctl->n_miss_musl = 0u;
+        }
+        return;
     }
     load_scales_musl(a, S);
     const int ntl = LIST ? *a.ntlist : 1;
-    for (int lt = LIST ? (int)blockIdx.x : 0; lt < ntl; lt += LIST ? (int)gridDim.x : 1) {
+    for (int lt = LIST ? (int)blockIdx.x : 0; lt < ntl; lt += LIST ? (int)gridDim.x - 1 : 1) {
     const int t = LIST ? a.tlist[lt] : (int)blockIdx.x;
     if (!(LIST || a.all_tiles || a.tileflag[t])) return;
     int tx, ty, tz;
@@ -2250,8 +2262,8 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid2(StepArgs<R> a) {
 //   k_fbar_trial    per particle the step's dF = I + dt grad(nvel2) (the
 //                   update's own formula) and the trial J = Jbar det(dF),
 //                   stored; records max(J vol)
-//   k_fbar_scale    the fixed-point scale of the nodal sums from that bound
-//   k_fbar_scatter  sum_p N J vol into the nodes (int64 fixed point)
+//   k_fbar_scatter  sum_p N J vol into the nodes (int64 fixed point, the scale
+//                   from that bound)
 //   k_fbar_grid     nJbar = sum / nvof (0 where nvof <= mtol) into the free
 //                   gather field G; clears the sums and the nvof sums
 // FP32 keeps J - 1 in place of J (trial, projected and gathered): the sums
@@ -2316,6 +2328,7 @@ __device__ __forceinline__ R fbar_trial_j(const StepArgs<R> &a, const Particles<
 template <typename R, int OX, int OY, int OZ>
 __global__ void __launch_bounds__(256) k_fbar_trial(StepArgs<R> a) {
     __shared__ float sh_f[32];
+    pdl_wait();
     const Particles<R> &P = a.P;
     float jvmax = 0.0f;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < a.num; p += (int64_t)gridDim.x * blockDim.x) {
@@ -2331,15 +2344,22 @@ __global__ void __launch_bounds__(256) k_fbar_trial(StepArgs<R> a) {
     if (threadIdx.x == 0 && m > 0.0f) atomic_max_pos(&a.ctl->cur[C_JVMAX], m * 1.000001f);
 }
 
+// The fixed-point scale of the projected J vol sums, from the bound k_fbar_trial
+// recorded: by every CTA for itself (the caller's next barrier publishes it), and
+// by CTA 0 for k_fbar_grid.
 template <typename R>
-__global__ void k_fbar_scale(StepArgs<R> a) {
-    a.ctl->sc_fbar = make_fix(a.nump * (double)bits_f(a.ctl->cur[C_JVMAX]) * 1.0000001);
+__device__ __forceinline__ void fbar_scale(const StepArgs<R> &a, Fix &F) {
+    if (threadIdx.x != 0) return;
+    const Fix f = make_fix(a.nump * (double)bits_f(a.ctl->cur[C_JVMAX]) * 1.0000001);
+    F = f;
+    if (blockIdx.x == 0) a.ctl->sc_fbar = f;
 }
 
 template <typename R, int OX, int OY, int OZ>
 __global__ void __launch_bounds__(256) k_fbar_scatter(StepArgs<R> a) {
     __shared__ Fix F;
-    if (threadIdx.x == 0) F = a.ctl->sc_fbar;
+    pdl_wait();
+    fbar_scale(a, F);
     __syncthreads();
     const Particles<R> &P = a.P;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < a.num; p += (int64_t)gridDim.x * blockDim.x) {
@@ -2372,11 +2392,12 @@ __global__ void __launch_bounds__(256) k_fbar_scatter(StepArgs<R> a) {
 __global__ void __launch_bounds__(CELL_THREADS, 3) k_fbar_scatter_cell(StepArgs<float> a) {
     __shared__ float corner[8][BRC];
     __shared__ Fix F;
+    pdl_wait();
+    fbar_scale(a, F);   // before an empty brick leaves: CTA 0 records it
     const int b = blockIdx.x;
     const int lc = threadIdx.x >> 1, h = threadIdx.x & 1;
     const int *cs = a.cstart + (size_t)b * (BRC + 1);
     if (cs[0] == cs[BRC]) return;   // empty brick (uniform across the CTA)
-    if (threadIdx.x == 0) F = a.ctl->sc_fbar;
     int ox, oy, oz;
     brick_origin(b, a.nbrick, ox, oy, oz);
     const int cx = ox + (lc % BRX), cy = oy + (lc / BRX) % BRY, cz = oz + lc / (BRX * BRY);
@@ -2433,6 +2454,7 @@ template <typename R, bool LIST>
 __global__ void __launch_bounds__(256) k_fbar_grid(StepArgs<R> a) {
     __shared__ Scales S;
     __shared__ Fix F;
+    pdl_wait();
     load_scales(a, S);
     if (threadIdx.x == 0) F = a.ctl->sc_fbar;
     __syncthreads();
@@ -2485,6 +2507,7 @@ template <typename R, int OX, int OY, int OZ, bool FBAR = false>
 __global__ void __launch_bounds__(256) k_g2p_update(StepArgs<R> a) {
     __shared__ float sh_f[32];
     __shared__ int sh_i[32];
+    pdl_wait();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const size_t N = (size_t)a.g.nodec;
     const Particles<R> &P = a.P;
@@ -3216,13 +3239,13 @@ static int list_grid(const mpm_ctx *c, int per_sm) {
     return std::min(c->g.nbricks, per_sm * num_sms());
 }
 
-// The moment P2G and the cell scatters of a fused explicit step start the step
-// themselves (p2g_scales).  A step whose nodal sums are downloaded records its
+// The moment P2G, the affine P2G and the cell scatters of a fused explicit step start
+// the step themselves (p2g_scales).  A step whose nodal sums are downloaded records its
 // scales as well, and an implicit one may repeat its P2G: k_step_reset.
 static bool begins_itself(const mpm_ctx *c) {
     if (c->write_nodal_dl || c->nreal == 27 || !c->cell_scatter) return false;
     const bool linear32 = c->precision == 32 && c->g.order[0] == 1;
-    return linear32 ? !c->affine && c->tune.p2g_moments && c->tune.p2g_moments != 3 : true;
+    return linear32 ? c->affine || (c->tune.p2g_moments && c->tune.p2g_moments != 3) : true;
 }
 
 // The grid passes walk a list of the active tiles, which takes a launch to make;
@@ -3286,8 +3309,8 @@ static mpm_status launch_particle_kernel(mpm_ctx *c, int which) {
         if constexpr (sizeof(R) == 4 && OX == 1 && OY == 1 && OZ == 1) {
             if (c->affine && c->cell_scatter) {
                 // TPIC / APIC: per-cell register sums with the affine momentum
-                k_p2g_cell<2, true><<<c->g.nbricks, CELL_THREADS, 0, c->stream>>>(a);
-                k_p2g_misses<true><<<2 * num_sms(), 256, 0, c->stream>>>(a);
+                launch(c->pdl != 0, k_p2g_cell<2, true>, c->g.nbricks, CELL_THREADS, 0, c->stream, a);
+                launch(c->pdl != 0, k_p2g_misses<true>, 2 * num_sms(), 256, 0, c->stream, a);
                 timer_end(c, K_P2G);
                 c->launches += 2;
                 return check_launch(c);
@@ -3354,12 +3377,11 @@ static mpm_status launch_particle_kernel(mpm_ctx *c, int which) {
         size_t smem = (size_t)3 * BOX * sizeof(unsigned long long);
         if (c->affine) {
             const int nb = (int)std::min<int64_t>((c->num + 255) / 256, 8 * num_sms());
-            k_affine_gather<R, OX, OY, OZ><<<nb, 256, 0, c->stream>>>(a);
-            k_affine_scale<R><<<1, 1, 0, c->stream>>>(a);
+            launch(c->pdl != 0, k_affine_gather<R, OX, OY, OZ>, nb, 256, 0, c->stream, a);
             bool cell = false;
             if constexpr (sizeof(R) == 4 && OX == 1 && OY == 1 && OZ == 1) {
                 if (c->cell_scatter) {
-                    k_affine_musl_cell<<<c->g.nbricks, CELL_THREADS, 0, c->stream>>>(a);
+                    launch(c->pdl != 0, k_affine_musl_cell, c->g.nbricks, CELL_THREADS, 0, c->stream, a);
                     cell = true;
                 }
             }
@@ -3371,7 +3393,7 @@ static mpm_status launch_particle_kernel(mpm_ctx *c, int which) {
                                      (int)smem);
                 k_affine_musl<R, OX, OY, OZ><<<c->nwork_cap, 256, smem, c->stream>>>(a);
             }
-            c->launches += 2;
+            c->launches++;
         } else if (c->cell_scatter) {
             launch_gather<R>(a, c->g.order, num_sms(), c->pdl != 0, c->stream);
             launch_cell_scatter<R>(a, c->g.order, CELL_MUSL, c->g.nbricks, num_sms(), c->pdl != 0, c->stream);
@@ -3387,22 +3409,20 @@ static mpm_status launch_particle_kernel(mpm_ctx *c, int which) {
         if (c->fbar) {
             const int nb = (int)((c->num + 255) / 256);
             const int pg = (int)std::min<int64_t>(nb, 8 * num_sms());
-            k_fbar_trial<R, OX, OY, OZ><<<pg, 256, 0, c->stream>>>(a);
-            k_fbar_scale<R><<<1, 1, 0, c->stream>>>(a);
+            auto go = [&](auto k, int grid) { launch(c->pdl != 0, k, grid, 256, 0, c->stream, a); };
+            go(k_fbar_trial<R, OX, OY, OZ>, pg);
             bool cell = false;
             if constexpr (sizeof(R) == 4 && OX == 1 && OY == 1 && OZ == 1) {
                 if (c->cell_scatter) {
-                    k_fbar_scatter_cell<<<c->g.nbricks, CELL_THREADS, 0, c->stream>>>(a);
+                    launch(c->pdl != 0, k_fbar_scatter_cell, c->g.nbricks, CELL_THREADS, 0, c->stream, a);
                     cell = true;
                 }
             }
-            if (!cell) k_fbar_scatter<R, OX, OY, OZ><<<pg, 256, 0, c->stream>>>(a);
-            if (use_tile_list(c))
-                k_fbar_grid<R, true><<<std::min(c->g.ntiles, 6 * num_sms()), 256, 0, c->stream>>>(a);
-            else
-                k_fbar_grid<R, false><<<c->g.ntiles, 256, 0, c->stream>>>(a);
-            k_g2p_update<R, OX, OY, OZ, true><<<nb, 256, 0, c->stream>>>(a);
-            c->launches += 5;
+            if (!cell) go(k_fbar_scatter<R, OX, OY, OZ>, pg);
+            if (use_tile_list(c)) go(k_fbar_grid<R, true>, std::min(c->g.ntiles, 6 * num_sms()));
+            else go(k_fbar_grid<R, false>, c->g.ntiles);
+            go(k_g2p_update<R, OX, OY, OZ, true>, nb);
+            c->launches += 4;
             timer_end(c, K_G2P_UPDATE);
             return check_launch(c);
         }
@@ -3432,7 +3452,7 @@ static mpm_status launch_particle_kernel(mpm_ctx *c, int which) {
         }
         if (!staged) {
             const int nb = (int)((c->num + 255) / 256);
-            k_g2p_update<R, OX, OY, OZ><<<nb, 256, 0, c->stream>>>(a);
+            launch(c->pdl != 0, k_g2p_update<R, OX, OY, OZ>, nb, 256, 0, c->stream, a);
         }
         timer_end(c, K_G2P_UPDATE);
     }
@@ -3460,6 +3480,7 @@ static mpm_status grid_kernel(mpm_ctx *c, int which) {
     // persistent grids of as many CTAs as reside per SM: 4 for the first pass
     // (64 registers with its batched loads), 6 for the second (40)
     const int lgrid1 = std::min(c->g.ntiles, 4 * num_sms()), lgrid = std::min(c->g.ntiles, 6 * num_sms());
+    a.eu_parts = list ? lgrid1 : c->g.ntiles;
     if (which == 0) {
         timer_begin(c, K_GRID1);
         if (list) {
@@ -3468,13 +3489,13 @@ static mpm_status grid_kernel(mpm_ctx *c, int which) {
             launch(c->pdl != 0, k_grid1<R, true>, lgrid1, GRID_THREADS, 0, c->stream, a);
             c->launches++;
         } else {
-            k_grid1<R, false><<<c->g.ntiles, GRID_THREADS, 0, c->stream>>>(a);
+            launch(c->pdl != 0, k_grid1<R, false>, c->g.ntiles, GRID_THREADS, 0, c->stream, a);
         }
         timer_end(c, K_GRID1);
     } else {
         timer_begin(c, K_GRID2);
-        if (list) launch(c->pdl != 0, k_grid2<R, true>, lgrid, GRID_THREADS, 0, c->stream, a);
-        else k_grid2<R, false><<<c->g.ntiles, GRID_THREADS, 0, c->stream>>>(a);
+        if (list) launch(c->pdl != 0, k_grid2<R, true>, lgrid + 1, GRID_THREADS, 0, c->stream, a);
+        else launch(c->pdl != 0, k_grid2<R, false>, c->g.ntiles + 1, GRID_THREADS, 0, c->stream, a);
         timer_end(c, K_GRID2);
     }
     c->launches++;

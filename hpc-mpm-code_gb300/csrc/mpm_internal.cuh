@@ -78,8 +78,6 @@ struct DevCtl {
     unsigned int nxt[2][B_NB];
     unsigned int cur[C_NC];
     unsigned long long geup_acc;     // fixed-point sum of |geup|^2
-    double eu_norm;                  // sum nei^2 (deterministic per-tile reduction)
-    unsigned int tile_counter;
     unsigned int err_oob;
     unsigned int err_nonfinite;
     unsigned int tile_misses;
@@ -89,8 +87,8 @@ struct DevCtl {
     unsigned int n_miss_p2g;         // particles queued for the deferred P2G pass this step
     unsigned int n_miss_musl;        // particles queued for the deferred gather/MUSL pass this step
     Scales sc_p2g;                   // this step's P2G scales (k_step_reset)
-    Scales sc_musl;                  // this step's gather/MUSL scales (last CTA of k_grid1)
-    Fix sc_fbar;                     // F-bar: scale of the projected J vol sums (k_fbar_scale)
+    Scales sc_musl;                  // this step's gather/MUSL scales (musl_scales)
+    Fix sc_fbar;                     // F-bar: scale of the projected J vol sums (fbar_scale)
 };
 
 template <typename R>

@@ -31,7 +31,8 @@ struct StepArgs {
     const unsigned char *bcflag;
     const R *bcval;
     unsigned char *tileflag;
-    double *eu_part;
+    double *eu_part;            // sums of nei^2 by CTA of k_grid1
+    int eu_parts;               // how many
     DevCtl *ctl;
     const int *iprop;
     const double *matprop;
@@ -120,9 +121,9 @@ __device__ __forceinline__ void begin_step_ctl(const StepArgs<R> &a) {
 static_assert(B_NB <= 8 && C_NC <= 16, "one lane per slot");
 
 // The scales of a step: the P2G ones by k_step_reset or, where the P2G kernel
-// starts the step itself, by each of its CTAs; the gather/MUSL ones by the last
-// CTA of k_grid1 (they depend on the grid
-// maxima it records).  Kernels copy them into shared memory.
+// starts the step itself, by each of its CTAs; the gather/MUSL ones by the first
+// kernel that gathers (they depend on the grid maxima that k_grid1 records).
+// Kernels copy them into shared memory.
 template <typename R>
 __device__ __forceinline__ void load_scales_from(const Scales *src, Scales &sh) {
     constexpr int W = (int)(sizeof(Scales) / 4);
@@ -151,6 +152,29 @@ __device__ __forceinline__ void p2g_scales(const StepArgs<R> &a, Scales &sh) {
 template <typename R>
 __device__ __forceinline__ void load_scales_musl(const StepArgs<R> &a, Scales &sh) {
     load_scales_from<R>(&a.ctl->sc_musl, sh);
+}
+// The scales of the first kernel that gathers from k_grid1's fields: every CTA
+// derives them from the grid's maxima, and CTA 0 (`all`: every CTA, where CTA 0 may
+// have no work) records them for the passes behind it.  (The last CTA of k_grid1
+// did this before, 4 us of every step: it waited for all others, read back their
+// partials, and the gather waited for it.)
+template <typename R>
+__device__ __forceinline__ void musl_scales(const StepArgs<R> &a, Scales &sh, bool all = false) {
+    if (threadIdx.x < 6) {
+        const Fix f = threadIdx.x < 4 ? (&a.ctl->sc_p2g.m)[threadIdx.x] : make_fix(bound_musl(a, (int)threadIdx.x - 4));
+        (&sh.m)[threadIdx.x] = f;
+        if (all || blockIdx.x == 0) (&a.ctl->sc_musl.m)[threadIdx.x] = f;
+    }
+    __syncthreads();
+}
+// The momentum scale of the affine re-projection, from the velocities that the
+// gather recorded (the caller's next barrier publishes it); CTA 0 records it.
+template <typename R>
+__device__ __forceinline__ void affine_scales(const StepArgs<R> &a, Scales &sh) {
+    if (threadIdx.x != 0) return;
+    const Fix f = make_fix(a.nump * a.mmax * (double)bits_f(a.ctl->nxt[a.parity ^ 1][B_VMAX]) * 1.0000001);
+    sh.q = f;
+    if (blockIdx.x == 0) a.ctl->sc_musl.q = f;
 }
 
 // Block-wide reduction (fixed order: deterministic); result valid in thread 0.
