@@ -8,10 +8,10 @@
 //   SolveSolid (Newton)      solve_solid_implicit.cpp:65-103         -> implicit_newton
 //   BCNRSet / Predict        implicit_mpm_solid.h:55-64,
 //                            nonlinear_time_integration.cpp:59-71    -> k_imp_bcnr, k_imp_predict
-//   AssembleSystem           solve_solid_implicit.cpp:105-204        -> k_imp_assemble, k_imp_rhs_diag
+//   AssembleSystem           solve_solid_implicit.cpp:105-204        -> k_imp_assemble, k_imp_assemble_cells, k_imp_rhs_diag
 //   ComputeTangentModulus    solve_solid_implicit.cpp:34-63          -> pair loop of k_imp_assemble
 //   BuildDiagonalPreconditioner crsmat.cpp:87-184                     -> k_imp_rhs_diag, k_imp_scale
-//   MatVecMult               solver.cpp:405-433                      -> k_imp_matvec
+//   MatVecMult               solver.cpp:405-433                      -> k_imp_matvec, k_imp_matvec_split
 //   GPBiCGSafe               solver.cpp:19-141                       -> conjugate gradients (the scaled
 //                            system is symmetric), stopped on the same squared-norm ratio
 //   CheckNRConvergence       solver.cpp:484-593                      -> newton_residuals
@@ -1067,25 +1067,33 @@ __global__ void k_split_df(const double *__restrict__ x, float *__restrict__ xh,
 // plus e xl, and the row sums are carried as an unevaluated FP32 pair
 // (Knuth's two-sum for the high part).  About 44 bits of the sum, on the FP32
 // pipe (GB300 executes 2 FP64 FMAs per SM and clock, against 128 FP32 lanes).
+// The points' slots are split over MV_G threads as in k_imp_matvec_split, in the same
+// pair arithmetic (one thread per point: 90 us at 274,625 points; the learned step,
+// with five or six of them, 8.00 -> 7.81 ms).
 template <int RX, int RY, int RZ>
-__global__ void __launch_bounds__(256) k_imp_matvec_df(ImpArgs a, const float *A, const float *__restrict__ xh,
-                                                       const float *__restrict__ xl, double *y) {
+__global__ void __launch_bounds__(MV_NODES * MV_G) k_imp_matvec_df(ImpArgs a, const float *__restrict__ A,
+                                                                   const float *__restrict__ xh,
+                                                                   const float *__restrict__ xl, double *y) {
     constexpr int SX = 2 * RX + 1, SY = 2 * RY + 1, NS = SX * SY * (2 * RZ + 1);
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= a.nodec) return;
+    constexpr int SL = 2 * ((NS + 2 * MV_G - 1) / (2 * MV_G));
+    __shared__ float ph[MV_G][3][MV_NODES], pl[MV_G][3][MV_NODES];
+    const int lane = threadIdx.x % MV_NODES, grp = threadIdx.x / MV_NODES;
+    const int n = blockIdx.x * MV_NODES + lane;
     const size_t N = (size_t)a.nodec;
-    int i, j, k;
-    node_ijk(n, a.nnc, i, j, k);
     float sh[3] = {0.0f, 0.0f, 0.0f}, sl[3] = {0.0f, 0.0f, 0.0f};
+    int i = 0, j = 0, k = 0;
+    if (n < a.nodec) node_ijk(n, a.nnc, i, j, k);
 #pragma unroll
-    for (int s = 0; s < NS; s++) {
+    for (int q = 0; q < SL; q++) {
+        const int s = grp * SL + q;
+        if (s >= NS || n >= a.nodec) continue;
         const int ii = i + s % SX - RX, jj = j + (s / SX) % SY - RY, kk = k + s / (SX * SY) - RZ;
         if (ii < 0 || jj < 0 || kk < 0 || ii >= a.nnc[0] || jj >= a.nnc[1] || kk >= a.nnc[2]) continue;
         const size_t col = ii + (size_t)a.nnc[0] * (jj + (size_t)a.nnc[1] * kk);
         const float h[3] = {__ldg(xh + col), __ldg(xh + N + col), __ldg(xh + 2 * N + col)};
         const float l[3] = {__ldg(xl + col), __ldg(xl + N + col), __ldg(xl + 2 * N + col)};
         float e[9];
-        if ((s & 1) == 0) {
+        if ((q & 1) == 0) {   // SL is even
 #pragma unroll
             for (int t = 0; t < 4; t++) {
                 const float2 v = __ldg(reinterpret_cast<const float2 *>(A + aidx(s * 9 + 2 * t, n, a.qp)));
@@ -1118,9 +1126,20 @@ __global__ void __launch_bounds__(256) k_imp_matvec_df(ImpArgs a, const float *A
                 sl[r] += err + fmaf(ev, l[c], pe);
             }
     }
-    const unsigned char bf = a.bcflag[n];
 #pragma unroll
-    for (int c = 0; c < 3; c++) y[c * N + n] = (bf & (1 << c)) ? 0.0 : (double)sh[c] + (double)sl[c];
+    for (int c = 0; c < 3; c++) {
+        ph[grp][c][lane] = sh[c];
+        pl[grp][c][lane] = sl[c];
+    }
+    __syncthreads();
+    if (grp >= 3 || n >= a.nodec) return;
+    float s = ph[0][grp][lane], e = pl[0][grp][lane];
+#pragma unroll
+    for (int q = 1; q < MV_G; q++) {
+        pair_add(s, e, ph[q][grp][lane]);
+        e += pl[q][grp][lane];
+    }
+    y[grp * N + n] = (a.bcflag[n] & (1 << grp)) ? 0.0 : (double)s + (double)e;
 }
 
 // ScaleSolution + BCResidualSet: xs = x / D, r = b D (crsmat.cpp:190-209)
@@ -2063,13 +2082,14 @@ static void launch_matvec(mpm_ctx *c, const ImpArgs &a, int nb, const double *x,
         // FP32 operator, true residual / Newton check: double-float arithmetic
         const int n3 = 3 * c->g.nodec;
         k_split_df<<<(n3 + 255) / 256, 256, 0, c->stream>>>(x, s->dfx, s->dfx + n3, n3);
+        const int nbs = (c->g.nodec + MV_NODES - 1) / MV_NODES;
         const float *A = (const float *)s->A;
         if (o[0] == 1 && o[1] == 1 && o[2] == 1)
-            k_imp_matvec_df<1, 1, 1><<<nb, 256, 0, c->stream>>>(a, A, s->dfx, s->dfx + n3, y);
+            k_imp_matvec_df<1, 1, 1><<<nbs, MV_NODES * MV_G, 0, c->stream>>>(a, A, s->dfx, s->dfx + n3, y);
         else if (o[1] == 2)
-            k_imp_matvec_df<2, 2, 2><<<nb, 256, 0, c->stream>>>(a, A, s->dfx, s->dfx + n3, y);
+            k_imp_matvec_df<2, 2, 2><<<nbs, MV_NODES * MV_G, 0, c->stream>>>(a, A, s->dfx, s->dfx + n3, y);
         else
-            k_imp_matvec_df<2, 1, 2><<<nb, 256, 0, c->stream>>>(a, A, s->dfx, s->dfx + n3, y);
+            k_imp_matvec_df<2, 1, 2><<<nbs, MV_NODES * MV_G, 0, c->stream>>>(a, A, s->dfx, s->dfx + n3, y);
     } else if (hi) {
         go(float(), double());
     } else {
