@@ -9,21 +9,23 @@
 //                 module/material_point.cpp:179-185)
 //   g2p_musl      particle velocity gather, MUSL momentum re-scatter, |geup|^2
 //                 (var_trans_solid_explicit.cpp:211-240,101-129, material_point.cpp:192-217)
-//   k_grid2       MUSL nvel = p/m + BC, shifting b0, clears the accumulators
+//   k_grid2       MUSL nvel = p/m + BC, shifting b0 from sum nei^2
 //                 (var_trans_solid_explicit.cpp:131-146, material_point.cpp:219)
 //   k_g2p_update  F update, position update + shift, vol = J vol0, stress
 //                 (var_trans_solid_explicit.cpp:247-296,150-185)
 //
-// Two scatter formulations:
-//   * FP32 with linear shape functions (8 nodes per particle): one thread per
+// Scatter formulations:
+//   * FP32 with linear shape functions (8 nodes per particle): two threads per
 //     cell of a 4x4x8-cell brick.  Particles are sorted by (brick, cell, load
 //     index), so a thread sums its cell's particles into FP32 registers in a
 //     fixed order, writes them to shared memory as cell corners, and a node
 //     pass adds the 8 corners of each node in a fixed order before one int64
 //     fixed-point RED per node and field.  Runs are bitwise reproducible.
-//   * FP64, and quadratic B-splines: particles of a brick chunk convert every
-//     contribution to int64 fixed point and scatter into a shared staging box
-//     with atomics; the sums are exact and independent of particle order.
+//   * FP64, quadratic B-splines, and the implicit solid's P2G: per-cell register
+//     sums in mpm_cells.cu.
+//   * With mpm_config.scatter = 1, any of these: particles of a brick chunk convert
+//     every contribution to int64 fixed point and scatter into a shared staging
+//     box with atomics; the sums are exact and independent of particle order.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -2049,6 +2051,11 @@ constexpr int GRID_THREADS = 256;                            // threads of a gri
 constexpr int GRID_NPT = TILE * TILE * TILE / GRID_THREADS;  // nodes of a tile per thread
 static_assert(GRID_NPT * GRID_THREADS == TILE * TILE * TILE, "a grid-pass CTA covers its tile exactly");
 
+// Bound by the latency of its loads and, before, by a tail: 4 us per step in which the
+// last CTA added the partials of all and derived the gather's scales (now in k_grid2
+// and musl_scales), a reduction per tile, and eight 64-bit conversions per node on the
+// FP64 pipe (ll2f takes the integer pipes; 59 % of the FP64 pipe was busy).  With the
+// tile list: 8,000 particles 12.7 -> 9.7 us, 4,096,000 35.7 -> 26.4, 64 scenes 55.7 -> 44.4.
 template <typename R, bool LIST>
 __global__ void __launch_bounds__(GRID_THREADS) k_grid1(StepArgs<R> a) {
     pdl_wait();
@@ -3478,7 +3485,7 @@ static mpm_status grid_kernel(mpm_ctx *c, int which) {
     StepArgs<R> a = make_args<R>(c);
     const bool list = use_tile_list(c);
     // persistent grids of as many CTAs as reside per SM: 4 for the first pass
-    // (64 registers with its batched loads), 6 for the second (40)
+    // (64 registers with its batched loads), 6 for the second (40) and one CTA for b0
     const int lgrid1 = std::min(c->g.ntiles, 4 * num_sms()), lgrid = std::min(c->g.ntiles, 6 * num_sms());
     a.eu_parts = list ? lgrid1 : c->g.ntiles;
     if (which == 0) {

@@ -210,7 +210,7 @@ struct mpm_ctx {
     int stage = 0;   // 0 idle, 1 after p2g, 2 after grid update
     bool accum_dirty = false;
     bool write_nodal_dl = false;
-    int cell_scatter = 1;   // FP32 linear: per-cell register scatter (else staging-box atomics)
+    int cell_scatter = 1;   // per-cell register scatter (0: staging-box atomics)
     int tma_update = 1;     // FP32 linear: particle update with bulk-copy staged input
     int pdl = 1;            // step kernels launched with programmatic dependent launch (MPM_GB300_PDL=0: off)
     int alternate = 1;      // particle kernels walk bricks / chunks in alternating directions (MPM_GB300_ALTERNATE=0: forward)

@@ -87,7 +87,7 @@ typedef struct {
     int precision;      /* 32: FP32 particle/grid arithmetic; 64: FP64 */
     int shifting;       /* 1: DeltaCorrectionParticleShifting as the reference; 0: off */
     int resort_period;  /* physical re-sort of particles by brick every N steps (>= 1); 0 = default (8) */
-    int scatter;        /* 0: per-cell register scatter for FP32 linear grids (default); 1: staging-box atomics */
+    int scatter;        /* 0: per-cell register scatter and FP32 assembly (default); 1: atomics per particle */
     int implicit;       /* 1: implicit solid context (particles carry acceleration; mpm_gpu_implicit_*) */
     int fbar;           /* 1: F-bar projection (Fbar_flag, module/solid/explicit/fbar_projection.cpp:18-93);
                            explicit contexts only */
@@ -197,7 +197,7 @@ typedef struct {
     int64_t resorts;        /* physical re-sorts done */
     int64_t kernel_launches;/* kernels launched by this context */
     int64_t out_of_box;     /* particles found outside the grid (clamped) */
-    int64_t tile_misses;    /* particles scattered outside their tile's staging box, last step */
+    int64_t tile_misses;    /* particles scattered outside their sorted cell or staging box, last step */
     int32_t ntiles;
     int32_t nwork;
 } mpm_stats;
