@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_p2g_cell(StepArgs<float>
     __shared__ Scales S;
     __shared__ int sh_red[32];
     pdl_wait();
-    p2g_scales(a, S);   // before an empty brick leaves: CTA 0 starts the step
+    if (blockIdx.x == 0) p2g_scales(a, S);   // CTA 0 starts the step, also where its brick is empty
     const int b = blockIdx.x;
     const int lc = threadIdx.x >> 1, h = threadIdx.x & 1;
     const int *cs = a.cstart + (size_t)b * (BRC + 1);
@@ -242,7 +242,8 @@ __global__ void __launch_bounds__(CELL_THREADS, MINB) k_p2g_cell(StepArgs<float>
     brick_origin(b, a.nbrick, ox, oy, oz);
     const int cx = ox + (lc % BRX), cy = oy + (lc / BRX) % BRY, cz = oz + lc / (BRX * BRY);
     const int p0 = cs[lc], p1 = cs[lc + 1];
-    __syncthreads();
+    // one warp's work, beside the others' particles; read after the node pass's barrier
+    if (blockIdx.x != 0) p2g_scales(a, S);
     const float fxg = a.grav[0] * a.facl, fyg = a.grav[1] * a.facl, fzg = a.grav[2] * a.facl;
     const Particles<float> &P = a.P;
     float acc[NACC][4];
@@ -1901,7 +1902,7 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_affine_musl_cell(StepArgs<f
     __shared__ float corner[3 * 8][BRC];
     __shared__ Scales S;
     pdl_wait();
-    affine_scales(a, S);   // before an empty brick leaves: CTA 0 records the scale
+    if (blockIdx.x == 0) affine_scales(a, S);   // CTA 0 records the scale, also where its brick is empty
     const int b = blockIdx.x;
     const int lc = threadIdx.x >> 1, h = threadIdx.x & 1;
     const int *cs = a.cstart + (size_t)b * (BRC + 1);
@@ -1909,7 +1910,7 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_affine_musl_cell(StepArgs<f
     int ox, oy, oz;
     brick_origin(b, a.nbrick, ox, oy, oz);
     const int cx = ox + (lc % BRX), cy = oy + (lc / BRX) % BRY, cz = oz + lc / (BRX * BRY);
-    __syncthreads();
+    if (blockIdx.x != 0) affine_scales(a, S);   // read after the barrier below
     const size_t N = (size_t)a.g.nodec;
     const Particles<float> &P = a.P;
     float acc[3][4];
@@ -1945,8 +1946,9 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_affine_musl_cell(StepArgs<f
                     for (int f = 0; f < 3; f++) acc[f][i + 2 * j] += Nm * vn[f];
                 } else {
                     const size_t gn = node_id(a.g, px + i, py + j, pz + h);
+                    const Fix q = affine_fix(a);
 #pragma unroll
-                    for (int f = 0; f < 3; f++) atomic_add_i64(&a.acc2[f * N + gn], fx(Nm * vn[f], S.q));
+                    for (int f = 0; f < 3; f++) atomic_add_i64(&a.acc2[f * N + gn], fx(Nm * vn[f], q));
                 }
             }
     }

@@ -170,9 +170,13 @@ __device__ __forceinline__ void musl_scales(const StepArgs<R> &a, Scales &sh, bo
 // The momentum scale of the affine re-projection, from the velocities that the
 // gather recorded (the caller's next barrier publishes it); CTA 0 records it.
 template <typename R>
+__device__ __forceinline__ Fix affine_fix(const StepArgs<R> &a) {
+    return make_fix(a.nump * a.mmax * (double)bits_f(a.ctl->nxt[a.parity ^ 1][B_VMAX]) * 1.0000001);
+}
+template <typename R>
 __device__ __forceinline__ void affine_scales(const StepArgs<R> &a, Scales &sh) {
     if (threadIdx.x != 0) return;
-    const Fix f = make_fix(a.nump * a.mmax * (double)bits_f(a.ctl->nxt[a.parity ^ 1][B_VMAX]) * 1.0000001);
+    const Fix f = affine_fix(a);
     sh.q = f;
     if (blockIdx.x == 0) a.ctl->sc_musl.q = f;
 }
