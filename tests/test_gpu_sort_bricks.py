@@ -1,4 +1,4 @@
-"""The re-sort over grids of one and of several scan segments (8192 bricks each) and
+"""The re-sort over grids of one and of several scan segments (4096 bricks each) and
 with bricks that do and do not fit the cell sort's shared memory (4096 particles).
 
 A cell's particles come out in load order whatever the grid around the body, and
