@@ -14,20 +14,21 @@
 // shared-memory atomics, one per particle, node and field.  P2G class per step,
 // staging box -> here: FP64 linear, 201,872 particles, 296 -> 128 us; FP32
 // B-splines, 216,000 particles, 444 -> 66 us; FP64 B-splines, 46,656 particles,
-// 643 -> 146 us; implicit FP32 linear, 1,728,000 particles, 802 -> 62 us.
+// 643 -> 146 us; implicit FP32 linear, 1,728,000 particles, 802 -> 116 us (66 with plain
+// FP32 sums).
 //
-// FP32 B-splines form each contribution as the staging box (mpm_explicit.cu)
-// does and sum it in an unevaluated pair of FP32 numbers (two-sum: 48 bits),
-// which is as exact as the box's int64 sums and leaves the step's results as they
-// were.  (Plain FP32 sums took 47 us in place of 66, but the sums of 216
-// contributions are far more exact than an FP32 number, and the stresses of a
-// nearly uniform velocity field moved by 5e-5; int64 sums took 185 us, in the
-// float to int64 conversions.)  32 cells per CTA and two CTAs per SM: 16, 64 or
-// one CTA measured 78 to 95 us.
-// FP64 sums, and the FP32 ones of the implicit solid on linear grids, are kept
-// in the working precision.
+// FP32 (B-splines, and the implicit solid's P2G on linear grids) forms each
+// contribution as the staging box (mpm_explicit.cu) does and sums it in an
+// unevaluated pair of FP32 numbers (two-sum: 48 bits), which is as exact as the
+// box's int64 sums and leaves the step's results as they were.  (Plain FP32 sums
+// of the B-splines took 47 us in place of 66, but the sums of 216 contributions are
+// far more exact than an FP32 number, and the stresses of a nearly uniform velocity
+// field moved by 5e-5; the implicit P2G's nodal mass, 64 particles per cell, was up to
+// 3.2 x 2^-24 off, and within 2 x 2^-24 with pairs.  int64 sums took 185 us, in the float to int64 conversions.)
+// 32 cells per CTA and two CTAs per SM: 16, 64 or one CTA measured 78 to 95 us.
+// FP64 sums are kept in FP64.
 //
-// On those, within a cell the weights are polynomials of the offset t in [0, 1)
+// There, within a cell the weights are polynomials of the offset t in [0, 1)
 // from its lower face, with coefficients that depend on the cell alone
 // (CellAxis): no division, no search for the spline's piece.  FP64 grids are
 // bound by the FP64 pipe (2 FMAs per SM and clock; ncu: 71 % busy in the linear
@@ -172,13 +173,14 @@ __device__ __forceinline__ long long sum_fixed(const Pair2 &p, int w, const Fix 
 
 template <typename R, int OX, int OY, int OZ>
 struct CellShape {
-    // FP32 B-splines: sums as exact as the staging box's
-    static constexpr bool EXACT = sizeof(R) == 4 && OX == 2;
+    // FP32 (B-splines, and the implicit solid's P2G): sums as exact as the staging box's
+    static constexpr bool EXACT = sizeof(R) == 4;
     using Sum = typename std::conditional<EXACT, Pair2, R>::type;
     static constexpr int W = EXACT ? 2 : 1;               // fields per sum
     static constexpr int NX = OX + 1, NY = OY + 1, NZ = OZ + 1, NE = NX * NY * NZ;
-    // rows per thread: both rows of a z-layer when linear, one row otherwise
-    static constexpr int JP = (OX == 1 && OY == 1) ? NY : 1;
+    // rows per thread: both rows of a z-layer when FP64 and linear, one row otherwise
+    // (pairs take twice the registers)
+    static constexpr int JP = (!EXACT && OX == 1 && OY == 1) ? NY : 1;
     static constexpr int P = NZ * (NY / JP);              // threads per cell
     // cells of a CTA (z-slabs of a brick): as many as leave the accumulators,
     // 8 JP NX values per thread, in registers.  FP64 B-splines: 32 cells; with 64
@@ -203,7 +205,7 @@ __device__ __forceinline__ void cell_terms_exact(const StepArgs<R> &a, const Pie
     constexpr bool AFF = KIND == CELL_P2G_AFF || KIND == CELL_MUSL_AFF;
     const Particles<R> &P = a.P;
     R wx[OX + 1], dx[OX + 1], wy, dy, wz, dz;
-    if (cx >= 2 && cx <= a.g.nel[0] - 3) {   // no wall piece: constants instead of 21 registers
+    if (OX == 2 && cx >= 2 && cx <= a.g.nel[0] - 3) {   // no wall piece: constants instead of 21 registers
         constexpr R c1[3] = {0.5, -1, 0.5}, c2[3] = {-3, 3, 0}, c3[3] = {4.5, -1.5, 0}, e1[3] = {1, -2, 1},
                     e2[3] = {-3, 3, 0};
 #pragma unroll
