@@ -7,8 +7,8 @@
 // a cell's contributions to some of its nodes in registers in particle order,
 // without atomics: P threads per cell, thread (j, k) owning the nodes of one
 // row (all i) of the cell's (OX+1)(OY+1)(OZ+1) nodes, or the rows of one
-// z-layer when the shape is linear.  The sums of the CTA's cells go to shared
-// memory once and a node pass adds the cells around each node in a fixed order
+// z-layer on FP64 linear grids.  A crowded brick is cut into shares (share_run in
+// mpm_sort.cu).  The sums of the CTA's cells go to shared memory once and a node pass adds the cells around each node in a fixed order
 // before one int64 fixed-point RED per node and field.  Deterministic: every
 // sum is in a fixed order.  The staging box it replaces spent its time in 64-bit
 // shared-memory atomics, one per particle, node and field.  P2G class per step,
@@ -24,7 +24,8 @@
 // of the B-splines took 47 us in place of 66, but the sums of 216 contributions are
 // far more exact than an FP32 number, and the stresses of a nearly uniform velocity
 // field moved by 5e-5; the implicit P2G's nodal mass, 64 particles per cell, was up to
-// 3.2 x 2^-24 off, and within 2 x 2^-24 with pairs.  int64 sums took 185 us, in the float to int64 conversions.)
+// 3.2 x 2^-24 off, and within 2 x 2^-24 with pairs.  int64 sums took 185 us, in the float
+// to int64 conversions.)
 // 32 cells per CTA and two CTAs per SM: 16, 64 or one CTA measured 78 to 95 us.
 // FP64 sums are kept in FP64.
 //
@@ -35,6 +36,7 @@
 // P2G, 292 FP64 instructions per particle), so a row's products are formed once,
 // a node costs 11 FMAs, and the in-cell test reads the high words of the offsets
 // in place of 6 FP64 comparisons (135 -> 128 us).
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <type_traits>
@@ -278,16 +280,24 @@ __global__ void __launch_bounds__(CellShape<R, OX, OY, OZ>::THREADS, CellShape<R
     const int kk = part % C::NZ, j0 = (part / C::NZ) * JP;
     const Particles<R> &Q = a.P;
     int misses = 0;
-    const int nitem = *a.nblist * C::SLABS;
+    const int nbl = *a.nblist, nitem = (nbl + *a.nshares) * C::SLABS;
     for (int it = blockIdx.x; it < nitem; it += gridDim.x) {
-        const int b = a.blist[it / C::SLABS], slab = it % C::SLABS;
+        // the bricks, then the further shares of the crowded ones
+        const int bi = it / C::SLABS, slab = it % C::SLABS;
+        const BrickShare bs = bi < nbl ? BrickShare{a.blist[bi], 0, a.bshares[bi]} : a.shares[bi - nbl];
+        const int b = bs.brick;
         const int *cs = a.cstart + (size_t)b * (BRC + 1) + slab * CELLS;
         if (cs[0] == cs[CELLS]) continue;   // an empty slab (uniform across the CTA)
         int ox, oy, oz;
         brick_origin(b, a.nbrick, ox, oy, oz);
         oz += slab * C::BZ;
         const int cx = ox + lc % BRX, cy = oy + (lc / BRX) % BRY, cz = oz + lc / (BRX * BRY);
-        const int p0 = cs[lc], p1 = cs[lc + 1];
+        int p0 = cs[lc], p1 = cs[lc + 1];
+        if (bs.count > 1) {   // this share's run of the cell's particles
+            const long long m = p1 - p0;
+            p1 = p0 + (int)(m * (bs.share + 1) / bs.count);
+            p0 += (int)(m * bs.share / bs.count);
+        }
         Sum acc[NG][JP][NX];
 #pragma unroll
         for (int f = 0; f < NG; f++)
@@ -640,8 +650,13 @@ static void scatter_kind(const StepArgs<R> &a, int nbricks, int nsm, bool pdl, c
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q, k, C::THREADS, C::SMEM) != cudaSuccess || q < 1) q = 1;
         per_sm = q;
     }
-    const long long items = (long long)nbricks * C::SLABS;
-    const int grid = (int)(items < (long long)per_sm * nsm ? items : (long long)per_sm * nsm);
+    // A CTA per brick's slab, as many as are resident.  Where the bricks leave room, more
+    // for the shares of crowded ones, but not to the last place: the CTAs of a grid
+    // that fills the chip are dealt out so that some SMs get two of the first ones
+    // (FP64 linear, 97,336 particles, 168 bricks: 85 us in place of 53).
+    const long long full = (long long)per_sm * nsm, bricks = (long long)nbricks * C::SLABS,
+                    shares = a.num / SHARE_RUN * C::SLABS;
+    const int grid = (int)(bricks >= full ? full : std::max(bricks, std::min(full - 8, bricks + shares)));
     launch(pdl, k, grid, C::THREADS, C::SMEM, st, a);
     launch(pdl, k_cell_misses<R, OX, OY, OZ, KIND>, 2 * nsm, 256, 0, st, a);
 }

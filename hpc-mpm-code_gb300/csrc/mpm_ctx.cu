@@ -70,10 +70,12 @@ static void free_particles(mpm_ctx *c) {
     free_dev(c->d_perm2);
     free_dev(c->d_stage);
     free_dev(c->d_work);
+    free_dev(c->d_shares);
     c->pbuf[0] = c->pbuf[1] = nullptr;
     c->d_key = c->d_perm = c->d_tmp = c->d_perm2 = nullptr;
     c->d_stage = nullptr;
     c->d_work = nullptr;
+    c->d_shares = nullptr;
     c->num = 0;
 }
 
@@ -189,6 +191,8 @@ mpm_status mpm_gpu_create(const mpm_grid_desc *grid, const mpm_material_desc *ma
     alloc((void **)&c->d_nwork, sizeof(int));
     alloc((void **)&c->d_blist, sizeof(int) * g.nbricks);
     alloc((void **)&c->d_nblist, sizeof(int));
+    alloc((void **)&c->d_bshares, sizeof(int) * g.nbricks);
+    alloc((void **)&c->d_nshares, sizeof(int));
     alloc((void **)&c->d_tlist, sizeof(int) * g.ntiles);
     alloc((void **)&c->d_ntlist, sizeof(int));
     alloc((void **)&c->d_ctl, sizeof(DevCtl));
@@ -224,6 +228,7 @@ mpm_status mpm_gpu_create(const mpm_grid_desc *grid, const mpm_material_desc *ma
     cudaMemset(c->d_cstart, 0, sizeof(int) * (size_t)g.nbricks * (BRC + 1));
     cudaMemset(c->d_nwork, 0, sizeof(int));
     cudaMemset(c->d_nblist, 0, sizeof(int));
+    cudaMemset(c->d_nshares, 0, sizeof(int));
     cudaMemset(c->d_ntlist, 0, sizeof(int));
     cudaMemset(c->d_ctl, 0, sizeof(DevCtl));
     memset(c->h_ctl, 0, sizeof(DevCtl));
@@ -269,6 +274,8 @@ void mpm_gpu_destroy(mpm_ctx *c) {
     free_dev(c->d_nwork);
     free_dev(c->d_blist);
     free_dev(c->d_nblist);
+    free_dev(c->d_bshares);
+    free_dev(c->d_nshares);
     free_dev(c->d_tlist);
     free_dev(c->d_ntlist);
     free_dev(c->d_ctl);
@@ -380,6 +387,7 @@ mpm_status mpm_gpu_load_particles(mpm_ctx *c, int64_t n, const double *coord, co
     CK(cudaMalloc((void **)&c->d_perm2, sizeof(int) * N));
     c->nwork_cap = c->g.nbricks + (int)(N / CHUNK) + 1;
     CK(cudaMalloc((void **)&c->d_work, sizeof(WorkItem) * c->nwork_cap));
+    CK(cudaMalloc((void **)&c->d_shares, sizeof(BrickShare) * (N / SHARE_RUN + 1)));
     c->cur = 0;
     mpm_status s = c->precision == 64 ? upload_particles<double>(c, n, coord, vel, mass, vol0, F, stress, matid)
                                       : upload_particles<float>(c, n, coord, vel, mass, vol0, F, stress, matid);

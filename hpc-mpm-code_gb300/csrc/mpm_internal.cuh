@@ -31,6 +31,7 @@ constexpr int TILE = 8;              // node tile edge for the grid passes and a
 constexpr int BRX = 4, BRY = 4, BRZ = 8;   // particle brick: cells per brick edge
 constexpr int BRC = BRX * BRY * BRZ;       // cells per brick (one CTA thread per cell)
 constexpr int CHUNK = 1024;          // max particles per work item
+constexpr int SHARE_RUN = 32;        // particles of a cell that one share of a brick's work takes, at least (BrickShare)
 constexpr int SCAN_SEG = 4096;       // bricks per segment of the brick-count scan (mpm_sort.cu)
 constexpr int NACC = 8;              // P2G fields: mass, vof, mome xyz, force xyz
 constexpr int NKCLASS = 14;          // kernel classes for timing
@@ -106,6 +107,12 @@ struct WorkItem {
     int end;
 };
 
+// Share `share` of the `count` that a crowded brick's work is cut into.  (Share 0
+// belongs to the brick's entry in the list of non-empty bricks.)
+struct BrickShare {
+    int brick;
+    int share, count;
+};
 
 // Launch variants.  The ones mpm_gpu_autotune chooses between from measured
 // times (staged or direct, resident CTAs per SM) give bitwise identical
@@ -190,12 +197,15 @@ struct mpm_ctx {
     int *d_key = nullptr, *d_perm = nullptr, *d_tcount = nullptr, *d_tstart = nullptr, *d_tcursor = nullptr;
     int *d_tmp = nullptr, *d_perm2 = nullptr;   // per-brick cell sort
     int *d_cstart = nullptr;                    // nbricks * (BRC + 1) cell start offsets
-    int *d_scanpart = nullptr;                  // per-segment sums of the brick-count scan (3 per segment + totals)
+    int *d_scanpart = nullptr;                  // per-segment sums of the brick-count scan (3 per segment)
     double *d_stage = nullptr;                  // FP64 AoS staging for host <-> device particle state
     mpm::WorkItem *d_work = nullptr;
     int *d_nwork = nullptr;
     int *d_blist = nullptr;       // bricks holding particles, in brick order (rebuilt by every sort)
     int *d_nblist = nullptr;
+    int *d_bshares = nullptr;     // shares of the bricks of d_blist
+    mpm::BrickShare *d_shares = nullptr;   // the further shares of crowded bricks, in any order
+    int *d_nshares = nullptr;
     int *d_tlist = nullptr;       // active node tiles of the current step (tile order)
     int *d_ntlist = nullptr;
     int nwork_cap = 0;

@@ -15,7 +15,7 @@
 //                 list of non-empty bricks: a scan over segments
 //   k_scatter     particles grouped by brick (order within a brick arbitrary)
 //   k_cell_sort   per brick: cell histogram and starts, then each particle's
-//                 rank inside its cell by load index
+//                 rank inside its cell by load index; a crowded brick's shares
 //   k_permute     the particle fields moved into the sorted order
 #include <algorithm>
 
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_up(int nb, const int *__restric
 
 __global__ void __launch_bounds__(SCAN_T) k_scan_down(int nb, int nseg, int *bcount, int *bstart, int *bcursor,
                                                       WorkItem *work, int *nwork, int cap, int *blist, int *nblist,
-                                                      const int *part, int *cstart) {
+                                                      int *nshares, const int *part, int *cstart) {
     __shared__ Tri sh[32];
     pdl_wait();
     const int base = blockIdx.x * SCAN_SEG;
@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_down(int nb, int nseg, int *bco
     if ((int)blockIdx.x == nseg - 1 && threadIdx.x == 0) {
         *nwork = min(carry.k, cap);
         *nblist = carry.a;
+        *nshares = 0;   // counted by k_cell_sort
         bstart[nb] = carry.c;
     }
 }
@@ -212,11 +213,13 @@ __global__ void k_scatter(const int *key, int n, const int *bstart, int *bcursor
 constexpr int CS_T = 256, CS_CAP = 4096;
 __global__ void __launch_bounds__(CS_T) k_cell_sort(const int *bstart, const int *key, const int *pid, const int *tmp,
                                                     int *tmp2, int *perm, int *cstart, const int *blist,
-                                                    const int *nblist) {
+                                                    const int *nblist, int run, int *bshares, BrickShare *shares,
+                                                    int *nshares) {
     static_assert(CS_T >= BRC && BRC % 32 == 0 && BRC <= 256, "cell scan layout");
     __shared__ int s_cnt[BRC];         // counts, then cursors
     __shared__ int s_start[BRC + 1];
-    __shared__ int s_w[BRC / 32];
+    __shared__ int s_w[BRC / 32], s_max[BRC / 32];
+    __shared__ int s_shares, s_base;
     __shared__ int s_pid[CS_CAP], s_idx[CS_CAP];
     __shared__ unsigned char s_cell[CS_CAP];
     pdl_wait();
@@ -238,7 +241,8 @@ __global__ void __launch_bounds__(CS_T) k_cell_sort(const int *bstart, const int
                 const int u = __shfl_up_sync(0xffffffffu, v, o);
                 if ((tid & 31) >= o) v += u;
             }
-            if ((tid & 31) == 31) s_w[tid >> 5] = v;
+            const int mx = __reduce_max_sync(0xffffffffu, s_cnt[tid]);
+            if ((tid & 31) == 31) s_w[tid >> 5] = v, s_max[tid >> 5] = mx;
         }
         __syncthreads();
         if (tid < BRC) {
@@ -251,8 +255,15 @@ __global__ void __launch_bounds__(CS_T) k_cell_sort(const int *bstart, const int
                 s_start[BRC] = v;
                 cs[BRC] = lo + v;
             }
+            if (tid == 0) {
+                int mx = s_max[0];
+                for (int w = 1; w < BRC / 32; w++) mx = max(mx, s_max[w]);
+                s_shares = bshares[it] = max(1, (mx + run / 2) / run);
+                if (s_shares > 1) s_base = atomicAdd(nshares, s_shares - 1) - 1;
+            }
         }
         __syncthreads();
+        for (int q = 1 + tid; q < s_shares; q += CS_T) shares[s_base + q] = BrickShare{b, q, s_shares};
         const bool fits = num <= CS_CAP;
         for (int j = tid; j < num; j += CS_T) {
             const int i = tmp[lo + j], c = key[i] % BRC, q = atomicAdd(&s_cnt[c], 1);
@@ -308,6 +319,24 @@ __global__ void k_permute(const R *__restrict__ src, R *__restrict__ dst, const 
     di[N + j] = a1;
 }
 
+// Particles of a cell that one share takes.  The scatters of mpm_cells.cu give a
+// cell to a few threads, which walk its particles one after another, and a brick to a
+// CTA per slab: crowded cells in fewer bricks than the chip holds CTAs leave it idle.
+// So a brick whose fullest cell holds 48 particles or more is cut into shares, each
+// with a run of every cell's particles.  Where the bricks fill the chip (two CTAs per
+// SM), only what is three times their average load is cut: another share costs
+// another node pass (cut in two all the same, 970,299 FP64 particles at 27 per cell
+// took 1563 us per step in place of 1380, 1,000,000 at 64 per cell with APIC 2963 in
+// place of 2739).  Step without and with shares, and with the staging box: FP64 linear,
+// 216,000 particles at 64 per cell 775, 489 and 1161 us, at 216 per cell 1800, 465 and
+// 1262; FP64 APIC, 27,000 at 216 per cell 1775, 366 and 950; FP32 quadratic, 216,000 at
+// 216 per cell 409, 247 and 2489; a 4^3-cell corner of 1,000,000 FP64 particles
+// squeezed to 216 per cell 2315, 1638 and 2789.
+static int share_run(int64_t n, int nsm) {
+    const int64_t avg = n / ((int64_t)2 * nsm * BRC);
+    return (int)std::max<int64_t>(SHARE_RUN, 3 * avg);
+}
+
 template <typename R>
 static mpm_status sort_impl(mpm_ctx *c) {
     int n = (int)c->num;
@@ -340,7 +369,8 @@ static mpm_status sort_impl(mpm_ctx *c) {
             c->launches++;
         }
         launch(pdl, k_scan_down, nseg, SCAN_T, 0, c->stream, c->g.nbricks, nseg, c->d_tcount, c->d_tstart, c->d_tcursor,
-               c->d_work, c->d_nwork, c->nwork_cap, c->d_blist, c->d_nblist, (const int *)c->d_scanpart, c->d_cstart);
+               c->d_work, c->d_nwork, c->nwork_cap, c->d_blist, c->d_nblist, c->d_nshares, (const int *)c->d_scanpart,
+               c->d_cstart);
     }
     timer_end(c, K_SCAN);
     timer_begin(c, K_SCATTER);
@@ -351,7 +381,7 @@ static mpm_status sort_impl(mpm_ctx *c) {
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     launch(pdl, k_cell_sort, std::min(c->g.nbricks, 6 * nsm), CS_T, 0, c->stream, (const int *)c->d_tstart,
            (const int *)c->d_key, pid, (const int *)c->d_tmp, c->d_perm2, c->d_perm, c->d_cstart,
-           (const int *)c->d_blist, (const int *)c->d_nblist);
+           (const int *)c->d_blist, (const int *)c->d_nblist, share_run(n, nsm), c->d_bshares, c->d_shares, c->d_nshares);
     timer_end(c, K_SCATTER);
     timer_begin(c, K_PERMUTE);
     // a Tait-fluid context keeps J - 1 in the first F field and never reads the other eight
