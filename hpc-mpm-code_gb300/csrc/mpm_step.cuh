@@ -326,17 +326,26 @@ __device__ __forceinline__ bool off_faces(double t) {
     return hi > 0x3E112E0Bu && hi < 0x3FEFFFFFu;       // 1e-9 and 1 - 2^-20
 }
 // cell_of without its FP64 division away from the cell faces (a guess from FP32
-// arithmetic, which the offset confirms); t the offset in that cell
+// arithmetic, which the offset confirms); t the offset in that cell, oob set where
+// x lies outside the grid (the cell is then the nearest one)
 template <typename R>
-__device__ __forceinline__ int fast_cell(R x, const KGeom<R> &g, int d, R &t) {
+__device__ __forceinline__ int fast_cell(R x, const KGeom<R> &g, int d, R &t, bool &oob) {
     int c = __float2int_rd((float)(x - g.xmin[d]) * (float)g.inv_dx[d]);
     t = cell_t(x, g, d, c);
     if ((unsigned)c >= (unsigned)g.nel[d] || !off_faces(t)) {
-        bool oob = false;
         c = cell_of(x, g, d, oob);
         t = cell_t(x, g, d, c);
     }
     return c;
+}
+// axis_eval's weights of a point outside the grid: the linear hats fall off beyond
+// their node (1 - |x - x_i| / dx), where those of CellAxis would go on rising
+template <typename R, int O>
+__device__ __forceinline__ void outside_weights(R x, const KGeom<R> &g, int d, int c, R *w, R *dw) {
+    Axis<R, O> a;
+    axis_eval<R, O>(x, g, d, c, a);
+#pragma unroll
+    for (int k = 0; k <= O; k++) w[k] = a.w[k], dw[k] = a.dw[k];
 }
 
 // sum_n N_n f_n (VAL) and sum_n dN_n/dx f_n (GRAD) of a nodal field over a cell's
@@ -379,10 +388,17 @@ __device__ __forceinline__ void cell_field(const R *f, size_t b0, size_t sy, siz
 template <typename R, int OX, int OY, int OZ>
 __device__ __forceinline__ size_t cell_weights(const KGeom<R> &g, const R *x, CellWeights<R, OX, OY, OZ> &w) {
     R t0, t1, t2;
-    const int cx = fast_cell(x[0], g, 0, t0), cy = fast_cell(x[1], g, 1, t1), cz = fast_cell(x[2], g, 2, t2);
+    bool oob = false;
+    const int cx = fast_cell(x[0], g, 0, t0, oob), cy = fast_cell(x[1], g, 1, t1, oob),
+              cz = fast_cell(x[2], g, 2, t2, oob);
     CellAxis<R, OX>(cx, g.nel[0], g.inv_dx[0]).eval(t0, w.wx, w.dx);
     CellAxis<R, OY>(cy, g.nel[1], g.inv_dx[1]).eval(t1, w.wy, w.dy);
     CellAxis<R, OZ>(cz, g.nel[2], g.inv_dx[2]).eval(t2, w.wz, w.dz);
+    if (oob) {   // the weights of its P2G (k_cell_misses)
+        outside_weights<R, OX>(x[0], g, 0, cx, w.wx, w.dx);
+        outside_weights<R, OY>(x[1], g, 1, cy, w.wy, w.dy);
+        outside_weights<R, OZ>(x[2], g, 2, cz, w.wz, w.dz);
+    }
     return node_id(g, cx, cy, cz);
 }
 
