@@ -79,7 +79,7 @@ struct ImpState {
     double *gqq = nullptr, *gbeta = nullptr;  // |A p|^2 of each kept direction, projection coefficients
     float *gqf = nullptr;                   // FP32 copies of the kept images (GM * 3 * nodec), for the dots
     size_t gst = 0;                         // values per direction slot: 3 * nodec, up to a multiple of four
-    int64_t gcr_launches = 0;               // launches in g_gcr
+    int64_t cg_launches = 0, gcr_launches = 0;   // launches in g_cg and g_gcr
     float *gp32 = nullptr, *gq32 = nullptr;  // FP32 operator: the directions and images in FP32 (GM * 3 * nodec)
     float *p32 = nullptr;                   // FP32 operator: the CG direction in FP32
     float *nf32 = nullptr;                  // FP32 copies of ndispl, nvel, naccel (3 N each) and nei (N) for the particles
@@ -2329,11 +2329,12 @@ static mpm_status imp_cg(mpm_ctx *c, double eps, int kmax, int *iters) {
             const int64_t l0 = c->launches;
             if (!s->g_cg && capture_iters(c, &s->g_cg, [&] {
                     for (int k = 0; k < KCHECK; k++) cg_iteration(c, a, nb, k, 1);
+                    s->cg_launches = c->launches - l0;
                 }) != MPM_OK)
                 s->no_graph = true;
             if (s->g_cg) {
                 CKI(cudaGraphLaunch(s->g_cg, c->stream));
-                if (c->launches == l0) c->launches += 3 * KCHECK;   // the capture counted the first block
+                if (c->launches == l0) c->launches += s->cg_launches;   // the capture counted the first block
                 ran = true;
             }
         }
