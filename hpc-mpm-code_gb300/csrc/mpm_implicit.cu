@@ -2113,7 +2113,9 @@ static void launch_split(mpm_ctx *c, const ImpArgs &a, const TV *x, TY *y, const
     const int *o = c->g.order;
     const unsigned nb = (unsigned)((c->g.nodec + MV_NODES - 1) / MV_NODES);
     const TA *A = (const TA *)c->imp->A;
-    auto go = [&](auto k) { launch(true, k, nb, MV_NODES * MV_G, 0, c->stream, a, A, x, y, xd, part, cnt, scal, slot, num, done); };
+    auto go = [&](auto k) {
+        launch(c->pdl != 0, k, nb, MV_NODES * MV_G, 0, c->stream, a, A, x, y, xd, part, cnt, scal, slot, num, done);
+    };
     if (o[0] == 1 && o[1] == 1 && o[2] == 1) go(k_imp_matvec_split<TA, TC, 1, 1, 1, TV, TY>);
     else if (o[1] == 2) go(k_imp_matvec_split<TA, TC, 2, 2, 2, TV, TY>);
     else go(k_imp_matvec_split<TA, TC, 2, 1, 2, TV, TY>);
@@ -2139,7 +2141,7 @@ static void launch_matvec_cg(mpm_ctx *c, const ImpArgs &a, int nb, int cur, cons
         launch_split<float, float>(c, a, (const float *)s->p32, s->Ap, s->p, part, s->cnt + 3, s->scal, S_PAP, cur, done);
     if (!dot) {
         const int m = 3 * c->g.nodec;
-        launch(true, k_cg_dot, (m + 1023) / 1024, 256, 0, c->stream, (const double *)s->p, (const double *)s->Ap, m,
+        launch(c->pdl != 0, k_cg_dot, (m + 1023) / 1024, 256, 0, c->stream, (const double *)s->p, (const double *)s->Ap, m,
                s->part, s->cnt + 3, s->scal, cur, done);
         c->launches++;
     }
@@ -2293,9 +2295,9 @@ static void cg_iteration(mpm_ctx *c, const ImpArgs &a, int nb, int it, int stop)
     launch_matvec_cg(c, a, nb, cur, stop ? s->scal + S_DONE : nullptr);
     timer_end(c, K_MATVEC);
     timer_begin(c, K_KRYLOV);
-    launch(true, k_cg_update, nb, 256, 0, c->stream, a, s->scal, cur, s->xs, s->r, (const double *)s->p,
+    launch(c->pdl != 0, k_cg_update, nb, 256, 0, c->stream, a, s->scal, cur, s->xs, s->r, (const double *)s->p,
            (const double *)s->Ap, s->part, s->cnt + 4, stop);
-    launch(true, k_cg_dir, nb, 256, 0, c->stream, a, (const double *)s->scal, (const double *)s->r, s->p, s->p32, stop);
+    launch(c->pdl != 0, k_cg_dir, nb, 256, 0, c->stream, a, (const double *)s->scal, (const double *)s->r, s->p, s->p32, stop);
     timer_end(c, K_KRYLOV);
     c->launches += 3;
 }
@@ -2391,7 +2393,7 @@ static mpm_status gcr_iter(mpm_ctx *c, const ImpArgs &a, int nb, int u, int sl, 
     ImpState *s = c->imp;
     const size_t st = s->gst;
     const int m = 3 * c->g.nodec, nq = (m + 1023) / 1024;
-    const bool pdl = !c->timer.on;
+    const bool pdl = c->pdl != 0 && !c->timer.on;
     auto dots = [&](auto k, auto *Q, const float *Qf) {
         launch(pdl, k, nq, 256, 0, c->stream, Q, Qf, st, m, sl, u, s->gm, s->part, s->cnt, (const double *)s->gqq,
                s->gbeta);

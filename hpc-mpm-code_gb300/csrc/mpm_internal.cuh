@@ -19,6 +19,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <stdlib.h>
 
 #include <string>
 #include <vector>
@@ -100,6 +101,13 @@ struct Particles {
     R *Fb[9], *Jb, *Jt;   // F-bar contexts: def_grad_bar, det_def_grad_bar, trial J of the step (FP32: all minus I / 1)
     int *matid, *pid;
 };
+
+// Whether a new context launches its kernels with programmatic dependent launch
+// (MPM_GB300_PDL=0: off).
+inline int pdl_switch() {
+    const char *v = getenv("MPM_GB300_PDL");
+    return v ? atoi(v) != 0 : 1;
+}
 
 struct WorkItem {
     int tile;
@@ -222,7 +230,7 @@ struct mpm_ctx {
     bool write_nodal_dl = false;
     int cell_scatter = 1;   // per-cell register scatter (0: staging-box atomics)
     int tma_update = 1;     // FP32 linear: particle update with bulk-copy staged input
-    int pdl = 1;            // step kernels launched with programmatic dependent launch (MPM_GB300_PDL=0: off)
+    int pdl = mpm::pdl_switch();   // kernels launched with programmatic dependent launch
     int alternate = 1;      // particle kernels walk bricks / chunks in alternating directions (MPM_GB300_ALTERNATE=0: forward)
     mpm_status latched = MPM_OK;
     mpm::KernelTimer timer;

@@ -891,6 +891,7 @@ struct mpm_ns {
     cudaGraphExec_t graph = nullptr;   // NS_BLOCK GPBiCGSafe iterations (ns_graph)
     double graph_eps = 0.0;
     bool no_graph = false;
+    int pdl = pdl_switch();
     std::vector<int> bc_nodes[4];
     std::vector<double> bc_vals[4];
     // time step (mpm_ns_step): nodal state, P2G sums and bounds, particle scratch
@@ -1010,10 +1011,10 @@ extern "C" mpm_status mpm_ns_set_bc(mpm_ns *s, int comp, int n, const int *nodes
 static void ns_matvec(const mpm_ns *s, const double *x, double *y, const double *done, cudaStream_t st) {
     const unsigned nb = (unsigned)((s->nodec + NSV_NODES - 1) / NSV_NODES);
     if (s->nodec <= 32768)
-        launch(true, k_nsv_matvec<9>, nb, 9 * NSV_NODES, 0, st, s->a.g, (const double *)s->A,
+        launch(s->pdl != 0, k_nsv_matvec<9>, nb, 9 * NSV_NODES, 0, st, s->a.g, (const double *)s->A,
                (const unsigned char *)s->bcf, x, y, done);
     else
-        launch(true, k_nsv_matvec<3>, nb, 3 * NSV_NODES, 0, st, s->a.g, (const double *)s->A,
+        launch(s->pdl != 0, k_nsv_matvec<3>, nb, 3 * NSV_NODES, 0, st, s->a.g, (const double *)s->A,
                (const unsigned char *)s->bcf, x, y, done);
 }
 
@@ -1048,10 +1049,10 @@ static void ns_iteration(const mpm_ns *s, double eps, cudaStream_t st) {
     const int n = s->nodec, nb = (n + NSV_T - 1) / NSV_T;
     const double *done = s->scal + NS_DONE;
     ns_matvec(s, s->v.rr, s->v.Ar, done, st);
-    launch(true, k_gpb_1, nb, NSV_T, 0, st, n, s->v, s->part, s->cnt + 1, s->scal);
-    launch(true, k_gpb_2, (4 * n + 255) / 256, 256, 0, st, 4 * n, s->v, (const double *)s->scal);
+    launch(s->pdl != 0, k_gpb_1, nb, NSV_T, 0, st, n, s->v, s->part, s->cnt + 1, s->scal);
+    launch(s->pdl != 0, k_gpb_2, (4 * n + 255) / 256, 256, 0, st, 4 * n, s->v, (const double *)s->scal);
     ns_matvec(s, s->v.uu, s->v.Au, done, st);
-    launch(true, k_gpb_3, nb, NSV_T, 0, st, n, s->v, eps, s->part, s->cnt + 2, s->scal);
+    launch(s->pdl != 0, k_gpb_3, nb, NSV_T, 0, st, n, s->v, eps, s->part, s->cnt + 2, s->scal);
 }
 
 // The graph of NS_BLOCK iterations with stopping test eps, captured on a stream
