@@ -8,9 +8,10 @@
 // without atomics: P threads per cell, thread (j, k) owning the nodes of one
 // row (all i) of the cell's (OX+1)(OY+1)(OZ+1) nodes, or the rows of one
 // z-layer on FP64 linear grids.  A crowded brick is cut into shares (share_run in
-// mpm_sort.cu).  The sums of the CTA's cells go to shared memory once and a node pass adds the cells around each node in a fixed order
-// before one int64 fixed-point RED per node and field.  Deterministic: every
-// sum is in a fixed order.  The staging box it replaces spent its time in 64-bit
+// mpm_sort.cu).  The sums of the CTA's cells go to shared memory once and a node
+// pass adds the cells around each node in a fixed order before one int64
+// fixed-point RED per node and field.  Deterministic: every sum is in a fixed order,
+// or of integers.  The staging box it replaces spent its time in 64-bit
 // shared-memory atomics, one per particle, node and field.  P2G class per step,
 // staging box -> here: FP64 linear, 201,872 particles, 296 -> 128 us; FP32
 // B-splines, 216,000 particles, 444 -> 66 us; FP64 B-splines, 46,656 particles,

@@ -2048,7 +2048,6 @@ __global__ void __launch_bounds__(256) k_affine_musl(StepArgs<R> a) {
 }
 
 // ------------------------------------------------------------ grid pass 1
-constexpr int TILE_DIRECT = 608;                             // tiles up to which no list is made
 constexpr int GRID_THREADS = 256;                            // threads of a grid-pass CTA
 constexpr int GRID_NPT = TILE * TILE * TILE / GRID_THREADS;  // nodes of a tile per thread
 static_assert(GRID_NPT * GRID_THREADS == TILE * TILE * TILE, "a grid-pass CTA covers its tile exactly");
@@ -2057,7 +2056,8 @@ static_assert(GRID_NPT * GRID_THREADS == TILE * TILE * TILE, "a grid-pass CTA co
 // last CTA added the partials of all and derived the gather's scales (now in k_grid2
 // and musl_scales), a reduction per tile, and eight 64-bit conversions per node on the
 // FP64 pipe (ll2f takes the integer pipes; 59 % of the FP64 pipe was busy).  With the
-// tile list: 8,000 particles 12.7 -> 9.7 us, 4,096,000 35.7 -> 26.4, 64 scenes 55.7 -> 44.4.
+// tile list on both sides, its launch included: 8,000 particles 12.7 -> 9.7 us, 4,096,000
+// 35.7 -> 26.4, 64 scenes 55.7 -> 44.4.  (8,000 particles have few tiles and no list.)
 template <typename R, bool LIST>
 __global__ void __launch_bounds__(GRID_THREADS) k_grid1(StepArgs<R> a) {
     pdl_wait();
@@ -3263,8 +3263,13 @@ static bool begins_itself(const mpm_ctx *c) {
 // The grid passes walk a list of the active tiles, which takes a launch to make;
 // a grid whose tiles' CTAs are resident together (4 per SM) launches one CTA per
 // tile instead, which asks its tile's flag: 17 -> 13 us for both at 27 tiles, 24
-// -> 20 at 576, but 34 -> 54 us at 4,913 (spinning block, 128^3 cells).
-static bool use_tile_list(const mpm_ctx *c) { return !c->write_nodal_dl && c->g.ntiles > TILE_DIRECT; }
+// -> 20 at 576, but 34 -> 54 us at 4,913 (spinning block, 128^3 cells).  A step with the
+// list and without it, 512 tiles: PIC 29.8 and 26.9 us at 8,000 particles, 107.9 and 105.1
+// at 1,000,000; APIC 38.1 and 35.2; quadratic B-splines 51.2 and 48.5; FP32 F-bar 38.4 and
+// 36.0; FP64 129.5 and 126.7.  FP64 F-bar alone loses, 175.8 and 183.4, to a k_fbar_grid
+// that divides at the nodes of every tile.  729 tiles: PIC 29.9 and 27.9, FP64 at 64,000
+// particles 164.5 and 171.6.
+static bool use_tile_list(const mpm_ctx *c) { return !c->write_nodal_dl && c->g.ntiles > 4 * num_sms(); }
 
 // which: 0 P2G, 1 G2P + MUSL, 2 G2P update
 template <typename R, int OX, int OY, int OZ>

@@ -617,7 +617,10 @@ __global__ void __launch_bounds__(128) k_imp_assemble(ImpArgs a, PView<R> P, con
 // SM held to 168 registers, beat 32 cells in one CTA (592 to 741 us) and two or
 // four threads per row node (790 to 1018).  The class with scaling and RHS, per
 // Newton iteration: 1,728,000 particles 2217 -> 592 us, 232,320 372 -> 150, quadratic
-// B-splines (87,808) 870 -> 439.
+// B-splines (87,808) 870 -> 439.  A round's particles are neighbours in the sorted
+// order, so crowded cells take turns: at 216 particles per linear cell the class takes
+// 1060 us for 216,000 particles, as the atomics do, and 813 in place of 248 for 27,000
+// (a whole step of theirs still 2.5 ms in place of 3.6).
 // A particle outside its sorted cell scatters with atomics of its own.
 template <int OX, int OY, int OZ>
 struct AsmShape {
@@ -896,13 +899,6 @@ __device__ __forceinline__ double last_sums(const double *part, int nv) {
     if ((int)threadIdx.x < nv)
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += sh[threadIdx.x][w];
     return s;
-}
-
-// in the last block: the total of value j over all blocks (thread 0)
-__device__ __forceinline__ double last_sum(const double *part, int j, double *sh32) {
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) acc += __ldcg(part + (size_t)j * gridDim.x + i);
-    return block_sum(acc, sh32);
 }
 
 __global__ void k_finish(const double *part, int nblk, double *out, int slot) {
@@ -2259,9 +2255,9 @@ static mpm_status imp_p2g(mpm_ctx *c, double facl) {
 // guess (physical) and receives the physical solution.  Returns iterations.
 static constexpr int KCHECK = 8;   // Krylov iterations between residual checks (and per graph)
 // Within this factor of the tolerance (squared norms, 100x in the norm) the
-// solvers leave the 8-iteration graphs and check after every iteration, so
-// that a solve stops at the iteration that reaches the tolerance instead of
-// at the end of the next block of 8.
+// flexible GCR leaves the 8-iteration graphs and checks after every iteration, so
+// that a solve stops at the iteration that reaches the tolerance instead of at
+// the end of the next block of 8.  (CG stops itself on the device.)
 static constexpr double FINE_FACTOR = 1.0e4;
 
 static bool graphs_on(mpm_ctx *c) { return c->use_graph && c->stream != nullptr && !c->timer.on && !c->imp->no_graph; }

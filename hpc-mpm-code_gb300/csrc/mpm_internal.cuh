@@ -88,7 +88,7 @@ struct DevCtl {
     unsigned int err_timeout;        // bounded device waits that gave up
     unsigned int n_miss_p2g;         // particles queued for the deferred P2G pass this step
     unsigned int n_miss_musl;        // particles queued for the deferred gather/MUSL pass this step
-    Scales sc_p2g;                   // this step's P2G scales (k_step_reset)
+    Scales sc_p2g;                   // this step's P2G scales (p2g_scales, or k_step_reset)
     Scales sc_musl;                  // this step's gather/MUSL scales (musl_scales)
     Fix sc_fbar;                     // F-bar: scale of the projected J vol sums (fbar_scale)
 };

@@ -1007,7 +1007,9 @@ extern "C" mpm_status mpm_ns_set_bc(mpm_ns *s, int comp, int n, const int *nodes
 // chip with one warp per 32 of them: nine threads share a node up to 32,768
 // nodes (8,925 nodes: 50 us per GPBiCGSafe iteration against 62 with three and
 // 115 with one); on larger grids three do, which add six FP64 numbers per row
-// less (198,000 nodes: 441 against 481 and 572 us).
+// less (198,000 nodes: 441 against 481 and 572 us).  Whole steps with nine and with
+// three, whose iteration counts differ by a few per cent: 3,315 nodes 4.1 and 5.4 ms,
+// 19,251 11.2 and 11.2, 31,465 21.4 and 23.4, 44,485 30.0 and 29.1, 71,299 50.1 and 46.8.
 static void ns_matvec(const mpm_ns *s, const double *x, double *y, const double *done, cudaStream_t st) {
     const unsigned nb = (unsigned)((s->nodec + NSV_NODES - 1) / NSV_NODES);
     if (s->nodec <= 32768)
