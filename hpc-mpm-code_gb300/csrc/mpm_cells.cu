@@ -281,12 +281,10 @@ __global__ void __launch_bounds__(CellShape<R, OX, OY, OZ>::THREADS, CellShape<R
     const int kk = part % C::NZ, j0 = (part / C::NZ) * JP;
     const Particles<R> &Q = a.P;
     int misses = 0;
-    const int nbl = *a.nblist, nitem = (nbl + *a.nshares) * C::SLABS;
+    const int nitem = *a.nshares * C::SLABS;
     for (int it = blockIdx.x; it < nitem; it += gridDim.x) {
-        // the bricks, then the further shares of the crowded ones
-        const int bi = it / C::SLABS, slab = it % C::SLABS;
-        const BrickShare bs = bi < nbl ? BrickShare{a.blist[bi], 0, a.bshares[bi]} : a.shares[bi - nbl];
-        const int b = bs.brick;
+        const BrickShare bs = a.shares[it / C::SLABS];
+        const int b = bs.brick, slab = it % C::SLABS;
         const int *cs = a.cstart + (size_t)b * (BRC + 1) + slab * CELLS;
         if (cs[0] == cs[CELLS]) continue;   // an empty slab (uniform across the CTA)
         int ox, oy, oz;
@@ -295,9 +293,9 @@ __global__ void __launch_bounds__(CellShape<R, OX, OY, OZ>::THREADS, CellShape<R
         const int cx = ox + lc % BRX, cy = oy + (lc / BRX) % BRY, cz = oz + lc / (BRX * BRY);
         int p0 = cs[lc], p1 = cs[lc + 1];
         if (bs.count > 1) {   // this share's run of the cell's particles
-            const long long m = p1 - p0;
-            p1 = p0 + (int)(m * (bs.share + 1) / bs.count);
-            p0 += (int)(m * bs.share / bs.count);
+            const int run = (p1 - p0 + bs.count - 1) / bs.count;
+            p0 = min(p1, p0 + bs.share * run);
+            p1 = min(p1, p0 + run);
         }
         Sum acc[NG][JP][NX];
 #pragma unroll

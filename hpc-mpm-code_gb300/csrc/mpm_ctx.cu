@@ -190,7 +190,6 @@ mpm_status mpm_gpu_create(const mpm_grid_desc *grid, const mpm_material_desc *ma
     alloc((void **)&c->d_nwork, sizeof(int));
     alloc((void **)&c->d_blist, sizeof(int) * g.nbricks);
     alloc((void **)&c->d_nblist, sizeof(int));
-    alloc((void **)&c->d_bshares, sizeof(int) * g.nbricks);
     alloc((void **)&c->d_nshares, sizeof(int));
     alloc((void **)&c->d_tlist, sizeof(int) * g.ntiles);
     alloc((void **)&c->d_ntlist, sizeof(int));
@@ -273,7 +272,6 @@ void mpm_gpu_destroy(mpm_ctx *c) {
     free_dev(c->d_nwork);
     free_dev(c->d_blist);
     free_dev(c->d_nblist);
-    free_dev(c->d_bshares);
     free_dev(c->d_nshares);
     free_dev(c->d_tlist);
     free_dev(c->d_ntlist);
@@ -386,7 +384,7 @@ mpm_status mpm_gpu_load_particles(mpm_ctx *c, int64_t n, const double *coord, co
     CK(cudaMalloc((void **)&c->d_perm2, sizeof(int) * N));
     c->nwork_cap = c->g.nbricks + (int)(N / CHUNK) + 1;
     CK(cudaMalloc((void **)&c->d_work, sizeof(WorkItem) * c->nwork_cap));
-    CK(cudaMalloc((void **)&c->d_shares, sizeof(BrickShare) * (N / SHARE_RUN + 1)));
+    CK(cudaMalloc((void **)&c->d_shares, sizeof(BrickShare) * (c->g.nbricks + N / SHARE_RUN + 1)));
     c->cur = 0;
     mpm_status s = c->precision == 64 ? upload_particles<double>(c, n, coord, vel, mass, vol0, F, stress, matid)
                                       : upload_particles<float>(c, n, coord, vel, mass, vol0, F, stress, matid);

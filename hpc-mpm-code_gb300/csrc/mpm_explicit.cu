@@ -3176,7 +3176,6 @@ static StepArgs<R> make_args(mpm_ctx *c) {
     a.miss = c->d_tmp;
     a.blist = c->d_blist;
     a.nblist = c->d_nblist;
-    a.bshares = c->d_bshares;
     a.shares = c->d_shares;
     a.nshares = c->d_nshares;
     a.tlist = c->d_tlist;

@@ -115,9 +115,8 @@ struct WorkItem {
     int end;
 };
 
-// Share `share` of the `count` that a crowded brick's work is cut into.  (Share 0
-// belongs to the brick's entry in the list of non-empty bricks.)
-struct BrickShare {
+// Share `share` of the `count` that a brick's work is cut into (1 unless it is crowded).
+struct alignas(16) BrickShare {
     int brick;
     int share, count;
 };
@@ -211,8 +210,7 @@ struct mpm_ctx {
     int *d_nwork = nullptr;
     int *d_blist = nullptr;       // bricks holding particles, in brick order (rebuilt by every sort)
     int *d_nblist = nullptr;
-    int *d_bshares = nullptr;     // shares of the bricks of d_blist
-    mpm::BrickShare *d_shares = nullptr;   // the further shares of crowded bricks, in any order
+    mpm::BrickShare *d_shares = nullptr;   // the bricks of d_blist, then the further shares of crowded ones in any order
     int *d_nshares = nullptr;
     int *d_tlist = nullptr;       // active node tiles of the current step (tile order)
     int *d_ntlist = nullptr;

@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_down(int nb, int nseg, int *bco
     if ((int)blockIdx.x == nseg - 1 && threadIdx.x == 0) {
         *nwork = min(carry.k, cap);
         *nblist = carry.a;
-        *nshares = 0;   // counted by k_cell_sort
+        *nshares = carry.a;   // k_cell_sort adds to it
         bstart[nb] = carry.c;
     }
 }
@@ -213,7 +213,7 @@ __global__ void k_scatter(const int *key, int n, const int *bstart, int *bcursor
 constexpr int CS_T = 256, CS_CAP = 4096;
 __global__ void __launch_bounds__(CS_T) k_cell_sort(const int *bstart, const int *key, const int *pid, const int *tmp,
                                                     int *tmp2, int *perm, int *cstart, const int *blist,
-                                                    const int *nblist, int run, int *bshares, BrickShare *shares,
+                                                    const int *nblist, int run, BrickShare *shares,
                                                     int *nshares) {
     static_assert(CS_T >= BRC && BRC % 32 == 0 && BRC <= 256, "cell scan layout");
     __shared__ int s_cnt[BRC];         // counts, then cursors
@@ -258,7 +258,8 @@ __global__ void __launch_bounds__(CS_T) k_cell_sort(const int *bstart, const int
             if (tid == 0) {
                 int mx = s_max[0];
                 for (int w = 1; w < BRC / 32; w++) mx = max(mx, s_max[w]);
-                s_shares = bshares[it] = max(1, (mx + run / 2) / run);
+                s_shares = max(1, (mx + run / 2) / run);
+                shares[it] = BrickShare{b, 0, s_shares};
                 if (s_shares > 1) s_base = atomicAdd(nshares, s_shares - 1) - 1;
             }
         }
@@ -381,7 +382,8 @@ static mpm_status sort_impl(mpm_ctx *c) {
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     launch(pdl, k_cell_sort, std::min(c->g.nbricks, 6 * nsm), CS_T, 0, c->stream, (const int *)c->d_tstart,
            (const int *)c->d_key, pid, (const int *)c->d_tmp, c->d_perm2, c->d_perm, c->d_cstart,
-           (const int *)c->d_blist, (const int *)c->d_nblist, share_run(n, nsm), c->d_bshares, c->d_shares, c->d_nshares);
+           (const int *)c->d_blist, (const int *)c->d_nblist, share_run(n, nsm), c->d_shares,
+           c->d_nshares);
     timer_end(c, K_SCATTER);
     timer_begin(c, K_PERMUTE);
     // a Tait-fluid context keeps J - 1 in the first F field and never reads the other eight

@@ -17,8 +17,7 @@ struct StepArgs {
     int *miss;                  // particles that left their sorted cell, processed by a deferred pass
     const int *blist;           // bricks holding particles (brick order) and their count
     const int *nblist;
-    const int *bshares;         // shares of the bricks in blist
-    const BrickShare *shares;   // the further shares of crowded bricks and their count
+    const BrickShare *shares;   // the same bricks and the further shares of crowded ones, and their count
     const int *nshares;
     const int *tlist;           // active node tiles of this step (tile order) and their count
     const int *ntlist;
