@@ -2097,7 +2097,7 @@ static void launch_matvec(mpm_ctx *c, const ImpArgs &a, int nb, const double *x,
 // eight times as many CTAs as a pass over vectors has, and on a large grid their
 // partials cost more than a pass of its own over p and Ap: per product, with its own dot
 // against a separate one, 18.8 against 17.1 us (FP32) and 38.1 against 35.3 (FP64) at
-// 46,305 points, 86 against 63.4 (FP32) at 274,625; but 10.9 against 12.6 at 1,690 and
+// 46,305 points, 86 against 59 to 63 (FP32) at 274,625; but 10.9 against 12.6 at 1,690 and
 // 18.8 against 19.6 at 24,000 (B-spline stencil).
 // (One thread per point: 19.6 us FP32 at 1,690 points, 22.1 at 46,305, 65 at
 // 274,625; FP64 50.8 and 153 where the split takes 35.3 and 143.)
