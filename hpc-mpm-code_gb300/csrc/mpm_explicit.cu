@@ -2413,8 +2413,9 @@ __global__ void __launch_bounds__(256) k_fbar_trial(StepArgs<R> a) {
 }
 
 // The fixed-point scale of the projected J vol sums, from the bound k_fbar_trial
-// recorded: by every CTA for itself (the caller's next barrier publishes it), and
-// by CTA 0 for k_fbar_grid.
+// recorded: by every CTA with work for itself (the caller's next barrier publishes it;
+// in every CTA of a mostly empty grid it cost 14 of 107 us per step: 8,000 particles in
+// 200^3 cells), and by CTA 0 for k_fbar_grid.
 template <typename R>
 __device__ __forceinline__ void fbar_scale(const StepArgs<R> &a, Fix &F) {
     if (threadIdx.x != 0) return;
@@ -2461,11 +2462,12 @@ __global__ void __launch_bounds__(CELL_THREADS, 3) k_fbar_scatter_cell(StepArgs<
     __shared__ float corner[8][BRC];
     __shared__ Fix F;
     pdl_wait();
-    fbar_scale(a, F);   // before an empty brick leaves: CTA 0 records it
+    if (blockIdx.x == 0) fbar_scale(a, F);   // CTA 0 records it, also where its brick is empty
     const int b = blockIdx.x;
     const int lc = threadIdx.x >> 1, h = threadIdx.x & 1;
     const int *cs = a.cstart + (size_t)b * (BRC + 1);
     if (cs[0] == cs[BRC]) return;   // empty brick (uniform across the CTA)
+    if (blockIdx.x != 0) fbar_scale(a, F);
     int ox, oy, oz;
     brick_origin(b, a.nbrick, ox, oy, oz);
     const int cx = ox + (lc % BRX), cy = oy + (lc / BRX) % BRY, cz = oz + lc / (BRX * BRY);
