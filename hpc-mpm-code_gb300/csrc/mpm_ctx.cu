@@ -371,6 +371,7 @@ mpm_status mpm_gpu_load_particles(mpm_ctx *c, int64_t n, const double *coord, co
                                   const double *vol0, const double *F, const double *stress, const int *matid) {
     if (!c || n < 0 || n > (1LL << 30) || (n > 0 && (!coord || !mass || !vol0))) return MPM_ERR_BAD_ARG;
     CK(cudaStreamSynchronize(c->stream));
+    drop_graph(c);   // it holds the old particles' buffers, count and largest mass
     free_particles(c);
     c->num = n;
     size_t N = (size_t)(n > 0 ? n : 1);
