@@ -241,8 +241,11 @@ __global__ void __launch_bounds__(CS_T) k_cell_sort(const int *bstart, const int
                 const int u = __shfl_up_sync(0xffffffffu, v, o);
                 if ((tid & 31) >= o) v += u;
             }
-            const int mx = __reduce_max_sync(0xffffffffu, s_cnt[tid]);
-            if ((tid & 31) == 31) s_w[tid >> 5] = v, s_max[tid >> 5] = mx;
+            if ((tid & 31) == 31) s_w[tid >> 5] = v;
+            if (run > 0) {
+                const int mx = __reduce_max_sync(0xffffffffu, s_cnt[tid]);
+                if ((tid & 31) == 31) s_max[tid >> 5] = mx;
+            }
         }
         __syncthreads();
         if (tid < BRC) {
@@ -255,7 +258,7 @@ __global__ void __launch_bounds__(CS_T) k_cell_sort(const int *bstart, const int
                 s_start[BRC] = v;
                 cs[BRC] = lo + v;
             }
-            if (tid == 0) {
+            if (run > 0 && tid == 0) {
                 int mx = s_max[0];
                 for (int w = 1; w < BRC / 32; w++) mx = max(mx, s_max[w]);
                 s_shares = max(1, (mx + run / 2) / run);
@@ -264,7 +267,8 @@ __global__ void __launch_bounds__(CS_T) k_cell_sort(const int *bstart, const int
             }
         }
         __syncthreads();
-        for (int q = 1 + tid; q < s_shares; q += CS_T) shares[s_base + q] = BrickShare{b, q, s_shares};
+        if (run > 0)
+            for (int q = 1 + tid; q < s_shares; q += CS_T) shares[s_base + q] = BrickShare{b, q, s_shares};
         const bool fits = num <= CS_CAP;
         for (int j = tid; j < num; j += CS_T) {
             const int i = tmp[lo + j], c = key[i] % BRC, q = atomicAdd(&s_cnt[c], 1);
@@ -338,6 +342,11 @@ static int share_run(int64_t n, int nsm) {
     return (int)std::max<int64_t>(SHARE_RUN, 3 * avg);
 }
 
+// FP32 linear explicit grids have kernels of their own, which take whole bricks.
+static bool lists_shares(const mpm_ctx *c) {
+    return c->cell_scatter && !(c->precision == 32 && c->g.order[0] == 1 && c->nreal != 27);
+}
+
 template <typename R>
 static mpm_status sort_impl(mpm_ctx *c) {
     int n = (int)c->num;
@@ -382,8 +391,8 @@ static mpm_status sort_impl(mpm_ctx *c) {
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     launch(pdl, k_cell_sort, std::min(c->g.nbricks, 6 * nsm), CS_T, 0, c->stream, (const int *)c->d_tstart,
            (const int *)c->d_key, pid, (const int *)c->d_tmp, c->d_perm2, c->d_perm, c->d_cstart,
-           (const int *)c->d_blist, (const int *)c->d_nblist, share_run(n, nsm), c->d_shares,
-           c->d_nshares);
+           (const int *)c->d_blist, (const int *)c->d_nblist, lists_shares(c) ? share_run(n, nsm) : 0,
+           c->d_shares, c->d_nshares);
     timer_end(c, K_SCATTER);
     timer_begin(c, K_PERMUTE);
     // a Tait-fluid context keeps J - 1 in the first F field and never reads the other eight
